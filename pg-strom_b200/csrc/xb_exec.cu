@@ -141,7 +141,8 @@ xb_group_get(const xb_plan *plan, const XbRegs &R, uint32_t lane, char *entries,
 {
     const uint32_t gsz = plan->gent_size;
     uint64_t pos = hash & cap_mask;
-    const uint64_t limit = SMEM ? cap_mask : (cap_mask < XB_PROBE_LIMIT ? cap_mask : XB_PROBE_LIMIT);
+    const uint64_t bound = SMEM ? XB_SM_PROBES - 1 : XB_PROBE_LIMIT;
+    const uint64_t limit = cap_mask < bound ? cap_mask : bound;
     for (uint64_t probe = 0; probe <= limit; probe++) {
         char *e = entries + pos * gsz;
         xb_gent_head *h = (xb_gent_head *)e;
@@ -2298,6 +2299,26 @@ static uint64_t xb_next_pow2(uint64_t x)
     return p;
 }
 
+/*
+ * Entries of the per-CTA shared group table for est groups: a load of at
+ * most 1/4 where 48 KB hold that (four CTAs share an SM), up to 7/8 where
+ * they do not, and none beyond: most rows would search a crowded table and
+ * go to the global one all the same, whose entries are many enough by then
+ * for the L2's atomics (2M rows, 300 groups: 2.27 ms a query through a table
+ * of 256 entries, 1.35 ms without one).  Large entries count too: three
+ * groups of 288 bytes take 10.1 ms in the global table, 1.43 ms here.
+ */
+static uint32_t xb_sm_cap_for(double est, uint32_t gent_size)
+{
+    const uint64_t room = (48 * 1024) / xb_jit_sm_stride(gent_size);
+    if (est > (double)room)
+        return 0;
+    uint64_t cap = xb_next_pow2((uint64_t)(est * 4) + 16);
+    while (cap > room && cap > 8)
+        cap >>= 1;
+    return cap <= room && est * 8 <= (double)cap * 7 ? (uint32_t)cap : 0;
+}
+
 extern "C" int
 xpuB200OpenSession(xpuB200Device *dev, const kern_session_info *session, uint64_t session_sz,
                    const kern_multirels *kmrels, uint64_t kmrels_sz,
@@ -2436,14 +2457,7 @@ xpuB200OpenSession(xpuB200Device *dev, const kern_session_info *session, uint64_
         cudaMemsetAsync(s->h_gt.entries, 0, cap * plan->gent_size, st);
         DALLOC(sizeof(xb_gtable), &s->d_gt);
         cudaMemcpyAsync(s->d_gt, &s->h_gt, sizeof(xb_gtable), cudaMemcpyHostToDevice, st);
-        /* shared-memory table for small group counts */
-        if (est <= 2048 && plan->gent_size <= 256) {
-            uint32_t smc = (uint32_t)xb_next_pow2((uint64_t)(est * 4) + 16);
-            if (smc < 32) smc = 32;
-            while ((size_t)smc * plan->gent_size > 48 * 1024 && smc > 32) smc >>= 1;
-            if ((size_t)smc * plan->gent_size <= 48 * 1024)
-                s->sm_cap = smc;
-        }
+        s->sm_cap = xb_sm_cap_for(est, plan->gent_size);
     }
     /* test hooks, inert unless set: XPU_B200_WAIT_LIMIT shortens the
      * bounded wait on a BUSY group entry; XPU_B200_TEST_BUSY_GROUPS=1 marks

@@ -706,7 +706,8 @@ struct Gen {
         o << "template <bool SMEM>\n__device__ __forceinline__ char *\n"
              "xbj_group_get(const XbjRegs &R, const XbjEnv &E, char *entries, uint64_t cap_mask, uint32_t hash, bool *full)\n{\n"
              "    uint64_t pos = hash & cap_mask;\n"
-             "    const uint64_t limit = SMEM ? cap_mask : (cap_mask < XB_PROBE_LIMIT ? cap_mask : XB_PROBE_LIMIT);\n"
+             "    const uint64_t bound = SMEM ? XB_SM_PROBES - 1 : XB_PROBE_LIMIT;\n"
+             "    const uint64_t limit = cap_mask < bound ? cap_mask : bound;\n"
              "    for (uint64_t probe = 0; probe <= limit; probe++) {\n"
              "        char *e = entries + pos * (SMEM ? XBJ_SM_STRIDE : XBJ_GENT_SIZE);\n"
              "        xb_gent_head *h = (xb_gent_head *)e;\n"
