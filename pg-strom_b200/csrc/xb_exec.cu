@@ -3036,12 +3036,13 @@ static bool xb_part_prepare(xpuB200Session *s, uint64_t nunits, uint32_t format,
 /* the dump region, sized for a launch of 'grid' CTAs: every CTA's shared
  * table merged at exit, plus the rows in flight after the table asked to
  * grow (two 32-row batches per warp: the one a warp is in when the request
- * comes, and one more if its look at the flag came just before) when the
- * table's free half is smaller than twice those */
+ * comes, and one more if its look at the flag came just before; and the
+ * groups the warps had not counted yet) when the table's free half is
+ * smaller than twice those */
 static int xb_dump_ensure(xpuB200Session *s, int grid, uint32_t sm_cap, cudaStream_t st, kern_errorbuf *err)
 {
     const uint64_t cap = s->h_gt.cap_mask + 1;
-    const uint64_t inflight = (uint64_t)grid * XB_WARPS * 64;
+    const uint64_t inflight = (uint64_t)grid * XB_WARPS * (64 + XB_UNCOUNTED);
     uint64_t need = (uint64_t)grid * sm_cap;
     if (cap / 2 < 2 * inflight)
         need += inflight;

@@ -138,11 +138,15 @@ __device__ __forceinline__ void xb_gt_want_grow(xb_gtable *gt)
         atomicExch(&gt->grow, 1u);
 }
 
-/* count a new entry of the global table; once soft_cap entries are in
- * use the table asks to grow */
-__device__ __forceinline__ void xb_gt_count_new(xb_gtable *gt)
+/* new global entries a warp of a specialised kernel may leave uncounted
+ * between 32-row batches */
+#define XB_UNCOUNTED    31
+
+/* count new entries of the global table; once soft_cap entries are in use
+ * the table asks to grow */
+__device__ __forceinline__ void xb_gt_count_new(xb_gtable *gt, uint32_t k = 1)
 {
-    const unsigned long long n = atomicAdd((unsigned long long *)&gt->nused, 1ULL) + 1ULL;
+    const unsigned long long n = atomicAdd((unsigned long long *)&gt->nused, (unsigned long long)k) + k;
     if (n >= gt->soft_cap)
         xb_gt_want_grow(gt);
 }
@@ -736,7 +740,7 @@ struct alignas(16) XbSrc {
     uint32_t row0;                  /* ARROW / ROW: first row of the unit */
     uint32_t item;                  /* next item of the unit */
     uint32_t nitems;                /* items of the unit */
-    uint32_t __pad;
+    uint32_t newg;                  /* specialised kernels: new global groups not yet counted */
     uint32_t grow_buf[4];           /* specialised kernels, lane 0: bytes 48..63 of the
                                      * group table (its 'grow' word), fetched asynchronously */
 };

@@ -48,6 +48,7 @@ struct XbjEnv {
     uint32_t        part_cap;
     uint32_t        part_shift;
     uint32_t        replay;         /* in the replay: a full table leaves the record for later */
+    uint32_t       *newg;           /* shared memory: new global groups not yet counted in the table */
 };
 
 /* per-thread counters, 32-bit to spare registers; flushed into the launch
@@ -200,6 +201,17 @@ __device__ __forceinline__ uint32_t xbj_grow_seen(const uint32_t *buf, uint32_t 
     return *(volatile const uint32_t *)&buf[1];
 }
 
+/* add *newg new groups to the table's count (one thread; nobody is
+ * creating groups against newg meanwhile) */
+__device__ __forceinline__ void xbj_count_flush(xb_gtable *gt, uint32_t *newg)
+{
+    const uint32_t n = *(volatile uint32_t *)newg;
+    if (n) {
+        *(volatile uint32_t *)newg = 0;
+        xb_gt_count_new(gt, n);
+    }
+}
+
 __device__ __forceinline__ unsigned long long xbj_warp_sum(unsigned long long v)
 {
 #pragma unroll
@@ -256,6 +268,9 @@ xbj_body(const XbExecArgs &args, char *smem)
     E.part_cap = args.part_cap;
     E.part_shift = args.part_shift;
     E.replay = 0;
+    E.newg = &wsrc[threadIdx.x >> 5].newg;
+    if (lane == 0)
+        *E.newg = 0;
     XbjCnt C;
     C.raw = C.in = C.out = 0;
     C.gready = 0;
@@ -399,6 +414,10 @@ xbj_body(const XbExecArgs &args, char *smem)
             xbj_flush_cnt(C, args.st);
         if (__any_sync(XB_FULL, failed))
             break;
+        /* (at most XB_UNCOUNTED groups of a warp stay uncounted between
+         * batches, which the growth's dump region allows for) */
+        if (lane == 0 && *(volatile uint32_t *)E.newg > XB_UNCOUNTED)
+            xbj_count_flush(args.gt, E.newg);
         if (args.left_out && __shfl_sync(XB_FULL, xbj_grow_seen(src.grow_buf, lane), 0)) {
             /* the table is to grow: leave the rest for the resume launch */
             xb_src_leave(args, src, lane, item, nitems);
@@ -412,6 +431,9 @@ xbj_body(const XbExecArgs &args, char *smem)
     if (lane == 0)
         asm volatile("mbarrier.inval.shared::cta.b64 [%0];" :: "r"(xbj_smem_addr(mbar)) : "memory");
 #endif
+    __syncwarp();
+    if (lane == 0 && args.gt)
+        xbj_count_flush(args.gt, E.newg);
     /* statistics */
     {
         const unsigned long long raw = xbj_warp_sum(C.raw);
@@ -503,6 +525,7 @@ extern "C" __global__ void __launch_bounds__(XB_BLOCK, XBJ_MIN_BLOCKS)
 xbj_replay(const __grid_constant__ XbReplayArgs args)
 {
     __shared__ uint32_t cur;            /* the CTA's bucket */
+    __shared__ uint32_t newg;           /* groups created in it */
     XbjEnv E;
     E.plan = args.plan;
     E.st = args.st;
@@ -520,9 +543,14 @@ xbj_replay(const __grid_constant__ XbReplayArgs args)
     E.part_cap = 0;
     E.part_shift = 0;
     E.replay = 1;
+    E.newg = &newg;
+    if (threadIdx.x == 0)
+        newg = 0;
     for (;;) {
-        if (threadIdx.x == 0)
+        if (threadIdx.x == 0) {
+            xbj_count_flush(args.gt, &newg);    /* the last bucket's */
             cur = atomicAdd(args.cursor, 1u);
+        }
         __syncthreads();
         const uint32_t b = cur;
         if (b >= args.nparts)
