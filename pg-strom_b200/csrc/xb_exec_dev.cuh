@@ -301,6 +301,14 @@ xb_numeric_sum_value(const uint8_t *vl, int weight_d, uint8_t *p_kind, xb_i128 *
     return 0;
 }
 
+/* state flag of a numeric that is not a number's digits */
+__device__ __forceinline__ uint32_t xb_numeric_special(uint8_t kind)
+{
+    return kind == XB_NUM_PINF ? PAGG_NUMERIC_ATTRS__PINF
+         : kind == XB_NUM_NINF ? PAGG_NUMERIC_ATTRS__NINF
+         : PAGG_NUMERIC_ATTRS__NAN;
+}
+
 /* per-value updates of the actions that are not combined across lanes */
 __device__ __forceinline__ void
 xb_agg_numeric_add(char *s, const uint8_t *vl, int16_t weight, xb_status *st)
@@ -312,10 +320,7 @@ xb_agg_numeric_add(char *s, const uint8_t *vl, int16_t weight, xb_status *st)
         atomicAdd((unsigned long long *)s, 1ULL);
         xb_atomic_add_i128((uint64_t *)(s + 8), v);
     } else {
-        const uint32_t special = kind == XB_NUM_PINF ? PAGG_NUMERIC_ATTRS__PINF
-                               : kind == XB_NUM_NINF ? PAGG_NUMERIC_ATTRS__NINF
-                               : PAGG_NUMERIC_ATTRS__NAN;
-        atomicOr((unsigned int *)(s + 24), special);
+        atomicOr((unsigned int *)(s + 24), xb_numeric_special(kind));
     }
 }
 
@@ -335,10 +340,7 @@ xb_agg_numeric_add_sm(char *s, const uint8_t *vl, int16_t weight, xb_status *st,
     } else {
         if (nc)
             xb_red_shared_add_u32(s, 1u);
-        const uint32_t special = kind == XB_NUM_PINF ? PAGG_NUMERIC_ATTRS__PINF
-                               : kind == XB_NUM_NINF ? PAGG_NUMERIC_ATTRS__NINF
-                               : PAGG_NUMERIC_ATTRS__NAN;
-        atomicOr((unsigned int *)(s + 24), special);
+        atomicOr((unsigned int *)(s + 24), xb_numeric_special(kind));
     }
 }
 

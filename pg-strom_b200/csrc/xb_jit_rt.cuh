@@ -57,7 +57,19 @@ struct XbjCnt {
     uint32_t raw, in, out;
     uint32_t depth[XB_MAX_DEPTH + 1];
     uint64_t gready;                /* group-id entries this lane has seen ready */
+#ifdef XBJ_ACC
+    XbjAcc   acc;                   /* no GROUP BY keys: the aggregate of this lane's rows */
+#endif
 };
+
+/* the lanes' sum, in lane 0 */
+__device__ __forceinline__ unsigned long long xbj_warp_sum(unsigned long long v)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+        v += __shfl_down_sync(XB_FULL, v, o);
+    return v;
+}
 
 __device__ __forceinline__ void xbj_flush_cnt(XbjCnt &C, xb_status *st)
 {
@@ -117,6 +129,32 @@ __device__ __forceinline__ void xbj_prefetch_tuple(const uint8_t *page, uint32_t
 
 __device__ __forceinline__ void
 xbj_pipeline(XbjRegs &R, const XbjEnv &E, XbjCnt &C, bool &failed);
+
+#ifdef XBJ_ACC
+/* generated: a lane's aggregate, empty at first; all lanes of a warp added
+ * to the one group's entry */
+__device__ __forceinline__ void xbj_acc_init(XbjAcc &A);
+__device__ __forceinline__ void xbj_acc_flush(XbjAcc &A, const XbjEnv &E);
+
+/* s + c += x, the rounding error of the sum kept in c (TwoSum) */
+__device__ __forceinline__ void xbj_two_sum(double &s, double &c, double x)
+{
+    const double t = __dadd_rn(s, x);
+    const double bp = __dsub_rn(t, s);
+    c = __dadd_rn(c, __dadd_rn(__dsub_rn(s, __dsub_rn(t, bp)), __dsub_rn(x, bp)));
+    s = t;
+}
+
+/* the warp's (s, c) pairs added up in every lane */
+__device__ __forceinline__ void xbj_warp_two_sum(double &s, double &c)
+{
+    for (int o = 16; o > 0; o >>= 1) {
+        const double y = __shfl_xor_sync(XB_FULL, s, o), d = __shfl_xor_sync(XB_FULL, c, o);
+        xbj_two_sum(s, c, y);
+        c = __dadd_rn(c, d);
+    }
+}
+#endif
 
 #ifdef XBJ_PART
 /* the record's NULL-mask word carries this bit while the record waits for
@@ -212,13 +250,6 @@ __device__ __forceinline__ void xbj_count_flush(xb_gtable *gt, uint32_t *newg)
     }
 }
 
-__device__ __forceinline__ unsigned long long xbj_warp_sum(unsigned long long v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-        v += __shfl_down_sync(XB_FULL, v, o);
-    return v;
-}
 
 /* one launch's (or one mixed-launch command's) work for this CTA; ends
  * with the counters and the shared group table flushed, without a final
@@ -274,6 +305,9 @@ xbj_body(const XbExecArgs &args, char *smem)
     XbjCnt C;
     C.raw = C.in = C.out = 0;
     C.gready = 0;
+#ifdef XBJ_ACC
+    xbj_acc_init(C.acc);
+#endif
 #pragma unroll
     for (int d = 0; d <= XB_MAX_DEPTH; d++)
         C.depth[d] = 0;
@@ -432,6 +466,10 @@ xbj_body(const XbExecArgs &args, char *smem)
         asm volatile("mbarrier.inval.shared::cta.b64 [%0];" :: "r"(xbj_smem_addr(mbar)) : "memory");
 #endif
     __syncwarp();
+#ifdef XBJ_ACC
+    xbj_acc_flush(C.acc, E);
+    __syncwarp();
+#endif
     if (lane == 0 && args.gt)
         xbj_count_flush(args.gt, E.newg);
     /* statistics */
