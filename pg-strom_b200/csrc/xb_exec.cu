@@ -3223,7 +3223,6 @@ int xb_launch_on(xpuB200Session *s, const xb_task *d_tasks, uint32_t ntasks,
     a.ntasks = ntasks;
     a.nunits = nunits;
     a.format = format;
-    a.sm_cap = s->sm_cap;
     a.warp_bytes = s->warp_bytes;
     a.dst = s->launch_dst;
     a.dst_len = s->launch_dst_len;
@@ -3232,6 +3231,8 @@ int xb_launch_on(xpuB200Session *s, const xb_task *d_tasks, uint32_t ntasks,
     a.st = d_status;
     /* served launches (pooled slot streams) do not wait for a kernel build */
     void *fn = xb_session_jit(s, format, stream == s->stream);
+    /* (the first launch may adopt a tuned table size) */
+    a.sm_cap = s->sm_cap;
     int grid = fn ? s->jit_grid[format] : s->grid;
     /* a warp per unit, up to the resident warps: a heap page takes a warp
      * about 20 us whatever runs beside it (dependent loads), so a launch of
