@@ -48,26 +48,24 @@ xpuB200BatchCreate(xpuB200Session *s, const kern_data_store *const *kds_dev, uin
                       "the session projects rows into kds_dst: use xpuB200ExecTaskDst");
     XB_CUDA(cudaSetDevice(s->dev->dindex), err);
     std::vector<xb_task> tasks(nchunks);
-    std::vector<char> first_head;
     uint64_t base = 0, bytes = 0, rows = 0;
     uint32_t format = 0;
-    for (uint32_t i = 0; i < nchunks; i++) {
-        kern_data_store head;
+    for (uint32_t i = 0; i < nchunks; i++)
         if (((uintptr_t)kds_dev[i] & 7) != 0)
             return XB_ERR(err, ERRCODE_DEVICE_ERROR, "chunk %u is not 8-byte aligned", i);
-        XB_CUDA(cudaMemcpy(&head, kds_dev[i], offsetof(kern_data_store, colmeta), cudaMemcpyDeviceToHost), err);
-        std::vector<char> hb(KDS_HEAD_LENGTH(&head));
-        XB_CUDA(cudaMemcpy(hb.data(), kds_dev[i], hb.size(), cudaMemcpyDeviceToHost), err);
-        const kern_data_store *h = (const kern_data_store *)hb.data();
-        int rc = xb_check_kds(h, err);
+    std::vector<std::vector<char>> heads;
+    int rc = xb_fetch_heads(s->dev, s->stream, kds_dev, nchunks, heads, err);
+    if (rc) return rc;
+    for (uint32_t i = 0; i < nchunks; i++) {
+        const kern_data_store *h = (const kern_data_store *)heads[i].data();
+        rc = xb_check_kds(h, err);
         if (rc) return rc;
         if (i == 0) {
-            first_head = hb;
             format = (uint32_t)h->format;
             xb_note_layout(s, h);
         } else {
             /* one launch decodes every chunk with the same column layout */
-            const kern_data_store *f = (const kern_data_store *)first_head.data();
+            const kern_data_store *f = (const kern_data_store *)heads[0].data();
             if ((uint32_t)h->format != format || h->ncols != f->ncols ||
                 (h->format != KDS_FORMAT_ARROW &&
                  memcmp(h->colmeta, f->colmeta, sizeof(kern_colmeta) * h->ncols) != 0))
@@ -88,11 +86,15 @@ xpuB200BatchCreate(xpuB200Session *s, const kern_data_store *const *kds_dev, uin
     b->format = format;
     b->bytes = bytes;
     b->rows = rows;
-    if (cudaMalloc((void **)&b->d_tasks, sizeof(xb_task) * nchunks) != cudaSuccess) {
+    /* from the device's pool, on the session's stream: cudaMalloc and
+     * cudaFree of these few bytes took 0.3 to 5 ms of a query (unmapping
+     * waits for the whole device) */
+    if (cudaMallocAsync((void **)&b->d_tasks, sizeof(xb_task) * nchunks, s->stream) != cudaSuccess) {
+        cudaGetLastError();
         delete b;
         return XB_ERR(err, ERRCODE_DEVICE_FATAL, "out of device memory for the batch");
     }
-    cudaMemcpy(b->d_tasks, tasks.data(), sizeof(xb_task) * nchunks, cudaMemcpyHostToDevice);
+    cudaMemcpyAsync(b->d_tasks, tasks.data(), sizeof(xb_task) * nchunks, cudaMemcpyHostToDevice, s->stream);
     *p_batch = b;
     return 0;
 }
@@ -266,7 +268,7 @@ xpuB200BatchDestroy(xpuB200Batch *b)
 {
     if (!b) return;
     cudaSetDevice(b->sess->dev->dindex);
-    cudaFree(b->d_tasks);
+    cudaFreeAsync(b->d_tasks, b->sess->stream);
     delete b;
 }
 
@@ -405,6 +407,7 @@ xpuB200MixCreate(xpuB200Device *dev, uint32_t ncmds, xpuB200Session *const *sess
     std::vector<uint64_t> units(ncmds);
     std::vector<uint32_t> formats(ncmds);
     uint64_t bytes = 0, total_units = 0;
+    std::vector<std::vector<char>> heads;
     for (uint32_t i = 0; i < ncmds; i++) {
         xpuB200Session *s = sess[i];
         if (!s || s->dev != dev)
@@ -413,11 +416,12 @@ xpuB200MixCreate(xpuB200Device *dev, uint32_t ncmds, xpuB200Session *const *sess
             return XB_ERR(err, ERRCODE_DEVICE_ERROR, "command %u: projection sessions run through xpuB200ExecTaskDst", i);
         if (((uintptr_t)kds_dev[i] & 7) != 0)
             return XB_ERR(err, ERRCODE_DEVICE_ERROR, "command %u: chunk is not 8-byte aligned", i);
-        kern_data_store head;
-        XB_CUDA(cudaMemcpy(&head, kds_dev[i], offsetof(kern_data_store, colmeta), cudaMemcpyDeviceToHost), err);
-        std::vector<char> hb(KDS_HEAD_LENGTH(&head));
-        XB_CUDA(cudaMemcpy(hb.data(), kds_dev[i], hb.size(), cudaMemcpyDeviceToHost), err);
-        const kern_data_store *h = (const kern_data_store *)hb.data();
+    }
+    int hrc = xb_fetch_heads(dev, dev->stream, kds_dev, ncmds, heads, err);
+    if (hrc) return hrc;
+    for (uint32_t i = 0; i < ncmds; i++) {
+        xpuB200Session *s = sess[i];
+        const kern_data_store *h = (const kern_data_store *)heads[i].data();
         int rc = xb_check_kds(h, err);
         if (rc) return rc;
         {

@@ -25,6 +25,22 @@
 #include "xb_jit.h"
 #include "xpu_b200.h"
 
+/* pinned memory a session's launches report into: the status and the group
+ * table's header, read back together */
+struct xb_pinned {
+    xb_status       st;
+    xb_gtable       gt;
+};
+
+/* pinned memory (mapped on the GPU) that one fetch of chunk headers uses:
+ * XB_HEADS requests, then a slot of XB_HEAD_SLOT bytes for each */
+#define XB_HEADS        128
+#define XB_HEAD_SLOT    4096
+struct xb_head_scratch {
+    char           *mem = nullptr;
+    cudaEvent_t     ev = nullptr;
+};
+
 struct xpuB200Device {
     int             dindex;
     int             nsm;
@@ -36,8 +52,9 @@ struct xpuB200Device {
      * memory costs far more than a query's own host work */
     std::mutex      pool_lock;
     std::vector<cudaStream_t> free_streams;
-    std::vector<xb_status *> free_status;
-    std::vector<xb_status *> status_blocks;
+    std::vector<struct xb_pinned *> free_status;
+    std::vector<struct xb_pinned *> status_blocks;
+    std::vector<struct xb_head_scratch> free_heads;
     /* inner relations built for sessions with a join_inner_handle, kept
      * while sessions use them and, within inner_budget bytes, after */
     std::mutex      inner_lock;
@@ -94,7 +111,8 @@ struct xpuB200Session {
     xb_gtable       h_gt = {};
     xb_gtable      *d_gt = nullptr;
     xb_status      *d_status = nullptr;
-    xb_status      *h_status = nullptr;     /* pinned */
+    xb_pinned      *pinned = nullptr;
+    xb_status      *h_status = nullptr;     /* pinned->st */
     char           *d_src = nullptr;
     uint64_t        d_src_cap = 0;
     xb_task        *d_tasks = nullptr;      /* work queue of single-chunk launches */
@@ -194,6 +212,10 @@ static inline void xb_clear_error(kern_errorbuf *err)
 /* the core's functions the services call (xb_exec.cu) */
 void xb_account_status(xpuB200Session *s, const xb_status *hs, kern_exec_results *results);
 int xb_check_kds(const kern_data_store *kds, kern_errorbuf *err);
+/* the headers of n chunks in this device's memory (each 8-byte aligned),
+ * copied to the host */
+int xb_fetch_heads(xpuB200Device *dev, cudaStream_t st, const kern_data_store *const *kds, uint32_t n,
+                   std::vector<std::vector<char>> &heads, kern_errorbuf *err);
 uint32_t xb_chunk_units(const kern_data_store *head);
 void xb_fill_results(const xb_status *hs, uint32_t nrels, kern_exec_results *results);
 cudaStream_t xb_get_stream(xpuB200Device *dev);
@@ -217,7 +239,7 @@ std::tuple<int, uint64_t, uint32_t> xb_tune_key(xpuB200Session *s, uint32_t form
 int xb_gt_read(xpuB200Session *s, xb_gtable *g, kern_errorbuf *err);
 int xb_gt_grow(xpuB200Session *s, uint64_t min_entries, kern_errorbuf *err);
 int xb_gt_settle(xpuB200Session *s, kern_errorbuf *err);
-int xb_wait_status(xpuB200Session *s, kern_errorbuf *err);
+int xb_wait_status(xpuB200Session *s, kern_errorbuf *err, bool with_gt = false);
 
 /* mixed launches (xb_batch.cu), which the serving scheduler also issues:
  * the commands grouped by the kernel they run on, one launch per group */

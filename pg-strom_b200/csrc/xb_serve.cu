@@ -469,13 +469,13 @@ xpuB200Submit(xpuB200Session *s, const kern_data_store *kds_src, int kds_src_on_
     xb_cmd c;
     memset(&c, 0, sizeof(c));
     std::vector<char> hb;
-    kern_data_store head;
     if (kds_src_on_device) {
         if (((uintptr_t)kds_src & 7) != 0)
             return XB_ERR(err, ERRCODE_DEVICE_ERROR, "device chunk is not 8-byte aligned");
-        XB_CUDA(cudaMemcpy(&head, kds_src, offsetof(kern_data_store, colmeta), cudaMemcpyDeviceToHost), err);
-        hb.resize(KDS_HEAD_LENGTH(&head));
-        XB_CUDA(cudaMemcpy(hb.data(), kds_src, hb.size(), cudaMemcpyDeviceToHost), err);
+        std::vector<std::vector<char>> heads;
+        rc = xb_fetch_heads(dev, s->stream, &kds_src, 1, heads, err);
+        if (rc) return rc;
+        hb.swap(heads[0]);
     } else {
         hb.assign((const char *)kds_src, (const char *)kds_src + KDS_HEAD_LENGTH(kds_src));
     }
