@@ -1376,6 +1376,282 @@ __global__ void xb_final_write(XbFinalArgs args)
 }
 
 /* ----------------------------------------------------------------
+ * kds_final by tiles of the group table
+ *
+ * The table is read twice: once for the groups and item bytes of every
+ * tile (and hash partition), whose prefixes are the tuples' places, and
+ * once for the tuples.  A CTA lists its tile's groups in shared memory;
+ * then consecutive threads write consecutive 8-byte words of consecutive
+ * items, each word put together from the entry as the plan's program says
+ * (XbFinalProg), so that entries are read and items written in whole lines.
+ * Groups whose tuple the program does not cover (text or numeric keys, NULL
+ * keys) are written by a thread each.
+ * Bound by memory: the heads of all slots (a 32-byte sector of each), then
+ * entry and item bytes once.  10M groups in a table of 33.5M slots as eight
+ * parts: 2.9 ms a call, 32.8 ms with a size per slot, scanned twice for
+ * every part, and a thread per tuple writing bytes.
+ * ---------------------------------------------------------------- */
+
+/* item bytes of group e; fast: its tuple is the program's */
+__device__ __forceinline__ uint32_t
+xb_final_item(const XbTileArgs &a, const char *e, uint32_t nkeys, uint32_t keys_off, bool *fast)
+{
+    bool f = a.prog.nunits != 0;
+    const xb_keyimg *img = (const xb_keyimg *)(e + keys_off);
+    for (uint32_t k = 0; f && k < nkeys; k++)
+        f = img[k].isnull == 0;
+    *fast = f;
+    if (f)
+        return a.prog.item;
+    const uint32_t t_len = xb_write_group_tuple(a.plan, e, nullptr, 0);
+    return (uint32_t)PGSTROM_MAXALIGN((a.row_format ? 0 : offsetof(kern_hashitem, t)) + t_len);
+}
+
+/* the launch's index of a group's part, or -1 */
+__device__ __forceinline__ int xb_final_part(const XbTileArgs &a, uint32_t hash)
+{
+    if (a.nparts == 1)
+        return 0;
+    const uint32_t p = hash % a.nparts - a.part0;
+    return p < a.pset ? (int)p : -1;
+}
+
+__global__ void __launch_bounds__(XB_FINAL_TILE)
+xb_final_tiles(const __grid_constant__ XbTileArgs a)
+{
+    /* of each part: bytes beyond the program's item size (summed modulo
+     * 2^64), then groups */
+    extern __shared__ unsigned long long more[];
+    uint32_t *groups = (uint32_t *)(more + a.pset);
+    const uint32_t gsz = a.plan->gent_size, nkeys = a.plan->nkeys, koff = a.plan->gent_keys_off;
+    const char *entries = a.gt->entries;
+    for (uint32_t tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x) {
+        for (uint32_t p = threadIdx.x; p < a.pset; p += blockDim.x) {
+            more[p] = 0;
+            groups[p] = 0;
+        }
+        __syncthreads();
+        uint32_t n = 0;
+        const uint64_t s0 = (uint64_t)tile * a.tile_slots;
+        for (uint64_t i = s0 + threadIdx.x; i < s0 + a.tile_slots && i < a.cap; i += blockDim.x) {
+            const char *e = entries + i * gsz;
+            const xb_gent_head h = *(const xb_gent_head *)e;
+            const int p = h.state == XB_GSTATE_READY ? xb_final_part(a, h.hash) : -1;
+            if (p < 0)
+                continue;
+            bool fast;
+            const uint32_t sz = xb_final_item(a, e, nkeys, koff, &fast);
+            if (a.nparts == 1)
+                n++;
+            else
+                atomicAdd(&groups[p], 1u);
+            if (!fast)
+                atomicAdd(&more[p], (unsigned long long)sz - a.prog.item);
+        }
+        if (a.nparts == 1) {
+            n = __reduce_add_sync(XB_FULL, n);
+            if ((threadIdx.x & 31) == 0)
+                atomicAdd(&groups[0], n);
+        }
+        __syncthreads();
+        for (uint32_t p = threadIdx.x; p < a.pset; p += blockDim.x) {
+            a.count[(uint64_t)p * a.ntiles + tile] = groups[p];
+            a.bytes[(uint64_t)p * a.ntiles + tile] = (uint64_t)groups[p] * a.prog.item + more[p];
+        }
+        __syncthreads();
+    }
+}
+
+/* exclusive prefixes of n <= 4096 tile counts and bytes by one CTA */
+__global__ void __launch_bounds__(XB_FINAL_TILE)
+xb_final_scan_small(XbTileArgs a, uint32_t *count_scan, uint64_t *bytes_scan, uint32_t n)
+{
+    uint64_t cb = 0, bb = 0;
+    for (uint32_t i0 = 0; i0 < n; i0 += XB_FINAL_TILE) {
+        const uint32_t i = i0 + threadIdx.x;
+        const uint64_t c = i < n ? a.count[i] : 0, b = i < n ? a.bytes[i] : 0;
+        uint64_t ct, bt;
+        const uint64_t ci = xb_block_scan_incl<uint64_t, XbOpSum>(c, &ct);
+        const uint64_t bi = xb_block_scan_incl<uint64_t, XbOpSum>(b, &bt);
+        if (i < n) {
+            count_scan[i] = (uint32_t)(cb + ci - c);
+            bytes_scan[i] = bb + bi - b;
+        }
+        cb += ct;
+        bb += bt;
+    }
+}
+
+/* groups and item bytes of every part */
+__global__ void xb_final_totals(XbTileArgs a, uint64_t *totals)
+{
+    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < a.pset; p += gridDim.x * blockDim.x) {
+        const uint64_t i = (uint64_t)p * a.ntiles, j = i + a.ntiles - 1;
+        totals[2 * p] = (uint64_t)(a.count_scan[j] - a.count_scan[i]) + a.count[j];
+        totals[2 * p + 1] = a.bytes_scan[j] - a.bytes_scan[i] + a.bytes[j];
+    }
+}
+
+/* the parts' headers, from the session's definition, and empty hash slots */
+__global__ void xb_final_heads(char *out, const XbFinalPart *part, const uint64_t *head, uint32_t head_len,
+                               uint32_t row_format)
+{
+    const XbFinalPart P = part[blockIdx.y];
+    uint64_t *o = (uint64_t *)(out + P.out);
+    const uint64_t nw = head_len / 8, stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < nw + P.nslots; i += stride) {
+        uint64_t w = i < nw ? head[i] : 0;
+        if (i == offsetof(kern_data_store, length) / 8)
+            w = P.length;
+        else if (i == offsetof(kern_data_store, usage) / 8)
+            w = P.length - P.items_base;
+        else if (i == offsetof(kern_data_store, nitems) / 8)
+            w = (w & ~0xffffffffULL) | P.nitems;
+        else if (i == offsetof(kern_data_store, format) / 8)
+            w = (w & ~0xffULL) | (uint8_t)(row_format ? KDS_FORMAT_ROW : KDS_FORMAT_HASH);
+        else if (i == offsetof(kern_data_store, hash_nslots) / 8)
+            w = (w & ~0xffffffffULL) | P.nslots;
+        o[i] = w;
+    }
+}
+static_assert(offsetof(kern_data_store, nitems) % 8 == 0 && offsetof(kern_data_store, format) % 8 == 0 &&
+              offsetof(kern_data_store, hash_nslots) % 8 == 0, "xb_final_heads patches the low half of a word");
+
+/* 4-byte unit u of the tuple of entry e */
+__device__ __forceinline__ uint32_t
+xb_final_unit(const char *e, uint32_t op, uint32_t src, uint32_t imm, uint32_t rowid)
+{
+    const uint64_t *su = (const uint64_t *)(e + (src & ~7u));
+    switch (op) {
+    case XB_FU_COPY:
+        return *(const uint32_t *)(e + src);
+    case XB_FU_ROWID:
+        return rowid;
+    case XB_FU_SUM_LO: case XB_FU_SUM_HI: {
+        const uint64_t v = __double_as_longlong(__dadd_rn(__longlong_as_double(su[0]), __longlong_as_double(su[1])));
+        return op == XB_FU_SUM_LO ? (uint32_t)v : (uint32_t)(v >> 32);
+    }
+    case XB_FU_MM_ATTRS:
+        return *(const uint32_t *)(su + 1) ? PAGG_MINMAX_ATTRS__VALID : 0;
+    case XB_FU_MMFP_LO: case XB_FU_MMFP_HI: {
+        const double d = *(const uint32_t *)(su + 1) ? xb_f64_from_ordered((int64_t)su[0])
+                                                     : (imm ? -1.7976931348623157e308 : 1.7976931348623157e308);
+        const uint64_t v = __double_as_longlong(d);
+        return op == XB_FU_MMFP_LO ? (uint32_t)v : (uint32_t)(v >> 32);
+    }
+    case XB_FU_NUM_ATTRS:
+        return imm | *(const uint32_t *)(e + src);
+    case XB_FU_FLT4:
+        return __float_as_uint((float)__longlong_as_double(su[0]));
+    default:
+        return imm;
+    }
+}
+
+__global__ void __launch_bounds__(XB_FINAL_TILE)
+xb_final_fill(const __grid_constant__ XbTileArgs a)
+{
+    /* nparts > 1, placed of each part in the tile: bytes of the groups that
+     * are not the program's (from the end of the part's bytes), groups, and
+     * groups of the program's */
+    extern __shared__ unsigned long long odd_bytes[];
+    uint32_t *groups = (uint32_t *)(odd_bytes + a.pset), *fasts = groups + a.pset;
+    __shared__ uint64_t prog[XB_FINAL_UNITS];
+    __shared__ uint64_t item[XB_FINAL_TILE];    /* place of the group's item in the output buffer */
+    __shared__ uint32_t slot[XB_FINAL_TILE];    /* its entry; bit 31: not the program's tuple */
+    __shared__ uint32_t rowid[XB_FINAL_TILE];
+    __shared__ uint32_t nlist;
+    const uint32_t gsz = a.plan->gent_size, nkeys = a.plan->nkeys, koff = a.plan->gent_keys_off;
+    const char *entries = a.gt->entries;
+    const uint32_t link = a.row_format ? 0 : (uint32_t)offsetof(kern_hashitem, t);
+    const uint32_t words = a.prog.nunits / 2;
+    for (uint32_t i = threadIdx.x; i < a.prog.nunits; i += blockDim.x)
+        prog[i] = ((uint64_t)a.prog.unit[i].imm << 32) | ((uint32_t)a.prog.unit[i].src << 16) | a.prog.unit[i].op;
+    for (uint32_t tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x) {
+        if (a.nparts > 1)
+            for (uint32_t p = threadIdx.x; p < a.pset; p += blockDim.x) {
+                odd_bytes[p] = 0;
+                groups[p] = fasts[p] = 0;
+            }
+        uint64_t n0 = 0, b0 = 0;                /* nparts == 1: placed so far */
+        const uint64_t s0 = (uint64_t)tile * a.tile_slots;
+        for (uint32_t sub = 0; sub < a.tile_slots && s0 + sub < a.cap; sub += XB_FINAL_TILE) {
+            const uint64_t i = s0 + sub + threadIdx.x;
+            const char *e = entries + i * gsz;
+            xb_gent_head h;
+            h.hash = 0;
+            h.state = XB_GSTATE_EMPTY;
+            if (i < a.cap)
+                h = *(const xb_gent_head *)e;
+            const int p = h.state == XB_GSTATE_READY ? xb_final_part(a, h.hash) : -1;
+            const bool ready = p >= 0;
+            bool fast = false;
+            const uint32_t sz = ready ? xb_final_item(a, e, nkeys, koff, &fast) : 0;
+            if (threadIdx.x == 0)
+                nlist = 0;
+            __syncthreads();
+            uint32_t rank = 0, at = 0;
+            uint64_t rel = 0;
+            const uint64_t pt = (uint64_t)(ready ? p : 0) * a.ntiles;
+            if (a.nparts == 1) {
+                /* in table order: (groups, bytes) scanned as one word */
+                uint64_t tot;
+                const uint64_t mine = ((uint64_t)(ready ? 1 : 0) << 40) | sz;
+                const uint64_t pre = xb_block_scan_incl<uint64_t, XbOpSum>(mine, &tot) - mine;
+                at = (uint32_t)(pre >> 40);
+                rank = (uint32_t)n0 + at;
+                rel = b0 + (pre & ((1ULL << 40) - 1));
+                n0 += tot >> 40;
+                b0 += tot & ((1ULL << 40) - 1);
+                if (threadIdx.x == 0)
+                    nlist = (uint32_t)(tot >> 40);
+            } else if (ready) {
+                rank = atomicAdd(&groups[p], 1u);
+                if (fast)
+                    rel = (uint64_t)atomicAdd(&fasts[p], 1u) * sz;
+                else
+                    rel = a.bytes[pt + tile] - sz - atomicAdd(&odd_bytes[p], (unsigned long long)sz);
+                at = atomicAdd(&nlist, 1u);
+            }
+            if (ready) {
+                const XbFinalPart &P = a.part[p];
+                rank += a.count_scan[pt + tile] - a.count_scan[pt];
+                rel += a.bytes_scan[pt + tile] - a.bytes_scan[pt] + P.items_base;
+                char *out = a.out + P.out;
+                uint64_t *hslots = (uint64_t *)(out + P.items_base) - P.nslots - P.nitems;
+                uint64_t *rowindex = hslots + P.nslots;
+                rowindex[rank] = P.length - (rel + link);
+                if (link)
+                    *(uint64_t *)(out + rel) =
+                        atomicExch((unsigned long long *)&hslots[h.hash % P.nslots],
+                                   (unsigned long long)(P.length - rel));
+                item[at] = P.out + rel + link;
+                slot[at] = (uint32_t)(i - s0) | (fast ? 0 : 0x80000000u);
+                rowid[at] = rank;
+                if (!fast) {
+                    char *t = out + rel + link;
+                    const uint32_t t_len = xb_write_group_tuple(a.plan, e, (kern_tupitem *)t, rank);
+                    for (uint32_t k = t_len; k < sz - link; k++)
+                        t[k] = 0;
+                }
+            }
+            __syncthreads();
+            for (uint32_t k = threadIdx.x; k < nlist * words; k += blockDim.x) {
+                const uint32_t j = k / words, w = k - j * words;
+                if (slot[j] & 0x80000000u)
+                    continue;
+                const char *ej = entries + (s0 + slot[j]) * gsz;
+                const uint64_t u0 = prog[2 * w], u1 = prog[2 * w + 1];
+                const uint32_t lo = xb_final_unit(ej, (uint32_t)u0 & 0xffff, (uint32_t)u0 >> 16, u0 >> 32, rowid[j]);
+                const uint32_t hi = xb_final_unit(ej, (uint32_t)u1 & 0xffff, (uint32_t)u1 >> 16, u1 >> 32, rowid[j]);
+                *(uint64_t *)(a.out + item[j] + 8 * w) = ((uint64_t)hi << 32) | lo;
+            }
+            __syncthreads();
+        }
+    }
+}
+
+/* ----------------------------------------------------------------
  * GPU-Sort of the final groups (kern_gpusort_prep_buffer,
  * kern_gpusort_exec_bitonic and the window-rank kernels of
  * cuda_gpusort.cu:15-996): every sort key of a group becomes one or two

@@ -126,6 +126,257 @@ static int xb_final_sort(xpuB200Session *s, XbFinalArgs fa, cudaStream_t st, All
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
+/* the fixed tuple of the session's groups as a program of 4-byte units
+ * (xb_write_group_tuple's layout with every key present), and the bytes of
+ * such an item; no units when a key's size or place depends on its value */
+static void xb_final_program(const xb_plan *plan, bool row_fmt, XbFinalProg *pg)
+{
+    pg->nunits = 0;
+    pg->item = 0;
+    uint8_t img[XB_FINAL_UNITS * 4] = {0};
+    uint16_t op[XB_FINAL_UNITS] = {0}, src[XB_FINAL_UNITS] = {0};
+    const uint32_t n = plan->naggs;
+    const uint32_t hoff = (uint32_t)PGSTROM_MAXALIGN(15 + (n + 7) / 8);
+    uint32_t t = hoff;
+    uint16_t infomask = HEAP_HASNULL;
+    auto put32 = [&](uint32_t at, uint32_t v) { memcpy(img + at, &v, 4); };
+    auto unit = [&](uint32_t at, uint16_t o, uint32_t s, uint32_t imm = 0) {
+        op[at / 4] = o;
+        src[at / 4] = (uint16_t)s;
+        put32(at, imm);
+    };
+    for (uint32_t j = 0; j < n; j++) {
+        const xb_agg &a = plan->aggs[j];
+        t = (uint32_t)PGSTROM_TYPEALIGN(a.attalign, t);
+        if ((t & 3) || t + 64 + ROWID_SIZE > sizeof(img))
+            return;
+        uint32_t nb = 0;
+        const uint32_t s = a.state_off;
+        switch (a.action) {
+        case KAGG_ACTION__VREF: {
+            if (a.key_index < 0)
+                break;
+            const uint32_t k = plan->gent_keys_off + sizeof(xb_keyimg) * a.key_index + offsetof(xb_keyimg, val);
+            switch (plan->keys[a.key_index].ld) {
+            case XB_LD_INT4: case XB_LD_DATE: nb = 4; unit(t, XB_FU_COPY, k); break;
+            case XB_LD_FLT4: nb = 4; unit(t, XB_FU_FLT4, k); break;
+            case XB_LD_INT8: case XB_LD_FLT8:
+                nb = 8;
+                unit(t, XB_FU_COPY, k);
+                unit(t + 4, XB_FU_COPY, k + 4);
+                break;
+            default: return;            /* varlena, or below 4 bytes */
+            }
+            break;
+        }
+        case KAGG_ACTION__NROWS_ANY: case KAGG_ACTION__NROWS_COND:
+            nb = 8;
+            unit(t, XB_FU_COPY, s);
+            unit(t + 4, XB_FU_COPY, s + 4);
+            break;
+        case KAGG_ACTION__PMIN_INT32: case KAGG_ACTION__PMIN_INT64:
+        case KAGG_ACTION__PMAX_INT32: case KAGG_ACTION__PMAX_INT64:
+        case KAGG_ACTION__PMIN_FP64: case KAGG_ACTION__PMAX_FP64: {
+            const bool fp = a.action == KAGG_ACTION__PMIN_FP64 || a.action == KAGG_ACTION__PMAX_FP64;
+            const uint32_t mx = a.action == KAGG_ACTION__PMAX_FP64 ? 1 : 0;
+            nb = 16;
+            put32(t, nb << 2);
+            unit(t + 4, XB_FU_MM_ATTRS, s);
+            unit(t + 8, fp ? XB_FU_MMFP_LO : XB_FU_COPY, s, mx);
+            unit(t + 12, fp ? XB_FU_MMFP_HI : XB_FU_COPY, fp ? s : s + 4, mx);
+            break;
+        }
+        case KAGG_ACTION__PSUM_INT: case KAGG_ACTION__PAVG_INT:
+        case KAGG_ACTION__PSUM_INT64: case KAGG_ACTION__PAVG_INT64:
+        case KAGG_ACTION__PSUM_NUMERIC: case KAGG_ACTION__PAVG_NUMERIC: {
+            const bool num = a.action == KAGG_ACTION__PSUM_NUMERIC || a.action == KAGG_ACTION__PAVG_NUMERIC;
+            const bool wide = num || a.action == KAGG_ACTION__PSUM_INT64 || a.action == KAGG_ACTION__PAVG_INT64;
+            nb = wide ? sizeof(kagg_state__psum_numeric_packed) : sizeof(kagg_state__psum_int_packed);
+            put32(t, nb << 2);
+            if (num)
+                unit(t + 4, XB_FU_NUM_ATTRS, s + 24, (uint32_t)a.weight & PAGG_NUMERIC_ATTRS__WEIGHT);
+            for (uint32_t k = 8; k < nb; k += 4)
+                unit(t + k, XB_FU_COPY, s + k - 8);
+            break;
+        }
+        case KAGG_ACTION__PSUM_FP: case KAGG_ACTION__PAVG_FP:
+        case KAGG_ACTION__STDDEV: case KAGG_ACTION__COVAR:
+            nb = a.action == KAGG_ACTION__STDDEV ? sizeof(kagg_state__stddev_packed)
+               : a.action == KAGG_ACTION__COVAR ? sizeof(kagg_state__covar_packed) : sizeof(kagg_state__psum_fp_packed);
+            put32(t, nb << 2);
+            unit(t + 8, XB_FU_COPY, s);
+            unit(t + 12, XB_FU_COPY, s + 4);
+            for (uint32_t k = 16; k < nb; k += 8) {
+                unit(t + k, XB_FU_SUM_LO, s + 2 * k - 24);
+                unit(t + k + 4, XB_FU_SUM_HI, s + 2 * k - 24);
+            }
+            break;
+        default:
+            break;
+        }
+        if (a.action != KAGG_ACTION__VREF && nb != 8)
+            infomask |= HEAP_HASVARWIDTH;
+        if (nb)
+            img[offsetof(kern_tupitem, t_bits) + (j >> 3)] |= (uint8_t)(1u << (j & 7));
+        t += nb;
+    }
+    if (t & 3)
+        return;
+    unit(t, XB_FU_ROWID, 0);
+    t += ROWID_SIZE;
+    const uint16_t im2 = (uint16_t)(n & HEAP_NATTS_MASK);
+    put32(0, t);
+    unit(offsetof(kern_tupitem, hash), XB_FU_COPY, offsetof(xb_gent_head, hash));
+    memcpy(img + offsetof(kern_tupitem, t_infomask2), &im2, 2);
+    memcpy(img + offsetof(kern_tupitem, t_infomask), &infomask, 2);
+    img[offsetof(kern_tupitem, t_hoff)] = (uint8_t)(hoff + MINIMAL_TUPLE_OFFSET);
+    pg->nunits = (uint32_t)PGSTROM_MAXALIGN(t) / 4;
+    for (uint32_t u = 0; u < pg->nunits; u++) {
+        pg->unit[u].op = op[u];
+        pg->unit[u].src = src[u];
+        memcpy(&pg->unit[u].imm, img + 4 * u, 4);
+    }
+    pg->item = (uint32_t)PGSTROM_MAXALIGN((row_fmt ? 0 : offsetof(kern_hashitem, t)) + t);
+}
+
+/* for tests: the item bytes of the session's program (0: none) */
+extern "C" uint32_t xb_final_program_item(const xb_plan *plan)
+{
+    XbFinalProg pg;
+    xb_final_program(plan, false, &pg);
+    return pg.nunits ? pg.item : 0;
+}
+
+/* The groups of a session as nparts kds_finals, in two steps: plan() counts
+ * the groups and item bytes of every part, write() puts the parts where the
+ * caller wants them.  Session lock held; work memory is the caller's to
+ * free (tmp). */
+struct XbFinalRun {
+    xpuB200Session *s;
+    const kern_data_store *fh;      /* the session's kds_final definition */
+    uint64_t        head_len = 0;
+    bool            row_fmt = false;
+    std::vector<void *> tmp;
+    XbTileArgs      ta;
+    uint64_t       *d_totals = nullptr;
+    void           *d_temp = nullptr;
+    uint32_t        set0 = UINT32_MAX;      /* the part set counted last */
+    std::vector<uint64_t> totals;           /* groups, item bytes of every part */
+
+    explicit XbFinalRun(xpuB200Session *sess) : s(sess)
+    {
+        const kern_session_info *session = (const kern_session_info *)s->h_session.data();
+        fh = (const kern_data_store *)(s->h_session.data() + session->groupby_kds_final);
+        head_len = KDS_HEAD_LENGTH(fh);
+        row_fmt = fh->format == KDS_FORMAT_ROW;
+    }
+    ~XbFinalRun()
+    {
+        for (void *p : tmp) cudaFreeAsync(p, s->stream);
+    }
+    bool alloc(size_t sz, void **p)
+    {
+        if (cudaMallocAsync(p, sz < 256 ? 256 : sz, s->stream) != cudaSuccess) { cudaGetLastError(); return false; }
+        tmp.push_back(*p);
+        return true;
+    }
+    int grid() const { return (int)std::min<uint64_t>(ta.ntiles, (uint64_t)s->dev->nsm * 8); }
+
+    /* counts and prefixes of the parts from part0 on */
+    bool count(uint32_t part0)
+    {
+        cudaStream_t st = s->stream;
+        ta.part0 = part0;
+        ta.pset = std::min<uint32_t>(ta.nparts - part0, XB_FINAL_PARTS);
+        const uint64_t n = (uint64_t)ta.pset * ta.ntiles;
+        xb_final_tiles<<<grid(), XB_FINAL_TILE, 12 * ta.pset, st>>>(ta);
+        if (n <= 4096) {
+            xb_final_scan_small<<<1, XB_FINAL_TILE, 0, st>>>(ta, (uint32_t *)ta.count_scan, (uint64_t *)ta.bytes_scan,
+                                                              (uint32_t)n);
+        } else if (xb_scan<uint32_t, XbOpSum, true>(ta.count, (uint32_t *)ta.count_scan, n, d_temp, st) != cudaSuccess ||
+                   xb_scan<uint64_t, XbOpSum, true>(ta.bytes, (uint64_t *)ta.bytes_scan, n, d_temp, st) != cudaSuccess) {
+            return false;
+        }
+        xb_final_totals<<<(ta.pset + 255) / 256, 256, 0, st>>>(ta, d_totals + 2 * part0);
+        set0 = part0;
+        return cudaGetLastError() == cudaSuccess;
+    }
+    /* tiles small enough to spread the table over the GPU, and few enough
+     * that the counters of a launch's parts stay small */
+    int plan(uint32_t nparts, kern_errorbuf *err)
+    {
+        cudaStream_t st = s->stream;
+        memset(&ta, 0, sizeof(ta));
+        ta.plan = s->d_plan;
+        ta.gt = s->d_gt;
+        ta.cap = s->h_gt.cap_mask + 1;
+        ta.nparts = nparts;
+        ta.row_format = row_fmt ? 1 : 0;
+        xb_final_program(s->h_plan, row_fmt, &ta.prog);
+        const uint64_t pset = std::min<uint32_t>(nparts, XB_FINAL_PARTS);
+        uint64_t slots = XB_FINAL_TILE;
+        while (pset * ((ta.cap + slots - 1) / slots) > (4ULL << 20))
+            slots *= 2;
+        ta.tile_slots = (uint32_t)slots;
+        ta.ntiles = (uint32_t)((ta.cap + slots - 1) / slots);
+        const uint64_t n = pset * ta.ntiles;
+        if (!alloc(n * 4, (void **)&ta.count) || !alloc(n * 8, (void **)&ta.bytes) ||
+            !alloc(n * 4, (void **)&ta.count_scan) || !alloc(n * 8, (void **)&ta.bytes_scan) ||
+            !alloc(16ULL * nparts, (void **)&d_totals) || !alloc(xb_scan_temp_bytes<uint64_t>(n), &d_temp))
+            return XB_ERR(err, ERRCODE_DEVICE_FATAL, "out of device memory in Final");
+        totals.assign(2 * (size_t)nparts, 0);
+        for (uint32_t p = 0; p < nparts; p += XB_FINAL_PARTS)
+            if (!count(p))
+                return XB_ERR(err, ERRCODE_DEVICE_FATAL, "Final: %s", cudaGetErrorString(cudaGetLastError()));
+        XB_CUDA(cudaMemcpyAsync(totals.data(), d_totals, 16ULL * nparts, cudaMemcpyDeviceToHost, st), err);
+        XB_CUDA(cudaStreamSynchronize(st), err);
+        return 0;
+    }
+    /* the kds_final of part p, at out of the output buffer */
+    XbFinalPart part(uint32_t p, uint64_t out) const
+    {
+        XbFinalPart P;
+        P.out = out;
+        P.nitems = (uint32_t)totals[2 * p];
+        P.nslots = (uint32_t)(row_fmt ? 0 : KDS_GET_HASHSLOT_WIDTH(totals[2 * p]));
+        P.items_base = head_len + 8ULL * P.nslots + 8ULL * P.nitems;
+        P.length = P.items_base + totals[2 * p + 1];
+        return P;
+    }
+    int write(char *out, const std::vector<XbFinalPart> &parts, kern_errorbuf *err)
+    {
+        cudaStream_t st = s->stream;
+        const kern_session_info *session = (const kern_session_info *)s->h_session.data();
+        XbFinalPart *d_parts = nullptr;
+        uint64_t *d_head = nullptr;
+        if (!alloc(sizeof(XbFinalPart) * parts.size(), (void **)&d_parts) || !alloc(head_len, (void **)&d_head))
+            return XB_ERR(err, ERRCODE_DEVICE_FATAL, "out of device memory in Final");
+        XB_CUDA(cudaMemcpyAsync(d_parts, parts.data(), sizeof(XbFinalPart) * parts.size(), cudaMemcpyHostToDevice, st), err);
+        XB_CUDA(cudaMemcpyAsync(d_head, s->d_session + session->groupby_kds_final, head_len,
+                                cudaMemcpyDeviceToDevice, st), err);
+        ta.out = out;
+        for (uint32_t p0 = 0; p0 < ta.nparts; p0 += XB_FINAL_PARTS) {
+            if (set0 != p0 && !count(p0))
+                return XB_ERR(err, ERRCODE_DEVICE_FATAL, "Final: %s", cudaGetErrorString(cudaGetLastError()));
+            ta.part = d_parts + p0;
+            uint64_t most = 0;
+            for (uint32_t p = p0; p < p0 + ta.pset; p++)
+                most = std::max<uint64_t>(most, parts[p].nslots);
+            const unsigned gx = (unsigned)std::min<uint64_t>((head_len / 8 + most + 255) / 256, 1024);
+            xb_final_heads<<<dim3(gx, ta.pset), 256, 0, st>>>(out, ta.part, d_head, (uint32_t)head_len, ta.row_format);
+            xb_final_fill<<<grid(), XB_FINAL_TILE, ta.nparts > 1 ? 16 * ta.pset : 0, st>>>(ta);
+        }
+        cudaError_t rc = cudaGetLastError();
+        if (rc != cudaSuccess)
+            return XB_ERR(err, ERRCODE_DEVICE_FATAL, "Final: %s", cudaGetErrorString(rc));
+        return 0;
+    }
+};
+
+/* kds_final of a session with GPU-Sort keys */
+static int xb_final_sorted(xpuB200Session *s, void *kds_final_buf, uint64_t buf_sz, uint64_t *p_required,
+                           kern_exec_results *results, kern_errorbuf *err);
+
 extern "C" int
 xpuB200Final(xpuB200Session *s, void *kds_final_buf, uint64_t buf_sz, uint64_t *p_required,
              kern_exec_results *results, kern_errorbuf *err)
@@ -155,6 +406,40 @@ xpuB200Final(xpuB200Session *s, void *kds_final_buf, uint64_t buf_sz, uint64_t *
     /* groups waiting in the dump region join the table first */
     int src = xb_gt_settle(s, err);
     if (src) return src;
+    if (plan->nsort)
+        return xb_final_sorted(s, kds_final_buf, buf_sz, p_required, results, err);
+    XbFinalRun run(s);
+    int rc = run.plan(1, err);
+    if (rc) return rc;
+    const XbFinalPart P = run.part(0, 0);
+    if (p_required) *p_required = P.length;
+    if (results) {
+        results->final_nitems = P.nitems;
+        results->final_usage = P.length - P.items_base;
+        results->final_total = P.length;
+    }
+    if (!kds_final_buf || buf_sz < P.length) {
+        if (!kds_final_buf && buf_sz == 0)
+            return 0;           /* size query only */
+        return XB_ERR(err, ERRCODE_SUSPEND_NO_SPACE, "kds_final needs %llu bytes (buffer %llu)",
+                      (unsigned long long)P.length, (unsigned long long)buf_sz);
+    }
+    char *d_out = nullptr;
+    if (!run.alloc(P.length, (void **)&d_out))
+        return XB_ERR(err, ERRCODE_DEVICE_FATAL, "out of device memory for kds_final (%llu bytes)",
+                      (unsigned long long)P.length);
+    rc = run.write(d_out, std::vector<XbFinalPart>(1, P), err);
+    if (rc) return rc;
+    cudaMemcpyAsync(kds_final_buf, d_out, P.length, cudaMemcpyDeviceToHost, st);
+    if (cudaStreamSynchronize(st) != cudaSuccess)
+        return XB_ERR(err, ERRCODE_DEVICE_FATAL, "Final: %s", cudaGetErrorString(cudaGetLastError()));
+    return 0;
+}
+
+static int xb_final_sorted(xpuB200Session *s, void *kds_final_buf, uint64_t buf_sz, uint64_t *p_required,
+                           kern_exec_results *results, kern_errorbuf *err)
+{
+    cudaStream_t st = s->stream;
     const kern_session_info *session = (const kern_session_info *)s->h_session.data();
     const kern_data_store *fh = (const kern_data_store *)(s->h_session.data() + session->groupby_kds_final);
     const uint64_t head_len = KDS_HEAD_LENGTH(fh);
@@ -189,15 +474,13 @@ xpuB200Final(xpuB200Session *s, void *kds_final_buf, uint64_t buf_sz, uint64_t *
     fa.flag_scan = d_flag_scan;
     fa.row_format = row_fmt ? 1 : 0;
     int grid = s->dev->nsm * 8;
-    if (plan->nsort) {
-        int64_t *d_keep = nullptr;
-        if (xb_final_sort(s, fa, st, alloc, &d_keep) != 0) {
-            cleanup();
-            return XB_ERR(err, ERRCODE_DEVICE_FATAL, "GPU-Sort of the groups failed (%s)",
-                          cudaGetErrorString(cudaGetLastError()));
-        }
-        fa.keep = d_keep;
+    int64_t *d_keep = nullptr;
+    if (xb_final_sort(s, fa, st, alloc, &d_keep) != 0) {
+        cleanup();
+        return XB_ERR(err, ERRCODE_DEVICE_FATAL, "GPU-Sort of the groups failed (%s)",
+                      cudaGetErrorString(cudaGetLastError()));
     }
+    fa.keep = d_keep;
     /* the global table's entries pointer lives in h_gt */
     xb_final_sizes<<<grid, XB_BLOCK, 0, st>>>(fa);
     if (!alloc(xb_scan_temp_bytes<uint64_t>(cap), &d_temp)) {
@@ -360,111 +643,28 @@ xpuB200FinalParts(xpuB200Session *s, uint32_t nparts, void *parts_dev, uint64_t 
         return XB_ERR(err, ERRCODE_DEVICE_ERROR, "GPU-Sort applies to the merged groups, not to their parts");
     int rc = xb_gt_settle(s, err);
     if (rc) return rc;
-    cudaStream_t st = s->stream;
-    const kern_session_info *session = (const kern_session_info *)s->h_session.data();
-    const kern_data_store *fh = (const kern_data_store *)(s->h_session.data() + session->groupby_kds_final);
-    const uint64_t head_len = KDS_HEAD_LENGTH(fh);
-    const uint64_t cap = s->h_gt.cap_mask + 1;
-    std::vector<void *> tmp;
-    auto cleanup = [&]() { for (void *p : tmp) cudaFreeAsync(p, st); };
-    auto alloc = [&](size_t sz, void **p) -> bool {
-        if (cudaMallocAsync(p, sz < 256 ? 256 : sz, st) != cudaSuccess) { cudaGetLastError(); return false; }
-        tmp.push_back(*p);
-        return true;
-    };
-    uint64_t *d_sizes, *d_size_scan;
-    uint32_t *d_flags, *d_flag_scan;
-    void *d_temp = nullptr;
-    if (!alloc(cap * 8, (void **)&d_sizes) || !alloc(cap * 8, (void **)&d_size_scan) ||
-        !alloc(cap * 4, (void **)&d_flags) || !alloc(cap * 4, (void **)&d_flag_scan)) {
-        cleanup();
-        return XB_ERR(err, ERRCODE_DEVICE_FATAL, "out of device memory in FinalParts");
-    }
-    const size_t tsz_max = xb_scan_temp_bytes<uint64_t>(cap);
-    if (!alloc(tsz_max, &d_temp)) {
-        cleanup();
-        return XB_ERR(err, ERRCODE_DEVICE_FATAL, "out of device memory in FinalParts");
-    }
-    XbFinalArgs fa;
-    memset(&fa, 0, sizeof(fa));
-    fa.plan = s->d_plan;
-    fa.gt = s->d_gt;
-    fa.cap = cap;
-    fa.sizes = d_sizes;
-    fa.flags = d_flags;
-    fa.size_scan = d_size_scan;
-    fa.flag_scan = d_flag_scan;
-    fa.part_div = nparts;
-    const int grid = s->dev->nsm * 8;
-    /* sizes of part p (its items and groups) into the arrays */
-    auto size_part = [&](uint32_t p, uint64_t *p_items, uint64_t *p_groups) -> int {
-        fa.part_rem = p;
-        xb_final_sizes<<<grid, XB_BLOCK, 0, st>>>(fa);
-        xb_scan<uint64_t, XbOpSum, true>(d_sizes, d_size_scan, cap, d_temp, st);
-        xb_scan<uint32_t, XbOpSum, true>(d_flags, d_flag_scan, cap, d_temp, st);
-        uint64_t last_size = 0, last_scan = 0;
-        uint32_t last_flag = 0, last_fscan = 0;
-        cudaMemcpyAsync(&last_size, d_sizes + cap - 1, 8, cudaMemcpyDeviceToHost, st);
-        cudaMemcpyAsync(&last_scan, d_size_scan + cap - 1, 8, cudaMemcpyDeviceToHost, st);
-        cudaMemcpyAsync(&last_flag, d_flags + cap - 1, 4, cudaMemcpyDeviceToHost, st);
-        cudaMemcpyAsync(&last_fscan, d_flag_scan + cap - 1, 4, cudaMemcpyDeviceToHost, st);
-        if (cudaStreamSynchronize(st) != cudaSuccess)
-            return -1;
-        *p_items = last_scan + last_size;
-        *p_groups = (uint64_t)last_fscan + last_flag;
-        return 0;
-    };
-    std::vector<uint64_t> items(nparts), groups(nparts);
+    XbFinalRun run(s);
+    rc = run.plan(nparts, err);
+    if (rc) return rc;
+    std::vector<XbFinalPart> parts;
     uint64_t total = 0;
     for (uint32_t p = 0; p < nparts; p++) {
-        if (size_part(p, &items[p], &groups[p]) != 0) {
-            cleanup();
-            return XB_ERR(err, ERRCODE_DEVICE_FATAL, "FinalParts: %s", cudaGetErrorString(cudaGetLastError()));
-        }
-        const uint64_t nslots = KDS_GET_HASHSLOT_WIDTH(groups[p]);
+        parts.push_back(run.part(p, total));
         part_offsets[p] = total;
-        total += xb_align256(head_len + 8 * nslots + 8 * groups[p] + items[p]);
+        total += xb_align256(parts[p].length);
     }
     part_offsets[nparts] = total;
     if (p_required) *p_required = total;
     if (!parts_dev || buf_sz < total) {
-        cleanup();
         if (!parts_dev && buf_sz == 0)
             return 0;           /* size query only */
         return XB_ERR(err, ERRCODE_SUSPEND_NO_SPACE, "the parts need %llu bytes (buffer %llu)",
                       (unsigned long long)total, (unsigned long long)buf_sz);
     }
-    std::vector<char> head((const char *)fh, (const char *)fh + head_len);
-    for (uint32_t p = 0; p < nparts; p++) {
-        uint64_t it, ng;
-        if (size_part(p, &it, &ng) != 0) {
-            cleanup();
-            return XB_ERR(err, ERRCODE_DEVICE_FATAL, "FinalParts: %s", cudaGetErrorString(cudaGetLastError()));
-        }
-        const uint64_t nslots = KDS_GET_HASHSLOT_WIDTH(ng);
-        const uint64_t items_base = head_len + 8 * nslots + 8 * ng;
-        const uint64_t length = items_base + it;
-        char *d_out = (char *)parts_dev + part_offsets[p];
-        kern_data_store *kh = (kern_data_store *)head.data();
-        kh->length = length;
-        kh->usage = it;
-        kh->nitems = (uint32_t)ng;
-        kh->format = KDS_FORMAT_HASH;
-        kh->hash_nslots = (uint32_t)nslots;
-        cudaMemcpyAsync(d_out, head.data(), head_len, cudaMemcpyHostToDevice, st);
-        cudaMemsetAsync(d_out + head_len, 0, length - head_len, st);
-        fa.kds_final = d_out;
-        fa.items_base = items_base;
-        fa.length = length;
-        fa.nslots = (uint32_t)nslots;
-        xb_final_write<<<grid, XB_BLOCK, 0, st>>>(fa);
-        /* the host header copy must outlive the copy: wait per part */
-        if (cudaStreamSynchronize(st) != cudaSuccess) {
-            cleanup();
-            return XB_ERR(err, ERRCODE_DEVICE_FATAL, "FinalParts: %s", cudaGetErrorString(cudaGetLastError()));
-        }
-    }
-    cleanup();
+    rc = run.write((char *)parts_dev, parts, err);
+    if (rc) return rc;
+    if (cudaStreamSynchronize(s->stream) != cudaSuccess)
+        return XB_ERR(err, ERRCODE_DEVICE_FATAL, "FinalParts: %s", cudaGetErrorString(cudaGetLastError()));
     return 0;
 }
 

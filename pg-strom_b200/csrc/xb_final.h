@@ -40,6 +40,58 @@ struct XbFinalArgs {
                                      * (nullptr: every group, in table order) */
 };
 
+/* the tuple of a group whose size and attribute offsets are the plan's
+ * alone (every key fixed-width of 4 or 8 bytes, none NULL), as 4-byte
+ * units: what each one is made of */
+enum {
+    XB_FU_CONST = 0,                /* imm */
+    XB_FU_COPY,                     /* 4 bytes of the entry */
+    XB_FU_ROWID,
+    XB_FU_SUM_LO, XB_FU_SUM_HI,     /* float8 sum + its compensation */
+    XB_FU_MM_ATTRS,                 /* min/max: valid flag */
+    XB_FU_MMFP_LO, XB_FU_MMFP_HI,   /* float8 min (imm 0) / max (imm 1) */
+    XB_FU_NUM_ATTRS,                /* numeric: imm | special flags */
+    XB_FU_FLT4,                     /* float8 image of a float4 key */
+};
+#define XB_FINAL_UNITS  128
+struct XbFinalProg {
+    uint32_t        nunits;         /* even; 0: the plan has no fixed tuple */
+    uint32_t        item;           /* bytes of an item, hash link included */
+    struct { uint16_t op, src; uint32_t imm; } unit[XB_FINAL_UNITS];
+};
+
+/* one hash partition of the groups, being written as a kds_final */
+struct XbFinalPart {
+    uint64_t        out;            /* its start in the output buffer */
+    uint64_t        items_base;     /* offset of the first item in the part */
+    uint64_t        length;
+    uint32_t        nslots;
+    uint32_t        nitems;
+};
+
+/* kds_final by tiles of the group table: the groups and item bytes of
+ * every (part, tile), then the tuples (xb_final_tiles, xb_final_fill) */
+#define XB_FINAL_TILE   256
+#define XB_FINAL_PARTS  1024        /* parts of one launch (their counters are in shared memory) */
+struct XbTileArgs {
+    const xb_plan  *plan;
+    const xb_gtable *gt;
+    uint64_t        cap;
+    uint32_t        tile_slots;     /* a multiple of XB_FINAL_TILE */
+    uint32_t        ntiles;
+    uint32_t        nparts;         /* of all: part = hash % nparts */
+    uint32_t        part0;          /* the parts [part0, part0 + pset) are this launch's */
+    uint32_t        pset;
+    uint32_t        row_format;
+    uint32_t       *count;          /* [(part - part0) * ntiles + tile] */
+    uint64_t       *bytes;
+    const uint32_t *count_scan;     /* exclusive prefixes of the two, over all parts */
+    const uint64_t *bytes_scan;
+    char           *out;
+    const XbFinalPart *part;
+    XbFinalProg     prog;
+};
+
 /* GPU-Sort: the sort keys of the ready groups, as radix words */
 struct XbSortArgs {
     const xb_plan  *plan;
@@ -99,6 +151,13 @@ struct XbRebuildArgs {
 /* the kernels (xb_exec.cu) */
 __global__ void xb_final_sizes(XbFinalArgs args);
 __global__ void xb_final_write(XbFinalArgs args);
+__global__ void __launch_bounds__(XB_FINAL_TILE) xb_final_tiles(const __grid_constant__ XbTileArgs a);
+__global__ void __launch_bounds__(XB_FINAL_TILE) xb_final_scan_small(XbTileArgs a, uint32_t *count_scan,
+                                                                      uint64_t *bytes_scan, uint32_t n);
+__global__ void xb_final_totals(XbTileArgs a, uint64_t *totals);
+__global__ void xb_final_heads(char *out, const XbFinalPart *part, const uint64_t *head, uint32_t head_len,
+                               uint32_t row_format);
+__global__ void __launch_bounds__(XB_FINAL_TILE) xb_final_fill(const __grid_constant__ XbTileArgs a);
 __global__ void xb_sort_gather(XbSortArgs a);
 __global__ void xb_sort_keys(XbSortArgs a);
 __global__ void xb_sort_pass_key64(const uint64_t *col, const uint32_t *idx, uint64_t *out, uint32_t n);
