@@ -4396,6 +4396,35 @@ xpuB200SessionInfo(xpuB200Session *s, char *buf, uint64_t buf_sz)
     return 0;
 }
 
+/* the word-wise byte functions of the kernels, for the host-side tests */
+extern "C" uint32_t xb_hash_words_of(const void *data, uint32_t len)
+{
+    return xb_hash_words((const uint8_t *)data, len);
+}
+
+extern "C" int xb_words_eq_of(const void *a, const void *b, uint32_t len)
+{
+    return xb_words_eq((const uint8_t *)a, (const uint8_t *)b, len);
+}
+
+/* the value of a numeric for a sum of scale weight, by the kernels'
+ * function (general == 0) or by the general decode and rescale */
+extern "C" int xb_numeric_sum_of(const void *vl, int weight, int general, uint8_t *kind, uint64_t *lo, uint64_t *hi)
+{
+    xb_i128 v = 0;
+    int rc;
+    if (general) {
+        int16_t w = 0;
+        rc = xb_numeric_decode((const uint8_t *)vl, kind, &w, &v);
+        v = !rc && *kind == XB_NUM_VALID ? xb_numeric_rescale(weight, w, v) : 0;
+    } else {
+        rc = xb_numeric_sum_value((const uint8_t *)vl, weight, kind, &v);
+    }
+    *lo = (uint64_t)v;
+    *hi = (uint64_t)((unsigned __int128)v >> 64);
+    return rc != 0;
+}
+
 extern "C" uint32_t
 xpuB200HashBytes(const void *data, uint32_t len)
 {

@@ -19,7 +19,7 @@
 #define XB_ROWS_UNIT    1024        /* rows per unit for ARROW / ROW chunks */
 #define XB_MIN_BLOCKS   2           /* resident CTAs per SM the kernel is built for */
 #define XB_PROBE_LIMIT  4096        /* max probes in the global group table */
-#define XB_SM_PROBES    8           /* max probes in a CTA's shared group table: a group that
+#define XB_SM_PROBES    32          /* max probes in a CTA's shared group table: a group that
                                      * finds no entry in reach goes to the global table (with
                                      * the whole table searched, every row of such a group
                                      * read all of it: a query over 2M rows with 1000 groups
@@ -222,85 +222,6 @@ __device__ __forceinline__ double xb_reg_f64(uint64_t v, int rk)
     return rk == XB_RK_FLT ? __longlong_as_double(v) : (double)(int64_t)v;
 }
 
-/* 10^k for k = 0..18 */
-__device__ __forceinline__ int64_t xb_pow10_i64(int k)
-{
-    int64_t p = 1;
-    for (int i = 0; i < k; i++)
-        p *= 10;
-    return p;
-}
-
-/*
- * The value of a numeric varlena rescaled to weight_d, for sums: the same
- * number as xb_numeric_rescale(weight_d, w, v) of xb_numeric_decode, which
- * normalises trailing zeros away first; rescaling the digits as stored
- * gives the same result (the removed digits are zeros).  Short numerics of
- * up to four base-10000 digits are read with aligned 8-byte loads (every
- * aligned word that overlaps the datum lies in its page or buffer) and
- * rescaled in 64-bit arithmetic; others take the general decode.
- * Returns 0, or 1 on a corrupt datum.
- */
-__device__ __forceinline__ int
-xb_numeric_sum_value(const uint8_t *vl, int weight_d, uint8_t *p_kind, xb_i128 *p_out)
-{
-    const uintptr_t a = (uintptr_t)vl;
-    const uint64_t *wp = (const uint64_t *)(a & ~(uintptr_t)7);
-    const uint32_t o = (uint32_t)(a & 7);
-    const uint64_t w0 = wp[0];
-    const uint32_t h = (uint32_t)(w0 >> (8 * o)) & 0xff;
-    const uint32_t len = (h >> 1) & 0x7f;
-    /* short varlena, short-format numeric, 0..4 digits, within 3 words */
-    if ((h & 1) && h != 1 && len >= 3 && len <= 11 && o + len <= 24) {
-        const uint64_t w1 = (o + len > 8) ? wp[1] : 0;
-        const uint64_t w2 = (o + len > 16) ? wp[2] : 0;
-        auto byte = [&](uint32_t i) -> uint32_t {
-            const uint32_t k = o + i;
-            const uint64_t w = k < 8 ? w0 : (k < 16 ? w1 : w2);
-            return (uint32_t)(w >> (8 * (k & 7))) & 0xff;
-        };
-        const uint32_t n_head = byte(1) | (byte(2) << 8);
-        if ((n_head & 0xC000) == 0x8000 && ((len - 3) & 1) == 0) {
-            const uint32_t ndigits = (len - 3) / 2;
-            int pgweight = n_head & 0x003F;
-            if (n_head & 0x0040)
-                pgweight |= ~0x003F;
-            int64_t v = 0;
-            for (uint32_t i = 0; i < ndigits; i++)
-                v = v * 10000 + (int16_t)(byte(3 + 2 * i) | (byte(4 + 2 * i) << 8));
-            if (n_head & 0x2000)
-                v = -v;
-            const int weight_s = 4 * ((int)ndigits - (pgweight + 1));
-            const int shift = weight_d - weight_s;
-            if (shift == 0 || v == 0) {
-                *p_kind = XB_NUM_VALID;
-                *p_out = v;
-                return 0;
-            }
-            if (shift < 0 && shift >= -18) {
-                *p_kind = XB_NUM_VALID;
-                *p_out = v / xb_pow10_i64(-shift);       /* truncates toward zero */
-                return 0;
-            }
-            if (shift > 0 && shift <= 18) {
-                const int64_t p = xb_pow10_i64(shift);
-                const uint64_t m = v < 0 ? (uint64_t)(-(v + 1)) + 1 : (uint64_t)v;
-                if (m <= (uint64_t)INT64_MAX / (uint64_t)p) {
-                    *p_kind = XB_NUM_VALID;
-                    *p_out = v * p;
-                    return 0;
-                }
-            }
-        }
-    }
-    int16_t w;
-    xb_i128 v;
-    if (xb_numeric_decode(vl, p_kind, &w, &v))
-        return 1;
-    *p_out = (*p_kind == XB_NUM_VALID) ? xb_numeric_rescale(weight_d, w, v) : 0;
-    return 0;
-}
-
 /* state flag of a numeric that is not a number's digits */
 __device__ __forceinline__ uint32_t xb_numeric_special(uint8_t kind)
 {
@@ -311,12 +232,9 @@ __device__ __forceinline__ uint32_t xb_numeric_special(uint8_t kind)
 
 /* per-value updates of the actions that are not combined across lanes */
 __device__ __forceinline__ void
-xb_agg_numeric_add(char *s, const uint8_t *vl, int16_t weight, xb_status *st)
+xb_agg_numeric_put(char *s, uint8_t kind, xb_i128 v)
 {
-    uint8_t kind; xb_i128 v;
-    if (xb_numeric_sum_value(vl, weight, &kind, &v)) {
-        XB_RAISE(st, ERRCODE_DEVICE_ERROR, XB_MSG_NUMERIC_CORRUPT);
-    } else if (kind == XB_NUM_VALID) {
+    if (kind == XB_NUM_VALID) {
         atomicAdd((unsigned long long *)s, 1ULL);
         xb_atomic_add_i128((uint64_t *)(s + 8), v);
     } else {
@@ -324,16 +242,35 @@ xb_agg_numeric_add(char *s, const uint8_t *vl, int16_t weight, xb_status *st)
     }
 }
 
-/* xb_agg_numeric_add for an entry of a shared-memory group table (shared
+__device__ __forceinline__ void
+xb_agg_numeric_add(char *s, const uint8_t *vl, int16_t weight, xb_status *st)
+{
+    uint8_t kind; xb_i128 v;
+    if (xb_numeric_sum_value(vl, weight, &kind, &v))
+        XB_RAISE(st, ERRCODE_DEVICE_ERROR, XB_MSG_NUMERIC_CORRUPT);
+    else
+        xb_agg_numeric_put(s, kind, v);
+}
+
+/* xb_agg_numeric_put for an entry of the global table (global reductions) */
+__device__ __forceinline__ void
+xb_agg_numeric_put_g(char *s, uint8_t kind, xb_i128 v)
+{
+    if (kind == XB_NUM_VALID) {
+        xb_red_g_add_u64(s, 1ULL);
+        xb_atomic_add_i128_g((uint64_t *)(s + 8), v);
+    } else {
+        xb_red_g_or_u32(s + 24, xb_numeric_special(kind));
+    }
+}
+
+/* xb_agg_numeric_put for an entry of a shared-memory group table (shared
  * form): 32-bit counter, 128-bit sum by word atomics; with nc the counter
  * holds the rows NOT counted (a special value, the caller adds NULLs) */
 __device__ __forceinline__ void
-xb_agg_numeric_add_sm(char *s, const uint8_t *vl, int16_t weight, xb_status *st, bool nc)
+xb_agg_numeric_put_sm(char *s, uint8_t kind, xb_i128 v, bool nc)
 {
-    uint8_t kind; xb_i128 v;
-    if (xb_numeric_sum_value(vl, weight, &kind, &v)) {
-        XB_RAISE(st, ERRCODE_DEVICE_ERROR, XB_MSG_NUMERIC_CORRUPT);
-    } else if (kind == XB_NUM_VALID) {
+    if (kind == XB_NUM_VALID) {
         if (!nc)
             xb_red_shared_add_u32(s, 1u);
         xb_shared_add_i128w(s + 8, v);

@@ -771,7 +771,7 @@ struct Gen {
          * distinct entry with the other lanes idle), so each lane updates
          * its entry directly */
         o << "__device__ __forceinline__ void xbj_update(char *e, const XbjRegs &R, const XbjEnv &E)\n{\n"
-             "    (void)E;\n";
+             "    (void)E;\n" << numeric_args();
         for (uint32_t i = 0; i < p->naggs; i++) {
             const xb_agg &a = p->aggs[i];
             if (a.state_sz == 0)
@@ -785,6 +785,42 @@ struct Gen {
         }
         o << "}\n\n";
         shared_form();
+    }
+
+    /* an update's numeric arguments, each decoded once per scale however
+     * many sums and averages take it (k<r>_<w>: its kind, x<r>_<w>: its
+     * value) */
+    static bool is_numeric_sum(const xb_agg &a)
+    {
+        return a.action == KAGG_ACTION__PSUM_NUMERIC || a.action == KAGG_ACTION__PAVG_NUMERIC;
+    }
+    static std::string num_id(const xb_agg &a)
+    {
+        return std::to_string(a.arg0) + (a.weight < 0 ? "_m" : "_") + std::to_string(a.weight < 0 ? -a.weight : a.weight);
+    }
+    std::string numeric_args() const
+    {
+        std::ostringstream r;
+        std::vector<std::string> seen;
+        for (uint32_t i = 0; i < p->naggs; i++) {
+            const xb_agg &a = p->aggs[i];
+            if (a.state_sz == 0 || !is_numeric_sum(a) ||
+                std::find(seen.begin(), seen.end(), num_id(a)) != seen.end())
+                continue;
+            const std::string id = num_id(a);
+            seen.push_back(id);
+            /* for the rows that any of them counts */
+            std::string any;
+            for (uint32_t k = i; k < p->naggs; k++)
+                if (p->aggs[k].state_sz && is_numeric_sum(p->aggs[k]) && num_id(p->aggs[k]) == id)
+                    any += (any.empty() ? "" : " || ") + agg_expr(p->aggs[k]).c;
+            r << "    uint8_t k" << id << " = XB_NUM_VALID; xb_i128 x" << id << " = 0;\n"
+                 "    if ((" << any << ") && xb_numeric_sum_value((const uint8_t *)" << V(a.arg0) << ", " << a.weight
+              << ", &k" << id << ", &x" << id << ")) {\n"
+                 "        XB_RAISE(E.st, ERRCODE_DEVICE_ERROR, XB_MSG_NUMERIC_CORRUPT);\n"
+                 "        return;\n    }\n";
+        }
+        return r.str();
     }
 
     /* C++ expressions of an aggregate: its filter (f), the condition under
@@ -867,12 +903,10 @@ struct Gen {
                 if (num) {
                     decl << "    uint32_t c" << I << ";\n";
                     init << "    " << c2 << " = 0;\n";
+                    const std::string id = num_id(a);
                     row << "    if (" << x.c << ") {\n"
-                           "        uint8_t kind_; xb_i128 v_;\n"
-                           "        if (xb_numeric_sum_value((const uint8_t *)" << V(a.arg0) << ", " << a.weight
-                        << ", &kind_, &v_)) { XB_RAISE(E.st, ERRCODE_DEVICE_ERROR, XB_MSG_NUMERIC_CORRUPT); }\n"
-                           "        else if (kind_ == XB_NUM_VALID) { " << n << "++; " << s << " += v_; }\n"
-                           "        else " << c2 << " |= xb_numeric_special(kind_);\n    }\n";
+                           "        if (k" << id << " == XB_NUM_VALID) { " << n << "++; " << s << " += x" << id << "; }\n"
+                           "        else " << c2 << " |= xb_numeric_special(k" << id << ");\n    }\n";
                 } else {
                     row << "    if (" << x.c << ") { " << n << "++; " << s << " += (xb_i128)(int64_t)" << V(a.arg0) << "; }\n";
                 }
@@ -932,7 +966,7 @@ struct Gen {
         acc_decl = decl.str();
         o << "__device__ __forceinline__ void xbj_acc_init(XbjAcc &A)\n{\n    A.rows = 0;\n" << init.str() << "}\n\n"
              "__device__ __forceinline__ void xbj_acc_row(XbjAcc &A, const XbjRegs &R, const XbjEnv &E)\n{\n"
-             "    (void)E;\n    A.rows = 1;\n" << row.str() << "}\n\n"
+             "    (void)E;\n    A.rows = 1;\n" << numeric_args() << row.str() << "}\n\n"
              "__device__ __forceinline__ void xbj_acc_put(XbjAcc &A, char *e, const bool leader)\n{\n" << put.str() << "}\n\n"
              /* all lanes of the warp */
              "__device__ __forceinline__ void xbj_acc_flush(XbjAcc &A, const XbjEnv &E)\n{\n"
@@ -1004,7 +1038,7 @@ struct Gen {
     void update_shared(const int R)
     {
         o << "__device__ __forceinline__ void xbj_update_sm(char *e, const XbjRegs &R, const XbjEnv &E)\n{\n"
-             "    (void)E;\n";
+             "    (void)E;\n" << numeric_args();
         for (uint32_t i = 0; i < p->naggs; i++) {
             const xb_agg &a = p->aggs[i];
             if (a.state_sz == 0)
@@ -1052,8 +1086,8 @@ struct Gen {
                 /* the helper counts valid values (or, with nc, special ones) */
                 if (nc)
                     o << "        if (!(" << c << ")) xb_red_shared_add_u32(" << S << ", 1u);\n";
-                o << "        if (" << c << ") xb_agg_numeric_add_sm(" << S << ", (const uint8_t *)" << V(a.arg0) << ", "
-                  << a.weight << ", E.st, " << (nc ? "true" : "false") << ");\n";
+                o << "        if (" << c << ") xb_agg_numeric_put_sm(" << S << ", k" << num_id(a) << ", x" << num_id(a)
+                  << ", " << (nc ? "true" : "false") << ");\n";
                 break;
             case KAGG_ACTION__PMIN_INT32: case KAGG_ACTION__PMIN_INT64: case KAGG_ACTION__PMIN_FP64:
             case KAGG_ACTION__PMAX_INT32: case KAGG_ACTION__PMAX_INT64: case KAGG_ACTION__PMAX_FP64: {
@@ -1162,8 +1196,8 @@ struct Gen {
     {
         switch (a.action) {
         case KAGG_ACTION__PSUM_NUMERIC: case KAGG_ACTION__PAVG_NUMERIC:
-            o << "        if (" << c << ") xb_agg_numeric_add(" << S << ", (const uint8_t *)" << V(a.arg0) << ", "
-              << a.weight << ", E.st);\n";
+            o << "        if (" << c << ") xb_agg_numeric_put_g(" << S << ", k" << num_id(a) << ", x" << num_id(a)
+              << ");\n";
             break;
         case KAGG_ACTION__STDDEV:
             o << "        if (" << c << ") xb_agg_stddev_add(" << S << ", " << xd << ");\n";

@@ -36,27 +36,10 @@ __device__ __forceinline__ void xb_raise(xb_status *st, uint32_t code, uint32_t 
  * text and numeric helpers
  * --------------------------------------------------------------- */
 
-/* byte-string equality; within a 16-byte block the loads are independent
- * (no early exit), so they are issued back to back instead of as a chain */
+/* byte-string equality */
 __device__ __forceinline__ bool xb_bytes_eq(const uint8_t *a, const uint8_t *b, uint32_t n)
 {
-    if (a == b)
-        return true;
-    uint32_t i = 0;
-    for (; i + 16 <= n; i += 16) {
-        uint32_t diff = 0;
-#pragma unroll
-        for (uint32_t k = 0; k < 16; k++)
-            diff |= (uint32_t)(a[i + k] ^ b[i + k]);
-        if (diff)
-            return false;
-    }
-    uint32_t diff = 0;
-#pragma unroll
-    for (uint32_t k = 0; k < 15; k++)
-        if (i + k < n)
-            diff |= (uint32_t)(a[i + k] ^ b[i + k]);
-    return diff == 0;
+    return xb_words_eq(a, b, n) != 0;
 }
 
 static __device__ __noinline__ bool xb_bytes_eq_ool(const uint8_t *a, const uint8_t *b, uint32_t n)
@@ -85,7 +68,7 @@ static __device__ __noinline__ int xb_numeric_cmp(const uint8_t *a, const uint8_
 
 static __device__ __noinline__ uint32_t xb_hash_text_ool(const uint8_t *p, uint32_t len)
 {
-    return xb_hash_bytes(p, len);
+    return xb_hash_words(p, len);
 }
 
 /* returns the hash, or sets *bad on a corrupt numeric */
