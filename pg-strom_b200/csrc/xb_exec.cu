@@ -1326,55 +1326,6 @@ xb_write_group_tuple(const xb_plan *plan, const char *e, kern_tupitem *ti, uint3
     return t_hoff;
 }
 
-__global__ void xb_final_sizes(XbFinalArgs args)
-{
-    const xb_plan *plan = args.plan;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < args.cap;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        const char *e = args.gt->entries + i * plan->gent_size;
-        const xb_gent_head *h = (const xb_gent_head *)e;
-        if (h->state == XB_GSTATE_READY && (!args.keep || args.keep[i] >= 0) &&
-            (args.part_div < 2 || h->hash % args.part_div == args.part_rem)) {
-            uint32_t t_len = xb_write_group_tuple(plan, e, nullptr, 0);
-            args.sizes[i] = PGSTROM_MAXALIGN((args.row_format ? 0 : offsetof(kern_hashitem, t)) + t_len);
-            args.flags[i] = 1;
-        } else {
-            args.sizes[i] = 0;
-            args.flags[i] = 0;
-        }
-    }
-}
-
-__global__ void xb_final_write(XbFinalArgs args)
-{
-    const xb_plan *plan = args.plan;
-    kern_data_store *kds = (kern_data_store *)args.kds_final;
-    uint64_t *hslots = (uint64_t *)(args.kds_final + KDS_HEAD_LENGTH(kds));
-    uint64_t *rowindex = hslots + args.nslots;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < args.cap;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        if (!args.flags[i])
-            continue;
-        const char *e = args.gt->entries + i * plan->gent_size;
-        const uint32_t rank = args.keep ? (uint32_t)args.keep[i] : args.flag_scan[i];
-        const uint64_t item_off = args.items_base + args.size_scan[i];
-        if (args.row_format) {
-            /* KDS_FORMAT_ROW: the tuple itself, found through the row index */
-            kern_tupitem *ti = (kern_tupitem *)(args.kds_final + item_off);
-            xb_write_group_tuple(plan, e, ti, rank);
-            rowindex[rank] = args.length - item_off;
-            continue;
-        }
-        kern_hashitem *hitem = (kern_hashitem *)(args.kds_final + item_off);
-        xb_write_group_tuple(plan, e, &hitem->t, rank);
-        rowindex[rank] = args.length - (item_off + offsetof(kern_hashitem, t));
-        const uint32_t hash = ((const xb_gent_head *)e)->hash;
-        unsigned long long mine = args.length - item_off;
-        unsigned long long prev = atomicExch((unsigned long long *)&hslots[hash % args.nslots], mine);
-        hitem->next = prev;
-    }
-}
-
 /* ----------------------------------------------------------------
  * kds_final by tiles of the group table
  *
@@ -1434,7 +1385,7 @@ xb_final_tiles(const __grid_constant__ XbTileArgs a)
         uint32_t n = 0;
         const uint64_t s0 = (uint64_t)tile * a.tile_slots;
         for (uint64_t i = s0 + threadIdx.x; i < s0 + a.tile_slots && i < a.cap; i += blockDim.x) {
-            const char *e = entries + i * gsz;
+            const char *e = entries + (a.list ? a.list[i] : i) * gsz;
             const xb_gent_head h = *(const xb_gent_head *)e;
             const int p = h.state == XB_GSTATE_READY ? xb_final_part(a, h.hash) : -1;
             if (p < 0)
@@ -1558,7 +1509,8 @@ xb_final_fill(const __grid_constant__ XbTileArgs a)
     uint32_t *groups = (uint32_t *)(odd_bytes + a.pset), *fasts = groups + a.pset;
     __shared__ uint64_t prog[XB_FINAL_UNITS];
     __shared__ uint64_t item[XB_FINAL_TILE];    /* place of the group's item in the output buffer */
-    __shared__ uint32_t slot[XB_FINAL_TILE];    /* its entry; bit 31: not the program's tuple */
+    __shared__ uint32_t slot[XB_FINAL_TILE];    /* its entry (tables have below 2^31); bit 31: not
+                                                 * the program's tuple */
     __shared__ uint32_t rowid[XB_FINAL_TILE];
     __shared__ uint32_t nlist;
     const uint32_t gsz = a.plan->gent_size, nkeys = a.plan->nkeys, koff = a.plan->gent_keys_off;
@@ -1577,7 +1529,8 @@ xb_final_fill(const __grid_constant__ XbTileArgs a)
         const uint64_t s0 = (uint64_t)tile * a.tile_slots;
         for (uint32_t sub = 0; sub < a.tile_slots && s0 + sub < a.cap; sub += XB_FINAL_TILE) {
             const uint64_t i = s0 + sub + threadIdx.x;
-            const char *e = entries + i * gsz;
+            const uint64_t ent = i >= a.cap ? 0 : a.list ? a.list[i] : i;
+            const char *e = entries + ent * gsz;
             xb_gent_head h;
             h.hash = 0;
             h.state = XB_GSTATE_EMPTY;
@@ -1626,7 +1579,7 @@ xb_final_fill(const __grid_constant__ XbTileArgs a)
                         atomicExch((unsigned long long *)&hslots[h.hash % P.nslots],
                                    (unsigned long long)(P.length - rel));
                 item[at] = P.out + rel + link;
-                slot[at] = (uint32_t)(i - s0) | (fast ? 0 : 0x80000000u);
+                slot[at] = (uint32_t)ent | (fast ? 0 : 0x80000000u);
                 rowid[at] = rank;
                 if (!fast) {
                     char *t = out + rel + link;
@@ -1640,7 +1593,7 @@ xb_final_fill(const __grid_constant__ XbTileArgs a)
                 const uint32_t j = k / words, w = k - j * words;
                 if (slot[j] & 0x80000000u)
                     continue;
-                const char *ej = entries + (s0 + slot[j]) * gsz;
+                const char *ej = entries + (uint64_t)slot[j] * gsz;
                 const uint64_t u0 = prog[2 * w], u1 = prog[2 * w + 1];
                 const uint32_t lo = xb_final_unit(ej, (uint32_t)u0 & 0xffff, (uint32_t)u0 >> 16, u0 >> 32, rowid[j]);
                 const uint32_t hi = xb_final_unit(ej, (uint32_t)u1 & 0xffff, (uint32_t)u1 >> 16, u1 >> 32, rowid[j]);
@@ -1676,12 +1629,147 @@ __device__ __forceinline__ uint64_t xb_sort_f64(double d)
     return (b >> 63) ? ~b : (b | (1ULL << 63));
 }
 
-__global__ void xb_sort_gather(XbSortArgs a)
+/* the entries of the groups, in table order (one part, counted) */
+__global__ void __launch_bounds__(XB_FINAL_TILE)
+xb_final_ents(const __grid_constant__ XbTileArgs a, uint32_t *ents)
 {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < a.cap;
-         i += (uint64_t)gridDim.x * blockDim.x)
-        if (a.flags[i])
-            a.ents[a.flag_scan[i]] = (uint32_t)i;
+    const uint32_t gsz = a.plan->gent_size;
+    const char *entries = a.gt->entries;
+    for (uint32_t tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x) {
+        const uint64_t s0 = (uint64_t)tile * a.tile_slots;
+        uint32_t n0 = a.count_scan[tile];
+        for (uint32_t sub = 0; sub < a.tile_slots && s0 + sub < a.cap; sub += XB_FINAL_TILE) {
+            const uint64_t i = s0 + sub + threadIdx.x;
+            const uint32_t ready = i < a.cap && ((const xb_gent_head *)(entries + i * gsz))->state == XB_GSTATE_READY;
+            uint32_t tot;
+            const uint32_t at = xb_block_scan_incl<uint32_t, XbOpSum>(ready, &tot) - ready;
+            if (ready)
+                ents[n0 + at] = (uint32_t)i;
+            n0 += tot;
+        }
+    }
+}
+
+/* ---- LIMIT n: the groups that can be among the first n ----------------
+ * Sorting every group to keep a thousand of them took 18 radix passes over
+ * all of them (1.7M groups, two keys: 1.75 ms of Final, 0.57 ms now); four
+ * digits of the first key pick the few that one CTA then sorts. */
+__device__ __forceinline__ uint64_t xb_top_word(const XbTopArgs &a, uint32_t r)
+{
+    return ((uint64_t)a.nul[r] << 63) | (a.hi[r] >> 1);
+}
+
+__global__ void xb_top_hist(XbTopArgs a, uint32_t digit)
+{
+    __shared__ uint32_t h[XB_TOP_BINS];
+    for (uint32_t i = threadIdx.x; i < XB_TOP_BINS; i += blockDim.x)
+        h[i] = 0;
+    __syncthreads();
+    const uint64_t prefix = a.prefix[0];
+    const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t r0 = blockIdx.x * blockDim.x; r0 < a.n; r0 += stride) {
+        const uint32_t r = r0 + threadIdx.x;
+        uint32_t bin = XB_TOP_BINS;
+        if (r < a.n) {
+            const uint64_t w = xb_top_word(a, r);
+            if (digit == 0 || (w >> (64 - 11 * digit)) == prefix)
+                bin = (uint32_t)(w >> (53 - 11 * digit)) & (XB_TOP_BINS - 1);
+        }
+        /* leading digits of one kind of value are few: one add per kind */
+        const uint32_t peers = __match_any_sync(XB_FULL, bin);
+        if (bin < XB_TOP_BINS && (uint32_t)(__ffs(peers) - 1) == (threadIdx.x & 31))
+            atomicAdd(&h[bin], (uint32_t)__popc(peers));
+    }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < XB_TOP_BINS; i += blockDim.x)
+        if (h[i])
+            atomicAdd(&a.hist[digit * XB_TOP_BINS + i], h[i]);
+}
+
+/* the digit at which the groups wanted are reached */
+__global__ void __launch_bounds__(XB_SCAN_BLOCK)
+xb_top_select(XbTopArgs a, uint32_t digit)
+{
+    const uint32_t per = XB_TOP_BINS / XB_SCAN_BLOCK;
+    const uint32_t *h = a.hist + digit * XB_TOP_BINS + threadIdx.x * per;
+    const uint64_t prefix = digit ? a.prefix[0] : 0, want = a.prefix[1];
+    uint64_t sum = 0, tot;
+    for (uint32_t k = 0; k < per; k++)
+        sum += h[k];
+    uint64_t before = xb_block_scan_incl<uint64_t, XbOpSum>(sum, &tot) - sum;
+    if (before < want && before + sum >= want) {
+        uint32_t k = 0;
+        while (before + h[k] < want)
+            before += h[k++];
+        a.prefix[0] = (prefix << 11) | (threadIdx.x * per + k);
+        a.prefix[1] = want - before;
+    }
+}
+
+__global__ void xb_top_gather(XbTopArgs a)
+{
+    const uint64_t prefix = a.prefix[0];
+    for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < a.n; r += gridDim.x * blockDim.x)
+        if ((xb_top_word(a, r) >> (64 - 11 * XB_TOP_DIGITS)) <= prefix) {
+            const uint32_t p = atomicAdd(a.ncand, 1u);
+            if (p < XB_SORT_SMALL)
+                a.cand[p] = r;
+        }
+}
+
+/* the m <= XB_SORT_SMALL groups cand[] (nullptr: all of them) in sort
+ * order, groups of equal keys by rank: a bitonic network over (leading
+ * bits, rank) in shared memory, the rest of the keys read on ties */
+__global__ void __launch_bounds__(1024)
+xb_sort_small(XbSortArgs a, const uint32_t *cand, uint32_t m, uint32_t *idx)
+{
+    __shared__ uint64_t lead[XB_SORT_SMALL];
+    __shared__ uint32_t rank[XB_SORT_SMALL];
+    uint32_t size = 2;
+    while (size < m)
+        size <<= 1;
+    for (uint32_t i = threadIdx.x; i < size; i += blockDim.x) {
+        const uint32_t r = i < m ? (cand ? cand[i] : i) : UINT32_MAX;
+        rank[i] = r;
+        lead[i] = r == UINT32_MAX ? UINT64_MAX : ((uint64_t)a.nul[r] << 63) | (a.keyw[r] >> 1);
+    }
+    __syncthreads();
+    const uint32_t nk = a.plan->nsort;
+    auto after = [&](uint32_t i, uint32_t j) -> bool {       /* i sorts after j */
+        if (lead[i] != lead[j])
+            return lead[i] > lead[j];
+        const uint32_t r = rank[i], q = rank[j];
+        if (r == UINT32_MAX || q == UINT32_MAX)
+            return r > q;
+        for (uint32_t k = 0; k < nk; k++) {
+            const uint8_t nr = a.nul[(uint64_t)k * a.n + r], nq = a.nul[(uint64_t)k * a.n + q];
+            if (nr != nq)
+                return nr > nq;
+            for (uint32_t w = 0; w < 2; w++) {
+                const uint64_t x = a.keyw[(2ULL * k + w) * a.n + r], y = a.keyw[(2ULL * k + w) * a.n + q];
+                if (x != y)
+                    return x > y;
+            }
+        }
+        return r > q;
+    };
+    for (uint32_t k = 2; k <= size; k <<= 1)
+        for (uint32_t d = k >> 1; d > 0; d >>= 1) {
+            for (uint32_t t = threadIdx.x; t < size / 2; t += blockDim.x) {
+                const uint32_t i = 2 * t - (t & (d - 1)), j = i + d;
+                if (after(i, j) == ((i & k) == 0)) {
+                    const uint64_t l = lead[i];
+                    const uint32_t r = rank[i];
+                    lead[i] = lead[j];
+                    rank[i] = rank[j];
+                    lead[j] = l;
+                    rank[j] = r;
+                }
+            }
+            __syncthreads();
+        }
+    for (uint32_t i = threadIdx.x; i < m; i += blockDim.x)
+        idx[i] = rank[i];
 }
 
 __global__ void xb_sort_keys(XbSortArgs a)
@@ -1869,10 +1957,12 @@ __global__ void xb_sort_keepflag(XbKeepArgs a)
     }
 }
 
-__global__ void xb_sort_keep(XbKeepArgs a, const uint32_t *keep_scan, int64_t *keep)
+/* the entries of the groups kept, in order */
+__global__ void xb_sort_keep(XbKeepArgs a, const uint32_t *keep_scan, uint32_t *list)
 {
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < a.n; p += gridDim.x * blockDim.x)
-        keep[a.ents[a.idx[p]]] = a.keep_flag[p] ? (int64_t)keep_scan[p] : -1;
+        if (a.keep_flag[p])
+            list[keep_scan[p]] = a.ents[a.idx[p]];
 }
 
 __global__ void xb_iota_u32(uint32_t *out, uint32_t n)
@@ -4158,187 +4248,6 @@ xpuB200TimeExecTask(xpuB200Session *s, const kern_data_store *kds_src_dev, int n
         total += ms;
     }
     *p_msec = niters > 0 ? total / niters : 0.0;
-    return 0;
-}
-
-/* ----------------------------------------------------------------
- * Final without device allocations
- *
- * xpuB200Final allocates its work arrays (per-slot tuple sizes, their
- * prefix sums, scan storage) and a device copy of kds_final from the
- * device's memory pool on every call.  Some callers cannot do that: a
- * service that has reserved the GPU's memory up front and hands out pieces
- * of its own pool (as PG-Strom's GPU service does with its device memory),
- * or one that must not allocate device memory while other sessions'
- * kernels run (a plain cudaFree waits for the whole device).  This variant writes
- * kds_final into memory the caller already owns and keeps its work arrays
- * in the fixed array below, which lives in the library's module on every
- * GPU that loads it until the process exits.
- * ---------------------------------------------------------------- */
-#define XB_FINAL_SCRATCH_BYTES  (8ULL << 20)        /* 8 MiB per GPU */
-#define XB_FINAL_SCRATCH_DEVS   64
-
-static __device__ __align__(256) char xb_final_scratch[XB_FINAL_SCRATCH_BYTES];
-
-/* device address of xb_final_scratch on each GPU, looked up once per device
- * (the host-side symbol is not a device address) */
-static void *xb_final_scratch_dptr[XB_FINAL_SCRATCH_DEVS];
-/* every session on one GPU shares that GPU's array: one call at a time
- * per GPU (calls for different GPUs use different arrays and run freely) */
-static std::mutex xb_final_scratch_lock[XB_FINAL_SCRATCH_DEVS];
-
-
-extern "C" int
-xpuB200FinalNoAlloc(xpuB200Session *s, void *kds_final_dev, uint64_t buf_sz, uint64_t *p_required,
-                    kern_exec_results *results, kern_errorbuf *err)
-{
-    xb_clear_error(err);
-    if (!s)
-        return XB_ERR(err, ERRCODE_DEVICE_ERROR, "invalid FinalNoAlloc arguments");
-    xb_sched_drain_session(s);
-    std::lock_guard<std::mutex> g(s->lock);
-    const int dindex = s->dev->dindex;
-    if (dindex < 0 || dindex >= XB_FINAL_SCRATCH_DEVS)
-        return XB_ERR(err, ERRCODE_DEVICE_ERROR, "FinalNoAlloc supports GPUs 0..%d", XB_FINAL_SCRATCH_DEVS - 1);
-    std::lock_guard<std::mutex> gs(xb_final_scratch_lock[dindex]);
-    XB_CUDA(cudaSetDevice(dindex), err);
-    if (!xb_final_scratch_dptr[dindex]) {
-        void *ptr = nullptr;
-        cudaError_t rc = cudaGetSymbolAddress(&ptr, xb_final_scratch);
-        if (rc != cudaSuccess || !ptr) {
-            cudaGetLastError();
-            return XB_ERR(err, ERRCODE_DEVICE_FATAL, "FinalNoAlloc: scratch address on GPU %d: %s",
-                          dindex, cudaGetErrorString(rc));
-        }
-        xb_final_scratch_dptr[dindex] = ptr;
-    }
-    char *scratch = (char *)xb_final_scratch_dptr[dindex];
-    cudaStream_t st = s->stream;
-    const xb_plan *plan = s->h_plan;
-    if (results) {
-        uint32_t cap = results->num_rels;
-        results->nitems_raw = (uint32_t)s->total_raw;
-        results->nitems_in = (uint32_t)s->total_in;
-        results->nitems_out = (uint32_t)s->total_out;
-        results->num_rels = plan->nrels;
-        for (uint32_t d = 1; d <= plan->nrels && d <= cap; d++)
-            results->stats[d - 1].nitems_out = (uint32_t)s->total_depth[d];
-        results->final_plan_task = true;
-    }
-    if (plan->nsort)
-        return XB_ERR(err, ERRCODE_DEVICE_ERROR, "a session with GPU-Sort keys needs xpuB200Final");
-    if (!plan->has_groupby) {
-        if (p_required) *p_required = 0;
-        return 0;
-    }
-    if (s->h_gt.dump) {
-        /* groups in the dump region join the table only when it grows,
-         * which allocates: that is xpuB200Final's work */
-        xb_gtable gh;
-        int grc = xb_gt_read(s, &gh, err);
-        if (grc) return grc;
-        if (gh.dump_used)
-            return XB_ERR(err, ERRCODE_DEVICE_ERROR,
-                          "FinalNoAlloc: %llu groups wait for the group table to grow; use xpuB200Final",
-                          (unsigned long long)gh.dump_used);
-    }
-    const kern_session_info *session = (const kern_session_info *)s->h_session.data();
-    const kern_data_store *fh = (const kern_data_store *)(s->h_session.data() + session->groupby_kds_final);
-    const uint64_t head_len = KDS_HEAD_LENGTH(fh);
-    const uint64_t cap = s->h_gt.cap_mask + 1;
-    const bool row_fmt = fh->format == KDS_FORMAT_ROW;
-
-    /* scratch layout: sizes | size prefix sums | flags | flag prefix sums | scan storage */
-    const uint64_t off_sscan = xb_align256(cap * 8);
-    const uint64_t off_flags = off_sscan + xb_align256(cap * 8);
-    const uint64_t off_fscan = off_flags + xb_align256(cap * 4);
-    const uint64_t off_temp = off_fscan + xb_align256(cap * 4);
-    uint64_t *d_sizes = (uint64_t *)scratch;
-    uint64_t *d_size_scan = (uint64_t *)(scratch + off_sscan);
-    uint32_t *d_flags = (uint32_t *)(scratch + off_flags);
-    uint32_t *d_flag_scan = (uint32_t *)(scratch + off_fscan);
-    void *d_temp = scratch + off_temp;
-    const uint64_t tsz_max = xb_scan_temp_bytes<uint64_t>(cap);
-    if (off_temp + tsz_max > XB_FINAL_SCRATCH_BYTES)
-        return XB_ERR(err, ERRCODE_DEVICE_ERROR,
-                      "FinalNoAlloc: the session's group table has %llu slots and needs %llu bytes of work "
-                      "space, above this entry point's fixed %llu bytes; use xpuB200Final",
-                      (unsigned long long)cap, (unsigned long long)(off_temp + tsz_max),
-                      (unsigned long long)XB_FINAL_SCRATCH_BYTES);
-    if (kds_final_dev) {
-        cudaPointerAttributes pa;
-        if (cudaPointerGetAttributes(&pa, kds_final_dev) != cudaSuccess) {
-            cudaGetLastError();
-            return XB_ERR(err, ERRCODE_DEVICE_ERROR, "FinalNoAlloc: kds_final_dev is not CUDA memory");
-        }
-        const bool ok = (pa.type == cudaMemoryTypeDevice && pa.device == dindex) ||
-                        pa.type == cudaMemoryTypeManaged ||
-                        (pa.type == cudaMemoryTypeHost && pa.devicePointer == kds_final_dev);
-        if (!ok)
-            return XB_ERR(err, ERRCODE_DEVICE_ERROR,
-                          "FinalNoAlloc: kds_final_dev must be memory of GPU %d (or mapped host memory)", dindex);
-    }
-    /* the previous call's values are still in the array: xb_final_sizes
-     * writes every size and flag below cap, and the scans overwrite their
-     * outputs, so no part of it needs clearing first */
-    XbFinalArgs fa;
-    memset(&fa, 0, sizeof(fa));
-    fa.plan = s->d_plan;
-    fa.gt = s->d_gt;
-    fa.cap = cap;
-    fa.sizes = d_sizes;
-    fa.flags = d_flags;
-    fa.size_scan = d_size_scan;
-    fa.flag_scan = d_flag_scan;
-    fa.row_format = row_fmt ? 1 : 0;
-    const int grid = s->dev->nsm * 8;
-    xb_final_sizes<<<grid, XB_BLOCK, 0, st>>>(fa);
-    xb_scan<uint64_t, XbOpSum, true>(d_sizes, d_size_scan, cap, d_temp, st);
-    xb_scan<uint32_t, XbOpSum, true>(d_flags, d_flag_scan, cap, d_temp, st);
-    uint64_t last_size = 0, last_scan = 0;
-    uint32_t last_flag = 0, last_fscan = 0;
-    cudaMemcpyAsync(&last_size, d_sizes + cap - 1, 8, cudaMemcpyDeviceToHost, st);
-    cudaMemcpyAsync(&last_scan, d_size_scan + cap - 1, 8, cudaMemcpyDeviceToHost, st);
-    cudaMemcpyAsync(&last_flag, d_flags + cap - 1, 4, cudaMemcpyDeviceToHost, st);
-    cudaMemcpyAsync(&last_fscan, d_flag_scan + cap - 1, 4, cudaMemcpyDeviceToHost, st);
-    if (cudaStreamSynchronize(st) != cudaSuccess)
-        return XB_ERR(err, ERRCODE_DEVICE_FATAL, "FinalNoAlloc: %s", cudaGetErrorString(cudaGetLastError()));
-    const uint64_t items = last_scan + last_size;
-    const uint64_t ngroups = (uint64_t)last_fscan + last_flag;
-    const uint64_t nslots = row_fmt ? 0 : KDS_GET_HASHSLOT_WIDTH(ngroups);
-    const uint64_t items_base = head_len + 8 * nslots + 8 * ngroups;
-    const uint64_t length = items_base + items;
-    if (p_required) *p_required = length;
-    if (results) {
-        results->final_nitems = (uint32_t)ngroups;
-        results->final_usage = items;
-        results->final_total = length;
-    }
-    if (!kds_final_dev || buf_sz < length) {
-        if (!kds_final_dev && buf_sz == 0)
-            return 0;           /* size query only */
-        return XB_ERR(err, ERRCODE_SUSPEND_NO_SPACE, "kds_final needs %llu bytes (buffer %llu)",
-                      (unsigned long long)length, (unsigned long long)buf_sz);
-    }
-    char *d_out = (char *)kds_final_dev;
-    std::vector<char> head((const char *)fh, (const char *)fh + head_len);
-    kern_data_store *kh = (kern_data_store *)head.data();
-    kh->length = length;
-    kh->usage = items;
-    kh->nitems = (uint32_t)ngroups;
-    kh->format = row_fmt ? KDS_FORMAT_ROW : KDS_FORMAT_HASH;
-    kh->hash_nslots = (uint32_t)nslots;
-    cudaMemcpyAsync(d_out, head.data(), head_len, cudaMemcpyHostToDevice, st);
-    /* slots, row index and items: the padding between and after the
-     * tuples' attributes is zero, so equal results are equal bytes */
-    cudaMemsetAsync(d_out + head_len, 0, length - head_len, st);
-    fa.kds_final = d_out;
-    fa.items_base = items_base;
-    fa.length = length;
-    fa.nslots = (uint32_t)nslots;
-    xb_final_write<<<grid, XB_BLOCK, 0, st>>>(fa);
-    if (cudaStreamSynchronize(st) != cudaSuccess)
-        return XB_ERR(err, ERRCODE_DEVICE_FATAL, "FinalNoAlloc: %s", cudaGetErrorString(cudaGetLastError()));
     return 0;
 }
 

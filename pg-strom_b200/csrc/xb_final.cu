@@ -6,6 +6,7 @@
  *
  *   xpuB200Final        kds_final in the reference layout, with GPU-Sort /
  *                       LIMIT / window rank of the groups
+ *   xpuB200FinalNoAlloc the same without device allocations
  *   xpuB200MergeFinal   another kds_final merged into a session's groups
  *   xpuB200FinalParts   the groups as hash partitions for the exchange step
  *   xpuB200InnerRebuild rows appended into a KDS_FORMAT_HASH inner buffer
@@ -22,109 +23,6 @@
 #include "xpu_b200.h"
 #include "xb_host.h"
 #include "xb_final.h"
-
-/* GPU-Sort of the session's groups: *p_keep receives, per group-table
- * entry, the group's output position or -1 (dropped by LIMIT or the window
- * rank).  fa carries the table and the flag arrays; alloc places device
- * memory that the caller frees.  Returns 0, or -1 when out of memory. */
-template <typename Alloc>
-static int xb_final_sort(xpuB200Session *s, XbFinalArgs fa, cudaStream_t st, Alloc alloc, int64_t **p_keep)
-{
-    const xb_plan *plan = s->h_plan;
-    const uint64_t cap = fa.cap;
-    const int grid = s->dev->nsm * 8;
-    fa.keep = nullptr;
-    xb_final_sizes<<<grid, XB_BLOCK, 0, st>>>(fa);              /* flags of every group */
-    void *d_t = nullptr;
-    if (!alloc(xb_scan_temp_bytes<uint32_t>(cap), &d_t)) return -1;
-    if (xb_scan<uint32_t, XbOpSum, true>(fa.flags, fa.flag_scan, cap, d_t, st) != cudaSuccess) return -1;
-    uint32_t lf = 0, ls = 0;
-    cudaMemcpyAsync(&lf, fa.flags + cap - 1, 4, cudaMemcpyDeviceToHost, st);
-    cudaMemcpyAsync(&ls, fa.flag_scan + cap - 1, 4, cudaMemcpyDeviceToHost, st);
-    if (cudaStreamSynchronize(st) != cudaSuccess) return -1;
-    const uint32_t n = lf + ls;
-    int64_t *keep = nullptr;
-    if (!alloc(cap * 8, (void **)&keep)) return -1;
-    cudaMemsetAsync(keep, 0xff, cap * 8, st);
-    *p_keep = keep;
-    if (n == 0)
-        return 0;
-    const uint32_t nk = plan->nsort;
-    uint32_t *ents, *idx, *idx2, *part, *peer, *pflag, *pcnt, *kflag, *kscan;
-    uint64_t *keyw, *k64a, *k64b;
-    uint8_t *nul, *k8a, *k8b;
-    if (!alloc((size_t)n * 4, (void **)&ents) || !alloc((size_t)n * 4, (void **)&idx) ||
-        !alloc((size_t)n * 4, (void **)&idx2) || !alloc((size_t)n * 16 * nk, (void **)&keyw) ||
-        !alloc((size_t)n * nk, (void **)&nul) || !alloc((size_t)n * 8, (void **)&k64a) ||
-        !alloc((size_t)n * 8, (void **)&k64b) || !alloc((size_t)n, (void **)&k8a) ||
-        !alloc((size_t)n, (void **)&k8b) || !alloc((size_t)n * 4, (void **)&part) ||
-        !alloc((size_t)n * 4, (void **)&peer) || !alloc((size_t)n * 4, (void **)&pflag) ||
-        !alloc((size_t)n * 4, (void **)&pcnt) || !alloc((size_t)n * 4, (void **)&kflag) ||
-        !alloc((size_t)n * 4, (void **)&kscan))
-        return -1;
-    XbSortArgs sa;
-    sa.plan = s->d_plan;
-    sa.gt = s->d_gt;
-    sa.cap = cap;
-    sa.flags = fa.flags;
-    sa.flag_scan = fa.flag_scan;
-    sa.ents = ents;
-    sa.keyw = keyw;
-    sa.nul = nul;
-    sa.n = n;
-    int g2 = (int)((n + XB_BLOCK - 1) / XB_BLOCK);
-    if (g2 > grid) g2 = grid;
-    xb_sort_gather<<<grid, XB_BLOCK, 0, st>>>(sa);
-    xb_sort_keys<<<g2, XB_BLOCK, 0, st>>>(sa);
-    xb_iota_u32<<<g2, XB_BLOCK, 0, st>>>(idx, n);
-    /* temporary storage for the largest of the sort and scan passes */
-    const size_t tt = std::max(xb_radix_temp_bytes(n), xb_scan_temp_bytes<uint32_t>(n));
-    void *d_tt = nullptr;
-    if (!alloc(tt, &d_tt)) return -1;
-    /* stable passes, least significant first: for each key from the last,
-     * its low word, its high word, then its NULL flag (each a stable radix
-     * sort of the word gathered in the current order, carrying the group
-     * indexes along) */
-    for (int k = (int)nk - 1; k >= 0; k--) {
-        for (int w = 1; w >= 0; w--) {
-            if (w == 1 && plan->sort[k].words < 2)
-                continue;
-            xb_sort_pass_key64<<<g2, XB_BLOCK, 0, st>>>(keyw + (2ULL * k + w) * n, idx, k64a, n);
-            if (xb_radix_sort<uint64_t>(k64a, k64b, idx, idx2, n, 64, d_tt, st) != cudaSuccess) return -1;
-        }
-        xb_sort_pass_key8<<<g2, XB_BLOCK, 0, st>>>(nul + (uint64_t)k * n, idx, k8a, n);
-        if (xb_radix_sort<uint8_t>(k8a, k8b, idx, idx2, n, 8, d_tt, st) != cudaSuccess) return -1;
-    }
-    XbRankArgs ra;
-    ra.plan = s->d_plan;
-    ra.idx = idx;
-    ra.keyw = keyw;
-    ra.nul = nul;
-    ra.n = n;
-    ra.part_start = part;
-    ra.peer_start = peer;
-    ra.peer_flag = pflag;
-    if (plan->sort_window) {
-        xb_sort_bounds<<<g2, XB_BLOCK, 0, st>>>(ra);
-        if (xb_scan<uint32_t, XbOpMax, false>(part, part, n, d_tt, st) != cudaSuccess ||
-            xb_scan<uint32_t, XbOpMax, false>(peer, peer, n, d_tt, st) != cudaSuccess ||
-            xb_scan<uint32_t, XbOpSum, false>(pflag, pcnt, n, d_tt, st) != cudaSuccess)
-            return -1;
-    }
-    XbKeepArgs ka;
-    ka.plan = s->d_plan;
-    ka.idx = idx;
-    ka.ents = ents;
-    ka.n = n;
-    ka.part_start = part;
-    ka.peer_start = peer;
-    ka.peer_cnt = pcnt;
-    ka.keep_flag = kflag;
-    xb_sort_keepflag<<<g2, XB_BLOCK, 0, st>>>(ka);
-    if (xb_scan<uint32_t, XbOpSum, true>(kflag, kscan, n, d_tt, st) != cudaSuccess) return -1;
-    xb_sort_keep<<<g2, XB_BLOCK, 0, st>>>(ka, kscan, keep);
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
-}
 
 /* the fixed tuple of the session's groups as a program of 4-byte units
  * (xb_write_group_tuple's layout with every key present), and the bytes of
@@ -257,6 +155,8 @@ struct XbFinalRun {
     uint64_t        head_len = 0;
     bool            row_fmt = false;
     std::vector<void *> tmp;
+    char           *scratch = nullptr;      /* work memory of the caller's, instead of the pool's */
+    uint64_t        scratch_left = 0;
     XbTileArgs      ta;
     uint64_t       *d_totals = nullptr;
     void           *d_temp = nullptr;
@@ -276,6 +176,14 @@ struct XbFinalRun {
     }
     bool alloc(size_t sz, void **p)
     {
+        if (scratch) {
+            sz = xb_align256(sz);
+            if (sz > scratch_left) return false;
+            *p = scratch;
+            scratch += sz;
+            scratch_left -= sz;
+            return true;
+        }
         if (cudaMallocAsync(p, sz < 256 ? 256 : sz, s->stream) != cudaSuccess) { cudaGetLastError(); return false; }
         tmp.push_back(*p);
         return true;
@@ -303,13 +211,14 @@ struct XbFinalRun {
     }
     /* tiles small enough to spread the table over the GPU, and few enough
      * that the counters of a launch's parts stay small */
-    int plan(uint32_t nparts, kern_errorbuf *err)
+    int plan(uint32_t nparts, kern_errorbuf *err, const uint32_t *list = nullptr, uint32_t nlist = 0)
     {
         cudaStream_t st = s->stream;
         memset(&ta, 0, sizeof(ta));
         ta.plan = s->d_plan;
         ta.gt = s->d_gt;
-        ta.cap = s->h_gt.cap_mask + 1;
+        ta.list = list;
+        ta.cap = list ? nlist : s->h_gt.cap_mask + 1;
         ta.nparts = nparts;
         ta.row_format = row_fmt ? 1 : 0;
         xb_final_program(s->h_plan, row_fmt, &ta.prog);
@@ -373,9 +282,261 @@ struct XbFinalRun {
     }
 };
 
-/* kds_final of a session with GPU-Sort keys */
-static int xb_final_sorted(xpuB200Session *s, void *kds_final_buf, uint64_t buf_sz, uint64_t *p_required,
-                           kern_exec_results *results, kern_errorbuf *err);
+/* GPU-Sort of the session's groups: the entries of those kept by LIMIT or
+ * the window rank, in order, in *p_list (work memory of run; *p_n of them).
+ * run has counted the groups of the whole table.  Returns 0, or -1. */
+static int xb_final_sort(XbFinalRun &run, uint32_t **p_list, uint32_t *p_n)
+{
+    xpuB200Session *s = run.s;
+    const xb_plan *plan = s->h_plan;
+    cudaStream_t st = s->stream;
+    const int grid = s->dev->nsm * 8;
+    const uint32_t n = (uint32_t)run.totals[0];
+    *p_n = 0;
+    if (n == 0)
+        return 0;
+    const uint32_t nk = plan->nsort;
+    uint32_t *ents, *idx, *list;
+    uint64_t *keyw;
+    uint8_t *nul;
+    if (!run.alloc((size_t)n * 4, (void **)&ents) || !run.alloc((size_t)n * 4, (void **)&idx) ||
+        !run.alloc((size_t)n * 4, (void **)&list) || !run.alloc((size_t)n * 16 * nk, (void **)&keyw) ||
+        !run.alloc((size_t)n * nk, (void **)&nul))
+        return -1;
+    *p_list = list;
+    XbSortArgs sa;
+    sa.plan = s->d_plan;
+    sa.gt = s->d_gt;
+    sa.ents = ents;
+    sa.keyw = keyw;
+    sa.nul = nul;
+    sa.n = n;
+    const int g2 = std::min((int)((n + XB_BLOCK - 1) / XB_BLOCK), grid);
+    xb_final_ents<<<run.grid(), XB_FINAL_TILE, 0, st>>>(run.ta, ents);
+    xb_sort_keys<<<g2, XB_BLOCK, 0, st>>>(sa);
+    uint32_t m = n;                 /* groups in idx, in sort order */
+    bool sorted = false;
+    if (n <= XB_SORT_SMALL) {
+        xb_sort_small<<<1, 1024, 0, st>>>(sa, nullptr, n, idx);
+        sorted = true;
+    } else if (plan->sort_limit > 0 && !plan->sort_window && plan->sort_limit <= XB_SORT_SMALL) {
+        /* the candidates, unless more than one CTA sorts share the last
+         * one's leading bits */
+        XbTopArgs ta;
+        char *mem;
+        const size_t hb = sizeof(uint32_t) * XB_TOP_DIGITS * XB_TOP_BINS;
+        if (!run.alloc(hb + 32 + 4 * XB_SORT_SMALL, (void **)&mem))
+            return -1;
+        cudaMemsetAsync(mem, 0, hb + 32, st);
+        ta.hi = keyw;
+        ta.nul = nul;
+        ta.n = n;
+        ta.hist = (uint32_t *)mem;
+        ta.prefix = (uint64_t *)(mem + hb);
+        ta.ncand = (uint32_t *)(mem + hb + 16);
+        ta.cand = (uint32_t *)(mem + hb + 32);
+        const uint64_t want = (uint64_t)plan->sort_limit;
+        cudaMemcpyAsync(&ta.prefix[1], &want, 8, cudaMemcpyHostToDevice, st);
+        const int g3 = std::min(g2, s->dev->nsm * 4);
+        for (uint32_t d = 0; d < XB_TOP_DIGITS; d++) {
+            xb_top_hist<<<g3, XB_BLOCK, 0, st>>>(ta, d);
+            xb_top_select<<<1, XB_SCAN_BLOCK, 0, st>>>(ta, d);
+        }
+        xb_top_gather<<<g3, XB_BLOCK, 0, st>>>(ta);
+        uint32_t nc = 0;
+        cudaMemcpyAsync(&nc, ta.ncand, 4, cudaMemcpyDeviceToHost, st);
+        if (cudaStreamSynchronize(st) != cudaSuccess) return -1;
+        if (nc <= XB_SORT_SMALL) {
+            xb_sort_small<<<1, 1024, 0, st>>>(sa, ta.cand, nc, idx);
+            m = nc;
+            sorted = true;
+        }
+    }
+    const size_t tt = std::max(xb_radix_temp_bytes(n), xb_scan_temp_bytes<uint32_t>(n));
+    void *d_tt = nullptr;
+    if (!run.alloc(tt, &d_tt)) return -1;
+    if (!sorted) {
+        /* stable passes, least significant first: for each key from the
+         * last, its low word, its high word, then its NULL flag (each a
+         * stable radix sort of the word gathered in the current order,
+         * carrying the group indexes along) */
+        uint32_t *idx2;
+        uint64_t *k64a, *k64b;
+        uint8_t *k8a, *k8b;
+        if (!run.alloc((size_t)n * 4, (void **)&idx2) || !run.alloc((size_t)n * 8, (void **)&k64a) ||
+            !run.alloc((size_t)n * 8, (void **)&k64b) || !run.alloc((size_t)n, (void **)&k8a) ||
+            !run.alloc((size_t)n, (void **)&k8b))
+            return -1;
+        xb_iota_u32<<<g2, XB_BLOCK, 0, st>>>(idx, n);
+        for (int k = (int)nk - 1; k >= 0; k--) {
+            for (int w = 1; w >= 0; w--) {
+                if (w == 1 && plan->sort[k].words < 2)
+                    continue;
+                xb_sort_pass_key64<<<g2, XB_BLOCK, 0, st>>>(keyw + (2ULL * k + w) * n, idx, k64a, n);
+                if (xb_radix_sort<uint64_t>(k64a, k64b, idx, idx2, n, 64, d_tt, st) != cudaSuccess) return -1;
+            }
+            xb_sort_pass_key8<<<g2, XB_BLOCK, 0, st>>>(nul + (uint64_t)k * n, idx, k8a, n);
+            if (xb_radix_sort<uint8_t>(k8a, k8b, idx, idx2, n, 8, d_tt, st) != cudaSuccess) return -1;
+        }
+    }
+    XbKeepArgs ka;
+    memset(&ka, 0, sizeof(ka));
+    uint32_t *kflag, *kscan;
+    if (!run.alloc((size_t)m * 4, (void **)&kflag) || !run.alloc((size_t)m * 4, (void **)&kscan))
+        return -1;
+    if (plan->sort_window) {
+        uint32_t *part, *peer, *pflag, *pcnt;
+        if (!run.alloc((size_t)m * 4, (void **)&part) || !run.alloc((size_t)m * 4, (void **)&peer) ||
+            !run.alloc((size_t)m * 4, (void **)&pflag) || !run.alloc((size_t)m * 4, (void **)&pcnt))
+            return -1;
+        XbRankArgs ra;
+        ra.plan = s->d_plan;
+        ra.idx = idx;
+        ra.keyw = keyw;
+        ra.nul = nul;
+        ra.n = n;
+        ra.part_start = part;
+        ra.peer_start = peer;
+        ra.peer_flag = pflag;
+        xb_sort_bounds<<<g2, XB_BLOCK, 0, st>>>(ra);
+        if (xb_scan<uint32_t, XbOpMax, false>(part, part, n, d_tt, st) != cudaSuccess ||
+            xb_scan<uint32_t, XbOpMax, false>(peer, peer, n, d_tt, st) != cudaSuccess ||
+            xb_scan<uint32_t, XbOpSum, false>(pflag, pcnt, n, d_tt, st) != cudaSuccess)
+            return -1;
+        ka.part_start = part;
+        ka.peer_start = peer;
+        ka.peer_cnt = pcnt;
+    }
+    ka.plan = s->d_plan;
+    ka.idx = idx;
+    ka.ents = ents;
+    ka.n = m;
+    ka.keep_flag = kflag;
+    xb_sort_keepflag<<<g2, XB_BLOCK, 0, st>>>(ka);
+    if (xb_scan<uint32_t, XbOpSum, true>(kflag, kscan, m, d_tt, st) != cudaSuccess) return -1;
+    xb_sort_keep<<<g2, XB_BLOCK, 0, st>>>(ka, kscan, list);
+    uint32_t lf = 0, ls = 0;
+    cudaMemcpyAsync(&lf, kflag + m - 1, 4, cudaMemcpyDeviceToHost, st);
+    cudaMemcpyAsync(&ls, kscan + m - 1, 4, cudaMemcpyDeviceToHost, st);
+    if (cudaStreamSynchronize(st) != cudaSuccess) return -1;
+    *p_n = lf + ls;
+    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+/* ----------------------------------------------------------------
+ * Final without device allocations
+ *
+ * xpuB200Final allocates its work arrays (the tiles' counts and their
+ * prefix sums, scan storage) and a device copy of kds_final from the
+ * device's memory pool on every call.  Some callers cannot do that: a
+ * service that has reserved the GPU's memory up front and hands out pieces
+ * of its own pool (as PG-Strom's GPU service does with its device memory),
+ * or one that must not allocate device memory while other sessions'
+ * kernels run (a plain cudaFree waits for the whole device).  This variant writes
+ * kds_final into memory the caller already owns and keeps its work arrays
+ * in the fixed array below, which lives in the library's module on every
+ * GPU that loads it until the process exits.
+ * ---------------------------------------------------------------- */
+#define XB_FINAL_SCRATCH_BYTES  (8ULL << 20)        /* 8 MiB per GPU */
+#define XB_FINAL_SCRATCH_SLOTS  262144ULL
+#define XB_FINAL_SCRATCH_DEVS   64
+
+static __device__ __align__(256) char xb_final_scratch[XB_FINAL_SCRATCH_BYTES];
+
+/* device address of xb_final_scratch on each GPU, looked up once per device
+ * (the host-side symbol is not a device address) */
+static void *xb_final_scratch_dptr[XB_FINAL_SCRATCH_DEVS];
+/* every session on one GPU shares that GPU's array: one call at a time
+ * per GPU (calls for different GPUs use different arrays and run freely) */
+static std::mutex xb_final_scratch_lock[XB_FINAL_SCRATCH_DEVS];
+
+
+extern "C" int
+xpuB200FinalNoAlloc(xpuB200Session *s, void *kds_final_dev, uint64_t buf_sz, uint64_t *p_required,
+                    kern_exec_results *results, kern_errorbuf *err)
+{
+    xb_clear_error(err);
+    if (!s)
+        return XB_ERR(err, ERRCODE_DEVICE_ERROR, "invalid FinalNoAlloc arguments");
+    xb_sched_drain_session(s);
+    std::lock_guard<std::mutex> g(s->lock);
+    const int dindex = s->dev->dindex;
+    if (dindex < 0 || dindex >= XB_FINAL_SCRATCH_DEVS)
+        return XB_ERR(err, ERRCODE_DEVICE_ERROR, "FinalNoAlloc supports GPUs 0..%d", XB_FINAL_SCRATCH_DEVS - 1);
+    std::lock_guard<std::mutex> gs(xb_final_scratch_lock[dindex]);
+    XB_CUDA(cudaSetDevice(dindex), err);
+    if (!xb_final_scratch_dptr[dindex]) {
+        void *ptr = nullptr;
+        cudaError_t rc = cudaGetSymbolAddress(&ptr, xb_final_scratch);
+        if (rc != cudaSuccess || !ptr) {
+            cudaGetLastError();
+            return XB_ERR(err, ERRCODE_DEVICE_FATAL, "FinalNoAlloc: scratch address on GPU %d: %s",
+                          dindex, cudaGetErrorString(rc));
+        }
+        xb_final_scratch_dptr[dindex] = ptr;
+    }
+    char *scratch = (char *)xb_final_scratch_dptr[dindex];
+    const xb_plan *plan = s->h_plan;
+    if (results) {
+        uint32_t cap = results->num_rels;
+        results->nitems_raw = (uint32_t)s->total_raw;
+        results->nitems_in = (uint32_t)s->total_in;
+        results->nitems_out = (uint32_t)s->total_out;
+        results->num_rels = plan->nrels;
+        for (uint32_t d = 1; d <= plan->nrels && d <= cap; d++)
+            results->stats[d - 1].nitems_out = (uint32_t)s->total_depth[d];
+        results->final_plan_task = true;
+    }
+    if (plan->nsort)
+        return XB_ERR(err, ERRCODE_DEVICE_ERROR, "a session with GPU-Sort keys needs xpuB200Final");
+    if (!plan->has_groupby) {
+        if (p_required) *p_required = 0;
+        return 0;
+    }
+    if (s->h_gt.dump) {
+        /* groups in the dump region join the table only when it grows,
+         * which allocates: that is xpuB200Final's work */
+        xb_gtable gh;
+        int grc = xb_gt_read(s, &gh, err);
+        if (grc) return grc;
+        if (gh.dump_used)
+            return XB_ERR(err, ERRCODE_DEVICE_ERROR,
+                          "FinalNoAlloc: %llu groups wait for the group table to grow; use xpuB200Final",
+                          (unsigned long long)gh.dump_used);
+    }
+    /* larger tables are xpuB200Final's, as they were when the work arrays
+     * had an element per slot */
+    const uint64_t cap = s->h_gt.cap_mask + 1;
+    if (cap > XB_FINAL_SCRATCH_SLOTS)
+        return XB_ERR(err, ERRCODE_DEVICE_ERROR,
+                      "FinalNoAlloc: the session's group table has %llu slots, above the %llu that this entry "
+                      "point's fixed work space of %llu bytes serves; use xpuB200Final",
+                      (unsigned long long)cap, (unsigned long long)XB_FINAL_SCRATCH_SLOTS,
+                      (unsigned long long)XB_FINAL_SCRATCH_BYTES);
+    XbFinalRun run(s);
+    run.scratch = scratch;
+    run.scratch_left = XB_FINAL_SCRATCH_BYTES;
+    int rc = run.plan(1, err);
+    if (rc) return rc;
+    const XbFinalPart P = run.part(0, 0);
+    if (p_required) *p_required = P.length;
+    if (results) {
+        results->final_nitems = P.nitems;
+        results->final_usage = P.length - P.items_base;
+        results->final_total = P.length;
+    }
+    if (!kds_final_dev || buf_sz < P.length) {
+        if (!kds_final_dev && buf_sz == 0)
+            return 0;           /* size query only */
+        return XB_ERR(err, ERRCODE_SUSPEND_NO_SPACE, "kds_final needs %llu bytes (buffer %llu)",
+                      (unsigned long long)P.length, (unsigned long long)buf_sz);
+    }
+    rc = run.write((char *)kds_final_dev, std::vector<XbFinalPart>(1, P), err);
+    if (rc) return rc;
+    if (cudaStreamSynchronize(s->stream) != cudaSuccess)
+        return XB_ERR(err, ERRCODE_DEVICE_FATAL, "FinalNoAlloc: %s", cudaGetErrorString(cudaGetLastError()));
+    return 0;
+}
 
 extern "C" int
 xpuB200Final(xpuB200Session *s, void *kds_final_buf, uint64_t buf_sz, uint64_t *p_required,
@@ -406,11 +567,21 @@ xpuB200Final(xpuB200Session *s, void *kds_final_buf, uint64_t buf_sz, uint64_t *
     /* groups waiting in the dump region join the table first */
     int src = xb_gt_settle(s, err);
     if (src) return src;
-    if (plan->nsort)
-        return xb_final_sorted(s, kds_final_buf, buf_sz, p_required, results, err);
     XbFinalRun run(s);
     int rc = run.plan(1, err);
     if (rc) return rc;
+    if (plan->nsort) {
+        uint32_t *list = nullptr, n = 0;
+        if (xb_final_sort(run, &list, &n) != 0)
+            return XB_ERR(err, ERRCODE_DEVICE_FATAL, "GPU-Sort of the groups failed (%s)",
+                          cudaGetErrorString(cudaGetLastError()));
+        if (n > 0 && (rc = run.plan(1, err, list, n)) != 0)
+            return rc;
+        if (n == 0) {
+            run.totals.assign(2, 0);
+            run.ta.cap = 0;
+        }
+    }
     const XbFinalPart P = run.part(0, 0);
     if (p_required) *p_required = P.length;
     if (results) {
@@ -434,116 +605,6 @@ xpuB200Final(xpuB200Session *s, void *kds_final_buf, uint64_t buf_sz, uint64_t *
     if (cudaStreamSynchronize(st) != cudaSuccess)
         return XB_ERR(err, ERRCODE_DEVICE_FATAL, "Final: %s", cudaGetErrorString(cudaGetLastError()));
     return 0;
-}
-
-static int xb_final_sorted(xpuB200Session *s, void *kds_final_buf, uint64_t buf_sz, uint64_t *p_required,
-                           kern_exec_results *results, kern_errorbuf *err)
-{
-    cudaStream_t st = s->stream;
-    const kern_session_info *session = (const kern_session_info *)s->h_session.data();
-    const kern_data_store *fh = (const kern_data_store *)(s->h_session.data() + session->groupby_kds_final);
-    const uint64_t head_len = KDS_HEAD_LENGTH(fh);
-    const uint64_t cap = s->h_gt.cap_mask + 1;
-    const bool row_fmt = fh->format == KDS_FORMAT_ROW;
-
-    uint64_t *d_sizes = nullptr, *d_size_scan = nullptr;
-    uint32_t *d_flags = nullptr, *d_flag_scan = nullptr;
-    char *d_out = nullptr;
-    void *d_temp = nullptr;
-    int rc = 0;
-    std::vector<void *> tmp;
-    auto alloc = [&](size_t sz, void **p) -> bool {
-        if (cudaMallocAsync(p, sz < 256 ? 256 : sz, st) != cudaSuccess) { cudaGetLastError(); return false; }
-        tmp.push_back(*p);
-        return true;
-    };
-    auto cleanup = [&]() { for (void *p : tmp) cudaFreeAsync(p, st); };
-    if (!alloc(cap * 8, (void **)&d_sizes) || !alloc(cap * 8, (void **)&d_size_scan) ||
-        !alloc(cap * 4, (void **)&d_flags) || !alloc(cap * 4, (void **)&d_flag_scan)) {
-        cleanup();
-        return XB_ERR(err, ERRCODE_DEVICE_FATAL, "out of device memory in Final");
-    }
-    XbFinalArgs fa;
-    memset(&fa, 0, sizeof(fa));
-    fa.plan = s->d_plan;
-    fa.gt = s->d_gt;
-    fa.cap = cap;
-    fa.sizes = d_sizes;
-    fa.flags = d_flags;
-    fa.size_scan = d_size_scan;
-    fa.flag_scan = d_flag_scan;
-    fa.row_format = row_fmt ? 1 : 0;
-    int grid = s->dev->nsm * 8;
-    int64_t *d_keep = nullptr;
-    if (xb_final_sort(s, fa, st, alloc, &d_keep) != 0) {
-        cleanup();
-        return XB_ERR(err, ERRCODE_DEVICE_FATAL, "GPU-Sort of the groups failed (%s)",
-                      cudaGetErrorString(cudaGetLastError()));
-    }
-    fa.keep = d_keep;
-    /* the global table's entries pointer lives in h_gt */
-    xb_final_sizes<<<grid, XB_BLOCK, 0, st>>>(fa);
-    if (!alloc(xb_scan_temp_bytes<uint64_t>(cap), &d_temp)) {
-        cleanup();
-        return XB_ERR(err, ERRCODE_DEVICE_FATAL, "out of device memory in Final");
-    }
-    xb_scan<uint64_t, XbOpSum, true>(d_sizes, d_size_scan, cap, d_temp, st);
-    xb_scan<uint32_t, XbOpSum, true>(d_flags, d_flag_scan, cap, d_temp, st);
-    uint64_t last_size = 0, last_scan = 0;
-    uint32_t last_flag = 0, last_fscan = 0;
-    cudaMemcpyAsync(&last_size, d_sizes + cap - 1, 8, cudaMemcpyDeviceToHost, st);
-    cudaMemcpyAsync(&last_scan, d_size_scan + cap - 1, 8, cudaMemcpyDeviceToHost, st);
-    cudaMemcpyAsync(&last_flag, d_flags + cap - 1, 4, cudaMemcpyDeviceToHost, st);
-    cudaMemcpyAsync(&last_fscan, d_flag_scan + cap - 1, 4, cudaMemcpyDeviceToHost, st);
-    if (cudaStreamSynchronize(st) != cudaSuccess) {
-        cleanup();
-        return XB_ERR(err, ERRCODE_DEVICE_FATAL, "Final: %s", cudaGetErrorString(cudaGetLastError()));
-    }
-    const uint64_t items = last_scan + last_size;
-    const uint64_t ngroups = (uint64_t)last_fscan + last_flag;
-    const uint64_t nslots = row_fmt ? 0 : KDS_GET_HASHSLOT_WIDTH(ngroups);
-    const uint64_t items_base = head_len + 8 * nslots + 8 * ngroups;
-    const uint64_t length = items_base + items;
-    if (p_required) *p_required = length;
-    if (results) {
-        results->final_nitems = (uint32_t)ngroups;
-        results->final_usage = items;
-        results->final_total = length;
-    }
-    if (!kds_final_buf || buf_sz < length) {
-        cleanup();
-        if (!kds_final_buf && buf_sz == 0)
-            return 0;           /* size query only */
-        return XB_ERR(err, ERRCODE_SUSPEND_NO_SPACE, "kds_final needs %llu bytes (buffer %llu)",
-                      (unsigned long long)length, (unsigned long long)buf_sz);
-    }
-    if (!alloc(length, (void **)&d_out)) {
-        cleanup();
-        return XB_ERR(err, ERRCODE_DEVICE_FATAL, "out of device memory for kds_final (%llu bytes)",
-                      (unsigned long long)length);
-    }
-    /* header: the session's kds_final definition with the actual sizes */
-    std::vector<char> head((const char *)fh, (const char *)fh + head_len);
-    kern_data_store *kh = (kern_data_store *)head.data();
-    kh->length = length;
-    kh->usage = items;
-    kh->nitems = (uint32_t)ngroups;
-    kh->format = row_fmt ? KDS_FORMAT_ROW : KDS_FORMAT_HASH;
-    kh->hash_nslots = (uint32_t)nslots;
-    cudaMemcpyAsync(d_out, head.data(), head_len, cudaMemcpyHostToDevice, st);
-    /* slots, row index and items: the padding between and after the
-     * tuples' attributes is zero, so equal results are equal bytes */
-    cudaMemsetAsync(d_out + head_len, 0, length - head_len, st);
-    fa.kds_final = d_out;
-    fa.items_base = items_base;
-    fa.length = length;
-    fa.nslots = (uint32_t)nslots;
-    xb_final_write<<<grid, XB_BLOCK, 0, st>>>(fa);
-    cudaMemcpyAsync(kds_final_buf, d_out, length, cudaMemcpyDeviceToHost, st);
-    if (cudaStreamSynchronize(st) != cudaSuccess)
-        rc = XB_ERR(err, ERRCODE_DEVICE_FATAL, "Final: %s", cudaGetErrorString(cudaGetLastError()));
-    cleanup();
-    return rc;
 }
 
 extern "C" int

@@ -5,9 +5,9 @@
  * their arguments: kds_final materialisation, GPU-Sort of the groups, the
  * merge of another kds_final into a session's group table and the
  * inner-buffer rebuild.  The host services that launch them live in
- * xb_final.cu (xpuB200Final, xpuB200MergeFinal, xpuB200FinalParts,
- * xpuB200InnerRebuild) and in xb_exec.cu (xpuB200FinalNoAlloc).  Internal;
- * the public interface is include/xpu_b200.h.
+ * xb_final.cu (xpuB200Final, xpuB200FinalNoAlloc, xpuB200MergeFinal,
+ * xpuB200FinalParts, xpuB200InnerRebuild).  Internal; the public interface
+ * is include/xpu_b200.h.
  */
 #ifndef XB_FINAL_H
 #define XB_FINAL_H
@@ -16,29 +16,9 @@
 #include <cstdint>
 #include "xb_plan.h"
 #include "xb_exec_dev.cuh"
+#include "xb_sort.cuh"
 
 #define XB_GENT_MAX     2048    /* largest group entry a merge stages per thread */
-
-/* kds_final materialisation: per-entry tuple sizes, then the tuples */
-struct XbFinalArgs {
-    const xb_plan  *plan;
-    xb_gtable      *gt;
-    uint64_t        cap;
-    uint64_t       *sizes;          /* per entry: item bytes (0 if empty) */
-    uint32_t       *flags;          /* per entry: 1 if ready */
-    uint64_t       *size_scan;
-    uint32_t       *flag_scan;
-    char           *kds_final;      /* device buffer (header already in place) */
-    uint64_t        items_base;     /* offset of the first item */
-    uint64_t        length;
-    uint32_t        nslots;
-    uint32_t        row_format;     /* KDS_FORMAT_ROW (no GROUP BY keys): kern_tupitems
-                                     * without hash links, nslots 0 */
-    uint32_t        part_div;       /* >= 2: only the groups with hash % part_div == part_rem */
-    uint32_t        part_rem;
-    const int64_t  *keep;           /* GPU-Sort: output position per entry, -1 dropped
-                                     * (nullptr: every group, in table order) */
-};
 
 /* the tuple of a group whose size and attribute offsets are the plan's
  * alone (every key fixed-width of 4 or 8 bytes, none NULL), as 4-byte
@@ -89,6 +69,8 @@ struct XbTileArgs {
     const uint64_t *bytes_scan;
     char           *out;
     const XbFinalPart *part;
+    const uint32_t *list;           /* the entries to write, in order (cap of them), or
+                                     * nullptr: every group, in table order */
     XbFinalProg     prog;
 };
 
@@ -96,13 +78,27 @@ struct XbTileArgs {
 struct XbSortArgs {
     const xb_plan  *plan;
     const xb_gtable *gt;
-    uint64_t        cap;
-    const uint32_t *flags;          /* per entry: 1 if ready */
-    const uint32_t *flag_scan;
-    uint32_t       *ents;           /* per rank: entry index */
+    const uint32_t *ents;           /* per rank: entry index */
     uint64_t       *keyw;           /* word w of key k at keyw[(2k + w) * n + r] */
     uint8_t        *nul;            /* NULL flag of key k at nul[k * n + r] */
     uint32_t        n;
+};
+
+/* the first 'want' groups by their first sort key: radix selection of its
+ * leading XB_TOP_BITS bits (the NULL flag, then the key's high word) by
+ * digits of 11 bits, then every group up to and including the last one's
+ * digits */
+#define XB_TOP_DIGITS   4
+#define XB_TOP_BINS     2048
+#define XB_SORT_SMALL   4096        /* groups that one CTA sorts */
+struct XbTopArgs {
+    const uint64_t *hi;             /* first key's high words and NULL flags */
+    const uint8_t  *nul;
+    uint32_t        n;
+    uint32_t       *hist;           /* XB_TOP_DIGITS * XB_TOP_BINS, zero */
+    uint64_t       *prefix;         /* [0] digits chosen so far, [1] groups still wanted */
+    uint32_t       *cand;           /* the groups picked, XB_SORT_SMALL at most */
+    uint32_t       *ncand;          /* how many there are */
 };
 
 /* groups kept, in order: LIMIT, or the window rank of each group within
@@ -149,8 +145,6 @@ struct XbRebuildArgs {
 };
 
 /* the kernels (xb_exec.cu) */
-__global__ void xb_final_sizes(XbFinalArgs args);
-__global__ void xb_final_write(XbFinalArgs args);
 __global__ void __launch_bounds__(XB_FINAL_TILE) xb_final_tiles(const __grid_constant__ XbTileArgs a);
 __global__ void __launch_bounds__(XB_FINAL_TILE) xb_final_scan_small(XbTileArgs a, uint32_t *count_scan,
                                                                       uint64_t *bytes_scan, uint32_t n);
@@ -158,13 +152,17 @@ __global__ void xb_final_totals(XbTileArgs a, uint64_t *totals);
 __global__ void xb_final_heads(char *out, const XbFinalPart *part, const uint64_t *head, uint32_t head_len,
                                uint32_t row_format);
 __global__ void __launch_bounds__(XB_FINAL_TILE) xb_final_fill(const __grid_constant__ XbTileArgs a);
-__global__ void xb_sort_gather(XbSortArgs a);
+__global__ void __launch_bounds__(XB_FINAL_TILE) xb_final_ents(const __grid_constant__ XbTileArgs a, uint32_t *ents);
+__global__ void xb_top_hist(XbTopArgs a, uint32_t digit);
+__global__ void __launch_bounds__(XB_SCAN_BLOCK) xb_top_select(XbTopArgs a, uint32_t digit);
+__global__ void xb_top_gather(XbTopArgs a);
+__global__ void __launch_bounds__(1024) xb_sort_small(XbSortArgs a, const uint32_t *cand, uint32_t m, uint32_t *idx);
 __global__ void xb_sort_keys(XbSortArgs a);
 __global__ void xb_sort_pass_key64(const uint64_t *col, const uint32_t *idx, uint64_t *out, uint32_t n);
 __global__ void xb_sort_pass_key8(const uint8_t *col, const uint32_t *idx, uint8_t *out, uint32_t n);
 __global__ void xb_sort_bounds(XbRankArgs a);
 __global__ void xb_sort_keepflag(XbKeepArgs a);
-__global__ void xb_sort_keep(XbKeepArgs a, const uint32_t *keep_scan, int64_t *keep);
+__global__ void xb_sort_keep(XbKeepArgs a, const uint32_t *keep_scan, uint32_t *list);
 __global__ void xb_iota_u32(uint32_t *out, uint32_t n);
 __global__ void __launch_bounds__(XB_BLOCK) xb_merge_final(XbMergeArgs args);
 __global__ void __launch_bounds__(XB_BLOCK) xb_inner_rebuild(XbRebuildArgs args);
