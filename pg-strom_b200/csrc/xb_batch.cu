@@ -142,8 +142,6 @@ static void xb_reset_groups(xpuB200Session *s)
     cudaStream_t st = s->stream;
     if (s->h_plan->has_groupby) {
         cudaMemsetAsync(s->h_gt.entries, 0, (s->h_gt.cap_mask + 1) * s->h_plan->gent_size, st);
-        if (s->h_gt.dump)
-            cudaMemsetAsync(s->h_gt.dump, 0, s->h_gt.dump_cap * s->h_plan->gent_size, st);
         s->h_gt.nused = 0;
         s->h_gt.arena_used = 0;
         s->h_gt.overflow = 0;

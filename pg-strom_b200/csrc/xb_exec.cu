@@ -3535,7 +3535,8 @@ static bool xb_part_prepare(xpuB200Session *s, uint64_t nunits, uint32_t format,
  * grow (two 32-row batches per warp: the one a warp is in when the request
  * comes, and one more if its look at the flag came just before; and the
  * groups the warps had not counted yet) when the table's free half is
- * smaller than twice those */
+ * smaller than twice those.  The entries are cleared as they are taken
+ * (xb_dump_slot): clearing the region was 45 MB a query */
 static int xb_dump_ensure(xpuB200Session *s, int grid, uint32_t sm_cap, cudaStream_t st, kern_errorbuf *err)
 {
     const uint64_t cap = s->h_gt.cap_mask + 1;
@@ -3560,7 +3561,6 @@ static int xb_dump_ensure(xpuB200Session *s, int grid, uint32_t sm_cap, cudaStre
         return XB_ERR(err, ERRCODE_DEVICE_FATAL, "out of device memory for the group dump (%llu entries)",
                       (unsigned long long)need);
     }
-    cudaMemsetAsync(d, 0, need * gsz, st);
     if (s->h_gt.dump)
         cudaFreeAsync(s->h_gt.dump, st);
     s->h_gt.dump = d;
@@ -3665,10 +3665,8 @@ int xb_gt_grow(xpuB200Session *s, uint64_t min_entries, kern_errorbuf *err)
     ga.arena_new = arena_new;
     const int grid = s->dev->nsm * 8;
     xb_gt_rehash<<<grid, XB_BLOCK, 0, st>>>(ga);
-    if (ndump) {
+    if (ndump)
         xb_gt_merge_dump<<<grid, XB_BLOCK, 0, st>>>(ga);
-        cudaMemsetAsync(g.dump, 0, ndump * gsz, st);
-    }
     cudaError_t lrc = cudaGetLastError();
     if (lrc != cudaSuccess)
         return XB_ERR(err, ERRCODE_DEVICE_FATAL, "group table growth: %s", cudaGetErrorString(lrc));

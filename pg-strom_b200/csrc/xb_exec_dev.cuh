@@ -159,7 +159,12 @@ __device__ __forceinline__ char *xb_dump_slot(xb_gtable *gt, uint32_t gent_size)
         return nullptr;
     xb_gt_want_grow(gt);
     const unsigned long long i = atomicAdd((unsigned long long *)&gt->dump_used, 1ULL);
-    return i < gt->dump_cap ? gt->dump + i * (uint64_t)gent_size : nullptr;
+    if (i >= gt->dump_cap)
+        return nullptr;
+    char *e = gt->dump + i * (uint64_t)gent_size;
+    for (uint32_t w = 0; w < gent_size / 8; w++)
+        ((uint64_t *)e)[w] = 0;
+    return e;
 }
 
 /* L2 prefetch of a contiguous range by the TMA engine (sm_90+) */

@@ -442,20 +442,28 @@ struct Gen {
      * the column descriptors as constants (the launch's columns are checked
      * once per CTA: lay_ok): the sequential walk of the general decode,
      * alignment before fixed-width columns and before varlenas that start
-     * with a pad byte, NULL-bitmap tests when the tuple has one.  Without a
-     * bitmap the offsets up to the first varlena are constants. */
-    void walk_body(bool nulls, const char *ind)
+     * with a pad byte, a column skipped where the tuple's NULL bitmap says
+     * so.  Tuples without a bitmap take the same code with every bit set: a
+     * walk of their own with constant offsets was a second pass for most
+     * warps (5% of NULLs leave a NULL in four of five 32-row batches).
+     * Queries over 4M rows 541 -> 494 us, every statistic over 2M 1046 ->
+     * 1008 us (with the dump region no longer cleared). */
+    void walk()
     {
+        o << "__device__ __forceinline__ bool\n"
+             "xbj_walk(XbjRegs &R, const uint8_t *pay, const uint32_t plen, const uint8_t *nullmap)\n{\n"
+             "    uint32_t o = 0;\n";
+        for (uint32_t j = 0; j < p->walk_ncols; j += 8)
+            o << "    const uint32_t nb" << j / 8 << " = nullmap ? nullmap[" << j / 8 << "] : 0xffu;\n";
         for (uint32_t j = 0; j < p->walk_ncols; j++) {
             const int len = p->walk_len[j], al = p->walk_align[j];
             std::vector<uint32_t> ls;
             for (uint32_t i = 0; i < p->nload0; i++)
                 if (p->load0[i].resno == (int)j + 1)
                     ls.push_back(i);
-            const std::string in = std::string(ind) + (nulls ? "    " : "");
-            o << ind << "/* column " << j + 1 << ": attlen " << len << ", attalign " << al << " */\n";
-            if (nulls)
-                o << ind << "if ((nullmap[" << j / 8 << "] >> " << j % 8 << ") & 1) {\n";
+            const std::string in = "        ";
+            o << "    /* column " << j + 1 << ": attlen " << len << ", attalign " << al << " */\n"
+                 "    if ((nb" << j / 8 << " >> " << j % 8 << ") & 1) {\n";
             if (len > 0) {
                 if (al > 1)
                     o << in << "o = (o + " << al - 1 << "u) & ~" << al - 1 << "u;\n";
@@ -485,30 +493,16 @@ struct Gen {
                 o << in << "    o += sz_;\n"
                   << in << "}\n";
             }
-            if (nulls) {
-                o << ind << "}";
-                if (!ls.empty()) {
-                    o << " else {\n";
-                    for (uint32_t i : ls)
-                        o << ind << "    " << N(p->load0[i].reg) << " = true;\n";
-                    o << ind << "}";
-                }
-                o << "\n";
+            o << "    }";
+            if (!ls.empty()) {
+                o << " else {\n";
+                for (uint32_t i : ls)
+                    o << in << N(p->load0[i].reg) << " = true;\n";
+                o << "    }";
             }
+            o << "\n";
         }
-    }
-
-    void walk()
-    {
-        o << "__device__ __forceinline__ bool\n"
-             "xbj_walk(XbjRegs &R, const uint8_t *pay, const uint32_t plen, const uint8_t *nullmap)\n{\n"
-             "    uint32_t o = 0;\n"
-             "    if (!nullmap) {\n";
-        walk_body(false, "        ");
-        o << "    } else {\n";
-        walk_body(true, "        ");
-        o << "    }\n"
-             "    (void)o;\n"
+        o << "    (void)o;\n"
              "    return true;\n}\n\n";
     }
 
