@@ -453,8 +453,6 @@ struct Gen {
         o << "__device__ __forceinline__ bool\n"
              "xbj_walk(XbjRegs &R, const uint8_t *pay, const uint32_t plen, const uint8_t *nullmap)\n{\n"
              "    uint32_t o = 0;\n";
-        for (uint32_t j = 0; j < p->walk_ncols; j += 8)
-            o << "    const uint32_t nb" << j / 8 << " = nullmap ? nullmap[" << j / 8 << "] : 0xffu;\n";
         for (uint32_t j = 0; j < p->walk_ncols; j++) {
             const int len = p->walk_len[j], al = p->walk_align[j];
             std::vector<uint32_t> ls;
@@ -463,7 +461,7 @@ struct Gen {
                     ls.push_back(i);
             const std::string in = "        ";
             o << "    /* column " << j + 1 << ": attlen " << len << ", attalign " << al << " */\n"
-                 "    if ((nb" << j / 8 << " >> " << j % 8 << ") & 1) {\n";
+                 "    if (!nullmap || ((nullmap[" << j / 8 << "] >> " << j % 8 << ") & 1)) {\n";
             if (len > 0) {
                 if (al > 1)
                     o << in << "o = (o + " << al - 1 << "u) & ~" << al - 1 << "u;\n";
