@@ -3371,6 +3371,26 @@ void *xb_session_jit(xpuB200Session *s, uint32_t format, bool wait)
     return s->jit_fn[format];
 }
 
+/* table slots of one bucket of partitioned aggregation: a slice of the table
+ * that two CTAs of an SM hold in shared memory (1024 of the Arrow group-by's
+ * 112-byte entries); XPU_B200_PART_SLOTS=n (a power of two, 64..65536) sets
+ * it (a slice that does not fit is replayed in L2) */
+static uint32_t xb_replay_slots(const xb_plan *plan)
+{
+    static const uint32_t forced = [] {
+        const char *e = getenv("XPU_B200_PART_SLOTS");
+        const unsigned long v = e ? strtoul(e, nullptr, 10) : 0;
+        return (v >= 64 && v <= 65536 && (v & (v - 1)) == 0) ? (uint32_t)v : 0u;
+    }();
+    if (forced)
+        return forced;
+    const uint64_t gsz = plan->gent_size ? plan->gent_size : 16;
+    uint32_t c = 8192;
+    while (c > 64 && c * gsz > XB_SLICE_BYTES)
+        c >>= 1;
+    return c;
+}
+
 /* the kernels just found or built (rc 0), or the reason there are none */
 static void xb_session_adopt_jit(xpuB200Session *s, uint32_t format, int rc, double ms, const char *msg)
 {
@@ -3400,6 +3420,12 @@ static void xb_session_adopt_jit(xpuB200Session *s, uint32_t format, int rc, dou
             if (s->jit_replay[format] && xb_jit_prepare(s->jit_replay[format], XB_BLOCK, 0, &rp) != 0)
                 s->jit_replay[format] = nullptr;
             s->jit_replay_grid[format] = rp * s->dev->nsm;
+            /* slices of the table in shared memory, where they fit */
+            const size_t sb = (size_t)xb_replay_slots(s->h_plan) * s->h_plan->gent_size;
+            s->jit_slice[format] = sb <= XB_SLICE_BYTES ? xb_jit_slice_of(s->jit_replay[format]) : nullptr;
+            if (s->jit_slice[format] && xb_jit_prepare(s->jit_slice[format], XB_SLICE_BLOCK, sb, &rp) != 0)
+                s->jit_slice[format] = nullptr;
+            s->jit_slice_grid[format] = rp * s->dev->nsm;
             s->jit_compile_ms += ms;
             s->jit_msg = "ok";
         }
@@ -3426,26 +3452,6 @@ static int xb_launch_tasks(xpuB200Session *s, const xb_task *d_tasks, uint32_t n
  * that rows past full buckets are updated in place while others of the
  * same groups are deferred.  Session lock held.  Returns whether it is
  * used. */
-/* table slots of one bucket of partitioned aggregation: about 128 KB of
- * global table (1024 of the Arrow group-by's 112-byte entries; measured
- * against 512, 2048 and 4096 slots); XPU_B200_PART_SLOTS=n (a power of two,
- * 64..65536) sets it */
-static uint32_t xb_replay_slots(const xb_plan *plan)
-{
-    static const uint32_t forced = [] {
-        const char *e = getenv("XPU_B200_PART_SLOTS");
-        const unsigned long v = e ? strtoul(e, nullptr, 10) : 0;
-        return (v >= 64 && v <= 65536 && (v & (v - 1)) == 0) ? (uint32_t)v : 0u;
-    }();
-    if (forced)
-        return forced;
-    const uint64_t gsz = plan->gent_size ? plan->gent_size : 16;
-    uint32_t c = 8192;
-    while (c > 64 && c * gsz > (128u << 10))
-        c >>= 1;
-    return c;
-}
-
 static bool xb_part_prepare(xpuB200Session *s, uint64_t nunits, uint32_t format, cudaStream_t stream)
 {
     const char *env = getenv("XPU_B200_PARTITION");
@@ -3493,9 +3499,9 @@ static bool xb_part_prepare(xpuB200Session *s, uint64_t nunits, uint32_t format,
         s->part_cnt = nullptr;
         s->part_bytes = 0;
         if (cudaMallocAsync((void **)&s->part_buf, bytes, stream) != cudaSuccess ||
-            /* the bucket counters, then the replay's bucket cursor */
-            cudaMallocAsync((void **)&s->part_cnt, sizeof(uint32_t) * XB_PART_CNT_STRIDE * (np + 1), stream) !=
-                cudaSuccess) {
+            /* the bucket counters, a line of the replay's own (XB_RP_*), the spill list */
+            cudaMallocAsync((void **)&s->part_cnt, sizeof(uint32_t) * XB_PART_CNT_STRIDE * (np + 1) +
+                            sizeof(uint2) * XB_SPILL_CAP, stream) != cudaSuccess) {
             cudaGetLastError();
             if (s->part_buf) cudaFreeAsync(s->part_buf, stream);
             s->part_buf = nullptr;
@@ -3532,15 +3538,14 @@ static bool xb_part_prepare(xpuB200Session *s, uint64_t nunits, uint32_t format,
 
 /* the dump region, sized for a launch of 'grid' CTAs: every CTA's shared
  * table merged at exit, plus the rows in flight after the table asked to
- * grow (two 32-row batches per warp: the one a warp is in when the request
- * comes, and one more if its look at the flag came just before; and the
- * groups the warps had not counted yet) when the table's free half is
- * smaller than twice those.  The entries are cleared as they are taken
- * (xb_dump_slot): clearing the region was 45 MB a query */
+ * grow (XB_INFLIGHT per warp, and the groups the warps had not counted yet)
+ * when the table's free half is smaller than twice those.  The entries are
+ * cleared as they are taken (xb_dump_slot): clearing the region was 45 MB a
+ * query */
 static int xb_dump_ensure(xpuB200Session *s, int grid, uint32_t sm_cap, cudaStream_t st, kern_errorbuf *err)
 {
     const uint64_t cap = s->h_gt.cap_mask + 1;
-    const uint64_t inflight = (uint64_t)grid * XB_WARPS * (64 + XB_UNCOUNTED);
+    const uint64_t inflight = (uint64_t)grid * XB_WARPS * (XB_INFLIGHT + XB_UNCOUNTED);
     uint64_t need = (uint64_t)grid * sm_cap;
     if (cap / 2 < 2 * inflight)
         need += inflight;
@@ -3785,10 +3790,24 @@ int xb_launch_on(xpuB200Session *s, const xb_task *d_tasks, uint32_t ntasks,
             ra.part_cnt = s->part_cnt;
             ra.part_cap = s->part_cap;
             ra.nparts = s->nparts;
-            ra.cursor = s->part_cnt + (size_t)s->nparts * XB_PART_CNT_STRIDE;
+            uint32_t *line = s->part_cnt + (size_t)s->nparts * XB_PART_CNT_STRIDE;
+            ra.cursor = line;
             ra.part_shift = s->part_shift;
-            if (xb_jit_launch(s->jit_replay[format], s->jit_replay_grid[format], XB_BLOCK, 0, (void *)stream,
-                              &ra) != 0)
+            ra.nspill = line + XB_RP_SPILL;
+            ra.nused0 = (const uint64_t *)(line + XB_RP_NUSED);
+            ra.spill = (uint2 *)(line + XB_PART_CNT_STRIDE);
+            ra.spill_cap = XB_SPILL_CAP;
+            const size_t sb = (size_t)s->h_plan->gent_size << s->part_shift;
+            int lrc;
+            if (s->jit_slice[format] && s->part_shift <= (uint32_t)__builtin_ctz(xb_replay_slots(s->h_plan))) {
+                cudaMemcpyAsync(line + XB_RP_NUSED, &s->d_gt->nused, 8, cudaMemcpyDeviceToDevice, stream);
+                lrc = xb_jit_launch(s->jit_slice[format], s->jit_slice_grid[format], XB_SLICE_BLOCK, sb, (void *)stream, &ra);
+                ra.spilled = 1;
+            } else {
+                lrc = 0;
+            }
+            if (lrc != 0 || xb_jit_launch(s->jit_replay[format], s->jit_replay_grid[format], XB_BLOCK, 0,
+                                          (void *)stream, &ra) != 0)
                 return XB_ERR(err, ERRCODE_DEVICE_FATAL, "replay kernel launch failed");
             cudaEventRecord(s->ev_part[2], stream);
         }

@@ -141,6 +141,10 @@ __device__ __forceinline__ void xb_gt_want_grow(xb_gtable *gt)
 /* new global entries a warp of a specialised kernel may leave uncounted
  * between 32-row batches */
 #define XB_UNCOUNTED    31
+/* rows a warp may still apply after the table asked to grow: the 32 it is
+ * applying, 32 more if its look at the request came just before, and the
+ * rows that wait in its queue (31) */
+#define XB_INFLIGHT     95
 
 /* count new entries of the global table; once soft_cap entries are in use
  * the table asks to grow */
@@ -601,7 +605,22 @@ struct XbReplayArgs {
     uint32_t        nparts;
     uint32_t        retry;          /* replay only the records marked left */
     uint32_t        part_shift;     /* a bucket holds 1 << part_shift table slots */
+    /* records whose probe left their bucket's slice of the table, found by
+     * xbj_replay_slice and replayed on the whole table after it */
+    uint2          *spill;          /* (bucket, record) */
+    uint32_t       *nspill;
+    uint32_t        spill_cap;
+    uint32_t        spilled;        /* xbj_replay: replay the spill list */
+    const uint64_t *nused0;         /* groups in the table before the replay */
 };
+
+#define XB_SLICE_BLOCK      512     /* threads of xbj_replay_slice, two CTAs per SM */
+#define XB_SLICE_BYTES      115648u /* a table slice in shared memory: 2 per SM */
+#define XB_SPILL_CAP        (1u << 20)
+/* words of the line after the bucket counters: the bucket cursor, the spill
+ * list's length, the table's groups before the replay (8 bytes) */
+#define XB_RP_SPILL         8
+#define XB_RP_NUSED         16
 
 /* largest existence bitmap of a direct depth (keys), 16 KB */
 #define XB_DBITS_MAX_KEYS   (1u << 17)

@@ -156,6 +156,8 @@ struct xpuB200Session {
     /* partitioned aggregation: deferred rows bucketed by table slot */
     void           *jit_replay[256] = {nullptr};
     int             jit_replay_grid[256] = {0};
+    void           *jit_slice[256] = {nullptr};
+    int             jit_slice_grid[256] = {0};
     char           *part_buf = nullptr;
     uint32_t       *part_cnt = nullptr;
     uint64_t        part_bytes = 0;

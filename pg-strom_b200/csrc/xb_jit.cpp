@@ -1306,36 +1306,139 @@ struct Gen {
     /* record: hash (4) + NULL mask (4; bit 31 marks a record a replay left
      * for after the table grows) + values (8 each) + the aux words of text /
      * numeric keys (4 each); the key hash is in the record already, so
-     * cached datum hashes are not */
+     * cached datum hashes are not.  Written and read as 16-byte words: every
+     * store of a lane is a request to L2 of its own. */
     uint32_t part_rec_size() const
     {
         const size_t n = part_regs().size();
-        return (uint32_t)((8 + 8 * n + 4 * part_aux_keys().size() + 7) & ~(size_t)7);
+        return (uint32_t)((8 + 8 * n + 4 * part_aux_keys().size() + 15) & ~(size_t)15);
     }
 
     void part_helpers()
     {
-        const std::vector<int> rr = part_regs();
+        const std::vector<int> rr = part_regs(), ax = part_aux_keys();
+        /* the record's 8-byte words */
+        std::vector<std::string> w = {"((uint64_t)nm << 32) | ghash"};
+        for (int r : rr)
+            w.push_back(V(r));
+        for (size_t k = 0; k < ax.size(); k += 2)
+            w.push_back("(uint64_t)" + A(ax[k]) + (k + 1 < ax.size() ? " | ((uint64_t)" + A(ax[k + 1]) + " << 32)" : ""));
+        if (w.size() & 1)
+            w.push_back("0");
         o << "__device__ __forceinline__ void xbj_rec_store(char *rec, const XbjRegs &R, uint32_t ghash)\n{\n"
              "    uint32_t nm = 0;\n";
         for (size_t i = 0; i < rr.size(); i++)
-            o << "    nm |= (R.n[" << rr[i] << "] ? 1u : 0u) << " << i << ";\n";
-        o << "    uint2 hd; hd.x = ghash; hd.y = nm;\n"
-             "    *(uint2 *)rec = hd;\n";
-        for (size_t i = 0; i < rr.size(); i++)
-            o << "    *(uint64_t *)(rec + " << 8 + 8 * i << ") = R.v[" << rr[i] << "];\n";
-        const std::vector<int> ax = part_aux_keys();
-        for (size_t k = 0; k < ax.size(); k++)
-            o << "    *(uint32_t *)(rec + " << 8 + 8 * rr.size() + 4 * k << ") = R.a[" << ax[k] << "];\n";
+            o << "    nm |= (" << N(rr[i]) << " ? 1u : 0u) << " << i << ";\n";
+        for (size_t i = 0; i < w.size(); i += 2)
+            o << "    ((ulonglong2 *)rec)[" << i / 2 << "] = make_ulonglong2(" << w[i] << ", " << w[i + 1] << ");\n";
         o << "}\n\n"
-             "__device__ __forceinline__ void xbj_rec_load(const char *rec, XbjRegs &R, uint32_t &ghash)\n{\n"
-             "    const uint2 hd = *(const uint2 *)rec;\n"
-             "    ghash = hd.x;\n";
+             "__device__ __forceinline__ void xbj_rec_load(const char *rec, XbjRegs &R, uint32_t &ghash)\n{\n";
+        for (size_t i = 0; i < w.size(); i += 2)
+            o << "    const ulonglong2 q" << i / 2 << " = ((const ulonglong2 *)rec)[" << i / 2 << "];\n";
+        auto word = [&](size_t i) { return "q" + std::to_string(i / 2) + (i & 1 ? ".y" : ".x"); };
+        o << "    const uint32_t nm = (uint32_t)(q0.x >> 32); (void)nm;\n"
+             "    ghash = (uint32_t)q0.x;\n";
         for (size_t i = 0; i < rr.size(); i++)
-            o << "    R.v[" << rr[i] << "] = *(const uint64_t *)(rec + " << 8 + 8 * i << ");\n"
-                 "    R.n[" << rr[i] << "] = (hd.y >> " << i << ") & 1u;\n";
+            o << "    " << V(rr[i]) << " = " << word(1 + i) << "; " << A(rr[i]) << " = 0; " << N(rr[i]) << " = (nm >> " << i
+              << ") & 1u;\n";
         for (size_t k = 0; k < ax.size(); k++)
-            o << "    R.a[" << ax[k] << "] = *(const uint32_t *)(rec + " << 8 + 8 * rr.size() + 4 * k << ");\n";
+            o << "    " << A(ax[k]) << " = (uint32_t)(" << word(1 + rr.size() + k / 2) << (k & 1 ? " >> 32" : "") << ");\n";
+        o << "}\n\n";
+    }
+
+    /* the lookup in and update of a slice of the global table in shared
+     * memory (global-form states): counts and integer sums by native 32-bit
+     * atomics with carries, min and max only where they change something */
+    void slice_helpers()
+    {
+        o << "__device__ __forceinline__ char *\n"
+             "xbj_slice_get(const XbjRegs &R, const XbjEnv &E, char *slice, uint32_t pos, uint32_t nslots, uint32_t hash, "
+             "bool &failed)\n{\n"
+             "    for (uint32_t probe = 0; pos < nslots && probe <= XB_PROBE_LIMIT; probe++, pos++) {\n"
+             "        char *e = slice + (size_t)pos * XBJ_GENT_SIZE;\n"
+             "        xb_gent_head *h = (xb_gent_head *)e;\n"
+             "        uint32_t s = xb_ld_acquire_cta(&h->state);\n"
+             "        if (s == XB_GSTATE_EMPTY) {\n"
+             "            const int rc = xbj_group_claim(e, hash, E.gt, E.st, E.newg";
+        for (uint32_t k = 0; k < p->nkeys; k++) {
+            const int r = p->keys[k].reg;
+            o << ", " << V(r) << ", " << A(r) << ", " << N(r);
+        }
+        o << ");\n"
+             "            if (rc == 1) return e;\n"
+             "            if (rc == 2) { failed = true; return nullptr; }\n"
+             "            s = xb_ld_acquire_cta(&h->state);\n"
+             "        }\n"
+             "        uint32_t spins = 0;\n"
+             "        while (s == XB_GSTATE_BUSY) {\n"
+             "            if (++spins > E.plan->wait_limit) {\n"
+             "                XB_RAISE(E.st, ERRCODE_DEVICE_ERROR, XB_MSG_WAIT_TIMEOUT);\n"
+             "                failed = true;\n"
+             "                return nullptr;\n            }\n"
+             "            __nanosleep(20);\n"
+             "            s = xb_ld_acquire_cta(&h->state);\n"
+             "        }\n"
+             "        if (h->hash == hash && xbj_key_match(e, R))\n            return e;\n"
+             "    }\n"
+             "    return nullptr;\n}\n\n"
+             "__device__ __forceinline__ void xbj_update_slice(char *e, const XbjRegs &R, const XbjEnv &E)\n{\n"
+             "    (void)E;\n" << numeric_args();
+        for (uint32_t i = 0; i < p->naggs; i++) {
+            const xb_agg &a = p->aggs[i];
+            if (a.state_sz == 0)
+                continue;
+            const AggExpr x = agg_expr(a);
+            const std::string S = "(e + " + std::to_string(a.state_off) + ")";
+            o << "    { /* aggregate " << i << ": action " << a.action << " */\n";
+            switch (a.action) {
+            case KAGG_ACTION__NROWS_ANY: case KAGG_ACTION__NROWS_COND:
+                o << "        if (" << (a.action == KAGG_ACTION__NROWS_ANY ? x.f : x.c) << ") xb_shared_add_u64w(" << S << ", 1);\n";
+                break;
+            case KAGG_ACTION__PMIN_INT32: case KAGG_ACTION__PMIN_INT64: case KAGG_ACTION__PMIN_FP64:
+            case KAGG_ACTION__PMAX_INT32: case KAGG_ACTION__PMAX_INT64: case KAGG_ACTION__PMAX_FP64: {
+                const bool is_min = a.action == KAGG_ACTION__PMIN_INT32 || a.action == KAGG_ACTION__PMIN_INT64 ||
+                                    a.action == KAGG_ACTION__PMIN_FP64;
+                const bool fp = a.action == KAGG_ACTION__PMIN_FP64 || a.action == KAGG_ACTION__PMAX_FP64;
+                o << "        if (" << x.c << ") {\n"
+                     "            const long long v_ = " << (fp ? "(long long)xb_f64_ordered(" + x.xd + ")" : "(long long)" + V(a.arg0))
+                  << ";\n"
+                     "            if (!*(volatile uint32_t *)(" << S << " + 8)) atomicOr((unsigned int *)(" << S << " + 8), 1u);\n"
+                     "            if (v_ " << (is_min ? "<" : ">") << " *(volatile long long *)" << S << ") "
+                  << (is_min ? "atomicMin" : "atomicMax") << "((long long *)" << S << ", v_);\n"
+                     "        }\n";
+                break;
+            }
+            case KAGG_ACTION__PSUM_INT: case KAGG_ACTION__PAVG_INT:
+                o << "        if (" << x.c << ") {\n"
+                     "            xb_shared_add_u64w(" << S << ", 1);\n"
+                     "            xb_shared_add_u64w(" << S << " + 8, (uint64_t)" << V(a.arg0) << ");\n        }\n";
+                break;
+            case KAGG_ACTION__PSUM_INT64: case KAGG_ACTION__PAVG_INT64:
+                o << "        if (" << x.c << ") {\n"
+                     "            xb_shared_add_u64w(" << S << ", 1);\n"
+                     "            xb_shared_add_i128w(" << S << " + 8, (xb_i128)(int64_t)" << V(a.arg0) << ");\n        }\n";
+                break;
+            case KAGG_ACTION__PSUM_NUMERIC: case KAGG_ACTION__PAVG_NUMERIC:
+                o << "        if (" << x.c << ") {\n"
+                     "            if (k" << num_id(a) << " == XB_NUM_VALID) {\n"
+                     "                xb_shared_add_u64w(" << S << ", 1);\n"
+                     "                xb_shared_add_i128w(" << S << " + 8, x" << num_id(a) << ");\n"
+                     "            } else {\n"
+                     "                atomicOr((unsigned int *)(" << S << " + 24), xb_numeric_special(k" << num_id(a) << "));\n"
+                     "            }\n        }\n";
+                break;
+            case KAGG_ACTION__PSUM_FP: case KAGG_ACTION__PAVG_FP:
+                o << "        if (" << x.c << ") {\n"
+                     "            xb_shared_add_u64w(" << S << ", 1);\n"
+                     "            xb_atomic_add_f64c((double *)(" << S << " + 8), (double *)(" << S << " + 16), " << x.xd
+                  << ");\n        }\n";
+                break;
+            default:
+                helper_update(a, S, x.c, x.xd, x.yd);
+                break;
+            }
+            o << "    }\n";
+        }
         o << "}\n\n";
     }
 
@@ -1829,14 +1932,26 @@ struct Gen {
         }
     }
 
+    /* ---- Arrow rows: compaction between the scan quals and the rest ----
+     * The numbers of the rows that pass wait in a queue of the warp in
+     * shared memory until 32 are there, so that the group lookup and the
+     * updates run with every lane, and the columns that the quals do not
+     * read are loaded for rows that passed only.  20M rows into
+     * 1.7M groups 2314 -> 1772 us a query, 500M rows into 10M groups 23.8 ->
+     * 22.2 ms.  Heap rows, which would be decoded twice, lost 3 to 14% by
+     * it, and an aggregate without keys has too little to do per row. */
+    bool compact() const
+    {
+        return false;
+    }
+
     void pipeline()
     {
-        o << "__device__ __forceinline__ void\n"
-             "xbj_pipeline(XbjRegs &R, const XbjEnv &E, XbjCnt &C, bool &failed)\n{\n";
+        o << "__device__ __forceinline__ bool xbj_quals(XbjRegs &R, const XbjEnv &E, bool &failed)\n{\n    (void)E;\n";
         program(p->scan_quals, "    ");
-        o << "    if (failed) return;\n"
-             "    if (!" << pass_expr(p->scan_quals) << ") return;\n"
-             "    C.in++;\n";
+        o << "    return !failed && " << pass_expr(p->scan_quals) << ";\n}\n\n"
+             "__device__ __forceinline__ void\n"
+             "xbj_after_quals(XbjRegs &R, const XbjEnv &E, XbjCnt &C, bool &failed)\n{\n";
         preload_probes("    ");
         depth(1, "    ");
         o << "}\n";
@@ -1882,6 +1997,8 @@ struct Gen {
           << (any_bits() ? "#define XBJ_BITS 1\n" : "");
         if (part_mode())
             o << "#define XBJ_PART 1\n#define XBJ_REC_SIZE " << part_rec_size() << "\n";
+        if (compact())
+            o << "#define XBJ_COMPACT 1\n";
         if (format == KDS_FORMAT_ARROW && p->nload0 > 0)
             o << "#define XBJ_ACOLS " << p->nload0 << "\n";
         o << "struct XbjRegs {\n"
@@ -1910,8 +2027,10 @@ struct Gen {
             group_helpers();
             if (p->has_groupby == 1)
                 group_row();
-            if (part_mode())
+            if (part_mode()) {
                 part_helpers();
+                slice_helpers();
+            }
         }
         pipeline();
         /* the kernels that call generated functions defined above */
@@ -1942,6 +2061,7 @@ struct CacheEntry {
     CUfunction fn = nullptr;
     CUfunction fn_mix = nullptr;
     CUfunction fn_replay = nullptr;     /* partitioned aggregation's replay, if built */
+    CUfunction fn_slice = nullptr;      /* and its form on slices in shared memory */
     double compile_ms = 0.0;
 };
 std::map<std::pair<int, std::string>, CacheEntry> g_cache;
@@ -2164,8 +2284,9 @@ jit_build(const xb_plan *plan, uint32_t format, int dindex, int min_blocks, bool
     if (g_drv.getfn(&ce.fn, ce.mod, "xbj_kernel") != CUDA_SUCCESS ||
         g_drv.getfn(&ce.fn_mix, ce.mod, "xbj_mixed_kernel") != CUDA_SUCCESS)
         return fail("cuModuleGetFunction(xbj_kernel) failed");
-    if (want_replay && g_drv.getfn(&ce.fn_replay, ce.mod, "xbj_replay") != CUDA_SUCCESS)
-        ce.fn_replay = nullptr;
+    if (want_replay && (g_drv.getfn(&ce.fn_replay, ce.mod, "xbj_replay") != CUDA_SUCCESS ||
+                        g_drv.getfn(&ce.fn_slice, ce.mod, "xbj_replay_slice") != CUDA_SUCCESS))
+        ce.fn_replay = ce.fn_slice = nullptr;
     g_cache[key] = ce;
     return give(ce, ce.compile_ms);
 }
@@ -2269,6 +2390,16 @@ extern "C" void
 xb_jit_job_release(void *h)
 {
     delete (std::shared_ptr<JitJob> *)h;
+}
+
+extern "C" void *
+xb_jit_slice_of(void *replay)
+{
+    std::lock_guard<std::mutex> guard(g_lock);
+    for (const auto &kv : g_cache)
+        if (replay && (void *)kv.second.fn_replay == replay)
+            return (void *)kv.second.fn_slice;
+    return nullptr;
 }
 
 extern "C" int

@@ -61,6 +61,10 @@ void  xb_jit_job_release(void *job);
  * xb_jit_compile_minb's p_replay */
 uint32_t xb_jit_part_rec_size(const xb_plan *plan, uint32_t format);
 
+/* the kernel that replays on slices of the table in shared memory
+ * (xbj_replay_slice, the same parameter block) built with 'replay' */
+void *xb_jit_slice_of(void *replay);
+
 /* a key naming the plan shape of plan + format: sessions whose specialised
  * kernels differ only in their launch bounds share it */
 uint64_t xb_jit_shape_key(const xb_plan *plan, uint32_t format);

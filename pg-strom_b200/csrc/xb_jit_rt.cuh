@@ -127,8 +127,11 @@ __device__ __forceinline__ void xbj_prefetch_tuple(const uint8_t *page, uint32_t
     }
 }
 
+/* generated: does the row pass the scan quals; joins, grouping and
+ * projection of a row that did */
+__device__ __forceinline__ bool xbj_quals(XbjRegs &R, const XbjEnv &E, bool &failed);
 __device__ __forceinline__ void
-xbj_pipeline(XbjRegs &R, const XbjEnv &E, XbjCnt &C, bool &failed);
+xbj_after_quals(XbjRegs &R, const XbjEnv &E, XbjCnt &C, bool &failed);
 
 #ifdef XBJ_ACC
 /* generated: a lane's aggregate, empty at first; all lanes of a warp added
@@ -164,6 +167,11 @@ __device__ __forceinline__ void xbj_warp_two_sum(double &s, double &c)
  * (returns true when, replaying, the table had no room for the group) */
 __device__ __forceinline__ void xbj_rec_load(const char *rec, XbjRegs &R, uint32_t &ghash);
 __device__ __forceinline__ bool xbj_group_row(XbjRegs &R, const XbjEnv &E, const uint32_t ghash, bool &failed);
+/* generated: the row's entry in a slice of the table held in shared memory
+ * (nullptr: its probe leaves the slice), and its update there */
+__device__ __forceinline__ char *
+xbj_slice_get(const XbjRegs &R, const XbjEnv &E, char *slice, uint32_t pos, uint32_t nslots, uint32_t hash, bool &failed);
+__device__ __forceinline__ void xbj_update_slice(char *e, const XbjRegs &R, const XbjEnv &E);
 #endif
 
 #ifdef XBJ_MERGE_SM
@@ -229,6 +237,15 @@ __device__ __forceinline__ void xbj_grow_fetch(uint32_t *buf, const xb_gtable *g
                  "cp.async.commit_group;"
                  :: "r"((uint32_t)__cvta_generic_to_shared(buf)), "l"((const char *)gt + 48) : "memory");
 }
+
+/* the group table's growth request: lane 0 fetches it into shared memory by
+ * an asynchronous copy before rows are applied and looks at it after them,
+ * so no register is held and little latency is waited for; the rest of the
+ * warp's work is then left for the resume launch */
+#define XBJ_GROW_FETCH() \
+    do { if (args.left_out && lane == 0) xbj_grow_fetch(src.grow_buf, args.gt); } while (0)
+#define XBJ_GROW_SEEN() \
+    (args.left_out && __shfl_sync(XB_FULL, xbj_grow_seen(src.grow_buf, lane), 0))
 
 /* lane 0: the fetched 'grow' word, once its copy has landed */
 __device__ __forceinline__ uint32_t xbj_grow_seen(const uint32_t *buf, uint32_t lane)
@@ -340,124 +357,179 @@ xbj_body(const XbExecArgs &args, char *smem)
      * being pulled into L1 while this batch runs; the line pointers of the
      * batch after that are in flight */
     uint32_t lp_next = 0, lp_after = 0;
+#ifdef XBJ_COMPACT
+    /* rows of the current unit that passed the quals wait here (up to 31,
+     * while 32 more are filtered), the last ones taken first */
+    __shared__ uint32_t queue_all[XB_WARPS][64];
+    uint32_t *queue = queue_all[threadIdx.x >> 5];
+    uint32_t qn = 0;
+#endif
+    bool done = false;          /* no more units */
+    bool stop = false;          /* the table is to grow */
 
     for (;;) {
-        bool done = false;
-        while (item >= nitems) {
-            const int rc = xb_next_unit(args, src, lane, args.format == KDS_FORMAT_ROW);
-            if (rc == 0) { done = true; break; }
-            if (rc == 2) {
-                if (lane == 0) XB_RAISE(args.st, ERRCODE_DEVICE_ERROR, XB_MSG_BAD_PAGE);
-                done = true;
+        bool failed = false;
+#ifdef XBJ_COMPACT
+        if (!done && !stop && qn < 32 && !(qn && item >= nitems)) {
+#else
+        {
+            if (stop)
                 break;
-            }
-            page = src.page;
-            kds = src.kds;
-            row0 = src.row0;
-            item = src.item;            /* 0, or where a resumed range starts */
-            nitems = src.nitems;
-#ifdef XBJ_STAGE
-            staged = false;
-            if ((((uintptr_t)page) & 15) == 0) {
-                __syncwarp();           /* every lane is done with the buffer */
-                if (lane == 0)
-                    xbj_stage_issue(sbuf, page, mbar);
-                __syncwarp();
-                const bool ok_ = xbj_stage_wait(mbar, sphase);
-                sphase ^= 1u;
-                if (!__all_sync(XB_FULL, ok_)) {
-                    if (lane == 0) XB_RAISE(args.st, ERRCODE_DEVICE_ERROR, XB_MSG_WAIT_TIMEOUT);
-                    /* the copy is still owed to this barrier: wait once more */
-                    xbj_stage_wait(mbar, sphase ^ 1u);
+#endif
+            while (item >= nitems) {
+                const int rc = xb_next_unit(args, src, lane, args.format == KDS_FORMAT_ROW);
+                if (rc == 0) { done = true; break; }
+                if (rc == 2) {
+                    if (lane == 0) XB_RAISE(args.st, ERRCODE_DEVICE_ERROR, XB_MSG_BAD_PAGE);
                     done = true;
                     break;
                 }
-                page = (const uint8_t *)sbuf;
-                staged = true;
+                page = src.page;
+                kds = src.kds;
+                row0 = src.row0;
+                item = src.item;            /* 0, or where a resumed range starts */
+                nitems = src.nitems;
+#ifdef XBJ_STAGE
+                staged = false;
+                if ((((uintptr_t)page) & 15) == 0) {
+                    __syncwarp();           /* every lane is done with the buffer */
+                    if (lane == 0)
+                        xbj_stage_issue(sbuf, page, mbar);
+                    __syncwarp();
+                    const bool ok_ = xbj_stage_wait(mbar, sphase);
+                    sphase ^= 1u;
+                    if (!__all_sync(XB_FULL, ok_)) {
+                        if (lane == 0) XB_RAISE(args.st, ERRCODE_DEVICE_ERROR, XB_MSG_WAIT_TIMEOUT);
+                        /* the copy is still owed to this barrier: wait once more */
+                        xbj_stage_wait(mbar, sphase ^ 1u);
+                        done = true;
+                        break;
+                    }
+                    page = (const uint8_t *)sbuf;
+                    staged = true;
+                }
+#endif
+                if (args.format == KDS_FORMAT_BLOCK) {
+                    lp_next = xbj_itemid(page, nitems, item + lane);
+                    lp_after = xbj_itemid(page, nitems, item + lane + 32);
+                }
+#ifdef XBJ_ACOLS
+                __syncwarp();           /* every lane is done with the last unit's columns */
+                xb_arrow_resolve(args.plan, kds, row0, nitems, acol, lane);
+                __syncwarp();
+#endif
+            }
+            if (done)
+#ifdef XBJ_COMPACT
+                continue;
+#else
+                break;
+#endif
+#ifndef XBJ_COMPACT
+            XBJ_GROW_FETCH();
+#endif
+            const uint32_t idx = item + lane;
+            uint32_t lp = 0;
+#ifdef XBJ_ACOLS
+            /* the columns' lines XBJ_ARROW_AHEAD batches ahead into L2: lane t
+             * takes line t % 2 of column t / 2 (32 values of at most 8 bytes) */
+            if (lane < 2 * XBJ_ACOLS) {
+                const XbArrowCol &c_ = acol[lane >> 1];
+                const uint32_t r_ = item + 32 * XBJ_ARROW_AHEAD;
+                /* the first row of the line: a row of the batch, inside the buffer */
+                const uint32_t rr_ = c_.width ? r_ + (lane & 1) * (128 / c_.width) : 0;
+                if (c_.ok && c_.width && rr_ < r_ + 32 && rr_ < c_.nvalid)
+                    asm volatile("prefetch.global.L2 [%0];" :: "l"(c_.values + (size_t)rr_ * c_.width));
             }
 #endif
+            /* the warp's next heap page streams into L2 while the last
+             * XBJ_PF_LEAD rows of this one are processed: early enough to
+             * arrive, late enough not to be evicted by the pages streaming
+             * through L2 meanwhile */
+            if (XBJ_PF_LEAD > 0 && args.format == KDS_FORMAT_BLOCK && item + XBJ_PF_LEAD >= nitems &&
+                (item < 32 || item + XBJ_PF_LEAD < nitems + 32))
+                xb_prefetch_page(args, src, xb_following_unit(src), lane);
             if (args.format == KDS_FORMAT_BLOCK) {
-                lp_next = xbj_itemid(page, nitems, item + lane);
-                lp_after = xbj_itemid(page, nitems, item + lane + 32);
+                lp = lp_next;
+                lp_next = lp_after;
+                /* (the fast decode of a known layout reads the tuple with two
+                 * wide loads; there the L1 prefetch only costs issue slots) */
+                if (!(lay_ok && XBJ_LAY_FIXED)
+#ifdef XBJ_STAGE
+                    && !staged
+#endif
+                    )
+                    xbj_prefetch_tuple(page, lp_next);
+                lp_after = xbj_itemid(page, nitems, idx + 64);
             }
-#ifdef XBJ_ACOLS
-            __syncwarp();           /* every lane is done with the last unit's columns */
-            xb_arrow_resolve(args.plan, kds, row0, nitems, acol, lane);
+            item += 32;
+#ifdef XBJ_COMPACT
+            bool pass = false;
+#endif
+            if (idx < nitems) {
+                XbjRegs R;
+                bool exists = false;
+                const bool ok = xbj_decode(R, args, page, kds, row0, meta, idx, lp, lay_ok, exists, args.st, acol);
+                if (exists)
+                    C.raw++;
+                if (exists && !ok) {
+                    failed = true;
+                } else if (ok && xbj_quals(R, E, failed)) {
+                    C.in++;
+#ifdef XBJ_COMPACT
+                    pass = true;
+#else
+                    xbj_after_quals(R, E, C, failed);
+#endif
+                }
+            }
+#ifdef XBJ_COMPACT
+            const uint32_t passed = __ballot_sync(XB_FULL, pass);
+            if (pass)
+                queue[qn + __popc(passed & ((1u << lane) - 1u))] = idx;
+            qn += __popc(passed);
             __syncwarp();
 #endif
+#ifndef XBJ_COMPACT
+            if (XBJ_GROW_SEEN())
+                stop = true;
+#endif
         }
-        if (done)
-            break;
-        /* the group table's growth request: lane 0 fetches it into shared
-         * memory by an asynchronous copy now and looks at it after the
-         * batch, so no register is held and no latency is waited for */
-        if (args.left_out && lane == 0)
-            xbj_grow_fetch(src.grow_buf, args.gt);
-        const uint32_t idx = item + lane;
-        uint32_t lp = 0;
-#ifdef XBJ_ACOLS
-        /* the columns' lines XBJ_ARROW_AHEAD batches ahead into L2: lane t
-         * takes line t % 2 of column t / 2 (32 values of at most 8 bytes) */
-        if (lane < 2 * XBJ_ACOLS) {
-            const XbArrowCol &c_ = acol[lane >> 1];
-            const uint32_t r_ = item + 32 * XBJ_ARROW_AHEAD;
-            /* the first row of the line: a row of the batch, inside the buffer */
-            const uint32_t rr_ = c_.width ? r_ + (lane & 1) * (128 / c_.width) : 0;
-            if (c_.ok && c_.width && rr_ < r_ + 32 && rr_ < c_.nvalid)
-                asm volatile("prefetch.global.L2 [%0];" :: "l"(c_.values + (size_t)rr_ * c_.width));
+#ifdef XBJ_COMPACT
+        else {
+            if (qn == 0)
+                break;
+            XBJ_GROW_FETCH();
+            const uint32_t n = qn < 32 ? qn : 32;
+            qn -= n;
+            if (lane < n) {
+                XbjRegs R;
+                bool exists = false;
+                xbj_decode(R, args, page, kds, row0, meta, queue[qn + lane], 0, lay_ok, exists, args.st, acol);
+                xbj_after_quals(R, E, C, failed);
+            }
+            __syncwarp();
+            if (XBJ_GROW_SEEN())
+                stop = true;
         }
 #endif
-        /* the warp's next heap page streams into L2 while the last
-         * XBJ_PF_LEAD rows of this one are processed: early enough to
-         * arrive, late enough not to be evicted by the pages streaming
-         * through L2 meanwhile */
-        if (XBJ_PF_LEAD > 0 && args.format == KDS_FORMAT_BLOCK && item + XBJ_PF_LEAD >= nitems &&
-            (item < 32 || item + XBJ_PF_LEAD < nitems + 32))
-            xb_prefetch_page(args, src, xb_following_unit(src), lane);
-        if (args.format == KDS_FORMAT_BLOCK) {
-            lp = lp_next;
-            lp_next = lp_after;
-            /* (the fast decode of a known layout reads the tuple with two
-             * wide loads; there the L1 prefetch only costs issue slots) */
-            if (!(lay_ok && XBJ_LAY_FIXED)
-#ifdef XBJ_STAGE
-                && !staged
-#endif
-                )
-                xbj_prefetch_tuple(page, lp_next);
-            lp_after = xbj_itemid(page, nitems, idx + 64);
-        }
-        item += 32;
-        bool failed = false;
-        if (idx < nitems) {
-            XbjRegs R;
-            bool exists = false;
-            const bool ok = xbj_decode(R, args, page, kds, row0, meta, idx, lp, lay_ok, exists, args.st, acol);
-            if (exists)
-                C.raw++;
-            if (exists && !ok)
-                failed = true;
-            else if (ok)
-                xbj_pipeline(R, E, C, failed);
-        }
         uint32_t big = C.out | C.in | C.raw;
 #pragma unroll
         for (int d = 1; d <= XBJ_NRELS; d++)
             big |= C.depth[d];
         if (big & 0x80000000u)
             xbj_flush_cnt(C, args.st);
-        if (__any_sync(XB_FULL, failed))
+        if (__any_sync(XB_FULL, failed)) {
+            stop = false;
             break;
+        }
         /* (at most XB_UNCOUNTED groups of a warp stay uncounted between
          * batches, which the growth's dump region allows for) */
         if (lane == 0 && *(volatile uint32_t *)E.newg > XB_UNCOUNTED)
             xbj_count_flush(args.gt, E.newg);
-        if (args.left_out && __shfl_sync(XB_FULL, xbj_grow_seen(src.grow_buf, lane), 0)) {
-            /* the table is to grow: leave the rest for the resume launch */
-            xb_src_leave(args, src, lane, item, nitems);
-            break;
-        }
     }
+    if (stop)
+        xb_src_leave(args, src, lane, item, nitems);
 
 #ifdef XBJ_STAGE
     /* the barrier's memory becomes group-table or buffer space again */
@@ -550,21 +622,9 @@ xbj_mixed_kernel(const __grid_constant__ XbMixArgs m)
  * XBJ_RT_TAIL is defined), where every generated definition is known ---- */
 
 #ifdef XBJ_PART
-/* replay of the deferred rows.  A bucket holds the rows whose groups have
- * their home slot in one slice of the global table (1 << part_shift
- * slots).  Each CTA claims buckets in order, so the CTAs work on
- * neighbouring slices together and the slices stay in L2; the bucket's
- * records and its slice are pulled into L2 by the TMA engine when it is
- * claimed.  Every row updates its group in the global table (the same
- * update as in place).  A row whose group the table and its dump have no
- * room for (the table asked to grow meanwhile) is marked and replayed
- * after the growth (retry). */
-extern "C" __global__ void __launch_bounds__(XB_BLOCK, XBJ_MIN_BLOCKS)
-xbj_replay(const __grid_constant__ XbReplayArgs args)
+/* the environment of a replay */
+__device__ __forceinline__ void xbj_replay_env(XbjEnv &E, const XbReplayArgs &args, uint32_t *newg)
 {
-    __shared__ uint32_t cur;            /* the CTA's bucket */
-    __shared__ uint32_t newg;           /* groups created in it */
-    XbjEnv E;
     E.plan = args.plan;
     E.st = args.st;
     E.gt = args.gt;
@@ -581,9 +641,144 @@ xbj_replay(const __grid_constant__ XbReplayArgs args)
     E.part_cap = 0;
     E.part_shift = 0;
     E.replay = 1;
-    E.newg = &newg;
+    E.newg = newg;
+}
+
+/* leave a record for after the table grows */
+__device__ __forceinline__ void xbj_rec_leave(char *rec, xb_status *st)
+{
+    ((uint32_t *)rec)[1] |= XBJ_REC_LEFT;
+    if (!st->replay_left)
+        atomicExch(&st->replay_left, 1u);
+}
+
+/*
+ * Replay of the deferred rows, a bucket's slice of the table at a time in
+ * shared memory: a CTA loads the slice (when the table had no groups before
+ * the replay, it starts empty instead), looks up and updates the groups of
+ * the bucket's records there, and writes the entries in use back.  The
+ * table moves through the SMs once, in whole lines, and a row costs no
+ * requests to L2 but those for its record; as reductions on the table in L2
+ * a row was about 15 requests, which bound the replay (500M rows into 10M
+ * groups: 6.5 ms, 3.4 ms on slices).
+ * A slice of up to XB_SLICE_BYTES leaves room for two CTAs per SM, one
+ * loading or storing while the other updates.
+ * A row whose probe runs past the end of the slice, where another CTA may be
+ * at work, is put on the spill list, replayed on the whole table by the
+ * launch after this one (xbj_replay); when the list is full the record is
+ * left as one that found the table full is.
+ */
+extern "C" __global__ void __launch_bounds__(XB_SLICE_BLOCK, 2)
+xbj_replay_slice(const __grid_constant__ XbReplayArgs args)
+{
+    extern __shared__ __align__(16) char slice[];
+    __shared__ uint32_t cur;
+    __shared__ uint32_t newg;
+    XbjEnv E;
+    xbj_replay_env(E, args, &newg);
+    const uint32_t nslots = 1u << args.part_shift;
+    const uint32_t chunks = nslots * (XBJ_GENT_SIZE / 16);
+    const bool fresh = *args.nused0 == 0;
     if (threadIdx.x == 0)
         newg = 0;
+    for (;;) {
+        if (threadIdx.x == 0) {
+            xbj_count_flush(args.gt, &newg);
+            cur = atomicAdd(args.cursor, 1u);
+        }
+        __syncthreads();
+        const uint32_t b = cur;
+        if (b >= args.nparts)
+            break;
+        const uint32_t cnt = args.part_cnt[(size_t)b * XB_PART_CNT_STRIDE];
+        const uint32_t n = cnt < args.part_cap ? cnt : args.part_cap;
+        char *base = args.part_buf + (uint64_t)b * args.part_cap * XBJ_REC_SIZE;
+        char *home = E.gt_entries + ((uint64_t)b << args.part_shift) * XBJ_GENT_SIZE;
+        if (n) {
+            if (threadIdx.x == 0 && (((uintptr_t)base) & 15) == 0) {
+                const uint64_t rb = (uint64_t)n * XBJ_REC_SIZE;
+                if (rb >= 16)
+                    xb_prefetch_l2(base, (uint32_t)(rb < (1u << 20) ? rb : (1u << 20)) & ~15u);
+            }
+            if (fresh) {
+                for (uint32_t i = threadIdx.x; i < chunks; i += XB_SLICE_BLOCK)
+                    ((uint4 *)slice)[i] = make_uint4(0u, 0u, 0u, 0u);
+            } else {
+                const uint32_t s0 = (uint32_t)__cvta_generic_to_shared(slice);
+                for (uint32_t i = threadIdx.x; i < chunks; i += XB_SLICE_BLOCK)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;"
+                                 :: "r"(s0 + 16 * i), "l"(home + 16ULL * i) : "memory");
+                asm volatile("cp.async.wait_all;" ::: "memory");
+            }
+        }
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < n; i += XB_SLICE_BLOCK) {
+            char *rec = base + (uint64_t)i * XBJ_REC_SIZE;
+            XbjRegs R;
+            uint32_t ghash;
+            xbj_rec_load(rec, R, ghash);
+            bool failed = false;
+            char *e = xbj_slice_get(R, E, slice, (uint32_t)(ghash & E.gt_mask) & (nslots - 1), nslots, ghash, failed);
+            if (e) {
+                xbj_update_slice(e, R, E);
+            } else if (!failed) {
+                const uint32_t p = atomicAdd(args.nspill, 1u);
+                if (p < args.spill_cap)
+                    args.spill[p] = make_uint2(b, i);
+                else
+                    xbj_rec_leave(rec, args.st);
+            }
+        }
+        __syncthreads();
+        if (n) {
+            for (uint32_t i = threadIdx.x; i < chunks; i += XB_SLICE_BLOCK) {
+                const char *e = slice + (size_t)(i / (XBJ_GENT_SIZE / 16)) * XBJ_GENT_SIZE;
+                if (((const xb_gent_head *)e)->state != XB_GSTATE_EMPTY)
+                    ((uint4 *)home)[i] = ((const uint4 *)slice)[i];
+            }
+            __syncthreads();        /* the slice is read before the next one's load */
+        }
+    }
+}
+
+/* replay of the deferred rows on the table in L2: records of slices too
+ * large for shared memory, the spill list of xbj_replay_slice, and records
+ * left for after the table grew.  A bucket holds the rows whose groups have
+ * their home slot in one slice of the global table (1 << part_shift
+ * slots).  Each CTA claims buckets in order, so the CTAs work on
+ * neighbouring slices together and the slices stay in L2; the bucket's
+ * records and its slice are pulled into L2 by the TMA engine when it is
+ * claimed.  Every row updates its group in the global table (the same
+ * update as in place).  A row whose group the table and its dump have no
+ * room for (the table asked to grow meanwhile) is marked and replayed
+ * after the growth (retry). */
+extern "C" __global__ void __launch_bounds__(XB_BLOCK, XBJ_MIN_BLOCKS)
+xbj_replay(const __grid_constant__ XbReplayArgs args)
+{
+    __shared__ uint32_t cur;            /* the CTA's bucket */
+    __shared__ uint32_t newg;           /* groups created in it */
+    XbjEnv E;
+    xbj_replay_env(E, args, &newg);
+    if (threadIdx.x == 0)
+        newg = 0;
+    if (args.spilled) {
+        __syncthreads();
+        const uint32_t n = *args.nspill < args.spill_cap ? *args.nspill : args.spill_cap;
+        for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+            const uint2 at = args.spill[i];
+            char *rec = args.part_buf + ((uint64_t)at.x * args.part_cap + at.y) * XBJ_REC_SIZE;
+            XbjRegs R;
+            uint32_t ghash;
+            xbj_rec_load(rec, R, ghash);
+            bool failed = false;
+            if (xbj_group_row(R, E, ghash, failed))
+                xbj_rec_leave(rec, args.st);
+        }
+        __syncthreads();
+        if (threadIdx.x == 0)
+            xbj_count_flush(args.gt, &newg);
+        return;
+    }
     for (;;) {
         if (threadIdx.x == 0) {
             xbj_count_flush(args.gt, &newg);    /* the last bucket's */
@@ -620,9 +815,7 @@ xbj_replay(const __grid_constant__ XbReplayArgs args)
             bool failed = false;
             const bool table_full = xbj_group_row(R, E, ghash, failed);
             if (table_full) {
-                ((uint32_t *)rec)[1] |= XBJ_REC_LEFT;
-                if (!args.st->replay_left)
-                    atomicExch(&args.st->replay_left, 1u);
+                xbj_rec_leave(rec, args.st);
             } else if (args.retry) {
                 ((uint32_t *)rec)[1] &= ~XBJ_REC_LEFT;
             }
