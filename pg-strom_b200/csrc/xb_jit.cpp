@@ -1942,7 +1942,7 @@ struct Gen {
      * it, and an aggregate without keys has too little to do per row. */
     bool compact() const
     {
-        return false;
+        return format == KDS_FORMAT_ARROW && p->scan_quals.count && p->has_groupby == 1;
     }
 
     void pipeline()

@@ -238,6 +238,14 @@ __device__ __forceinline__ void xbj_grow_fetch(uint32_t *buf, const xb_gtable *g
                  :: "r"((uint32_t)__cvta_generic_to_shared(buf)), "l"((const char *)gt + 48) : "memory");
 }
 
+/* new groups of a warp from which on it counts them: half of the rows it
+ * applies together */
+#ifdef XBJ_COMPACT
+#define XBJ_UNCOUNTED   15
+#else
+#define XBJ_UNCOUNTED   XB_UNCOUNTED
+#endif
+
 /* the group table's growth request: lane 0 fetches it into shared memory by
  * an asynchronous copy before rows are applied and looks at it after them,
  * so no register is held and little latency is waited for; the rest of the
@@ -525,7 +533,7 @@ xbj_body(const XbExecArgs &args, char *smem)
         }
         /* (at most XB_UNCOUNTED groups of a warp stay uncounted between
          * batches, which the growth's dump region allows for) */
-        if (lane == 0 && *(volatile uint32_t *)E.newg > XB_UNCOUNTED)
+        if (lane == 0 && *(volatile uint32_t *)E.newg > XBJ_UNCOUNTED)
             xbj_count_flush(args.gt, E.newg);
     }
     if (stop)
