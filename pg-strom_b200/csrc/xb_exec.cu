@@ -2634,6 +2634,9 @@ static_assert(XBJ_WARPS_PER_CTA == XB_WARPS, "specialised kernels assume the exe
  * aligned) for its 'grow' word, the second word there */
 static_assert(offsetof(xb_gtable, grow) == 52 && offsetof(xb_gtable, overflow) == 48,
               "the group table's grow word moved");
+/* xb_proj_head composes a tuple's header by words */
+static_assert(offsetof(kern_tupitem, t_infomask2) == 10 && offsetof(kern_tupitem, t_infomask) == 12 &&
+              offsetof(kern_tupitem, t_hoff) == 14 && offsetof(kern_tupitem, t_bits) == 15, "kern_tupitem");
 static_assert(offsetof(XbSrc, grow_buf) % 16 == 0, "XbSrc.grow_buf must be 16-byte aligned");
 
 int xb_set_error(kern_errorbuf *err, uint32_t code, const char *func, int line,

@@ -1168,8 +1168,32 @@ __device__ __forceinline__ uint32_t xb_proj_hoff(uint32_t nattrs, bool hasnull)
     return (uint32_t)PGSTROM_MAXALIGN(offsetof(kern_tupitem, t_bits) + (hasnull ? (nattrs + 7) / 8 : 0));
 }
 
+/* copy n bytes to a 4-byte aligned place: read as aligned words, written 4
+ * bytes at a time */
+__device__ __forceinline__ void xb_copy_words(char *dst, const uint8_t *src, uint32_t n)
+{
+    if (n == 0)
+        return;
+    XbWords r;
+    xb_words_start(&r, src, n);
+    uint32_t i = 0;
+    uint64_t w = 0;
+    for (; i + 4 <= n; i += 4) {
+        w = i & 4 ? w >> 32 : xb_words_next(&r);
+        *(uint32_t *)(dst + i) = (uint32_t)w;
+    }
+    if (i < n) {
+        w = i & 4 ? w >> 32 : xb_words_next(&r);
+        for (; i < n; i++, w >>= 8)
+            dst[i] = (char)w;
+    }
+}
+
 /* place attribute (ld, attalign) of value v / aux at offset t of the tuple
- * at base (measure only when base is nullptr); returns the offset after it */
+ * at base, 8-byte aligned (measure only when base is nullptr); returns the
+ * offset after it.  Fixed-width attributes are stored whole where attalign
+ * is their width (bytes one at a time were 56 stores of a 64-byte row:
+ * 2.9M tuples of 4M rows: 1.63 -> 1.50 ms) */
 __device__ __forceinline__ uint32_t
 xb_proj_attr(char *base, uint32_t t, int attalign, int ld, uint64_t v, uint32_t aux, uint16_t &infomask)
 {
@@ -1182,18 +1206,45 @@ xb_proj_attr(char *base, uint32_t t, int attalign, int ld, uint64_t v, uint32_t 
     }
     uint32_t nbytes = 0;
     switch (ld) {
-    case XB_LD_BOOL: { const uint8_t x = v ? 1 : 0; nbytes = 1; if (buf) xb_store(buf, &x, 1); break; }
-    case XB_LD_INT2: { const int16_t x = (int16_t)v; nbytes = 2; if (buf) xb_store(buf, &x, 2); break; }
+    case XB_LD_BOOL: nbytes = 1; if (buf) *buf = v ? 1 : 0; break;
+    case XB_LD_INT2: {
+        const int16_t x = (int16_t)v;
+        nbytes = 2;
+        if (buf) {
+            if (attalign >= 2) *(int16_t *)buf = x;
+            else xb_store(buf, &x, 2);
+        }
+        break;
+    }
     case XB_LD_INT4:
-    case XB_LD_DATE: { const int32_t x = (int32_t)v; nbytes = 4; if (buf) xb_store(buf, &x, 4); break; }
+    case XB_LD_DATE: {
+        const int32_t x = (int32_t)v;
+        nbytes = 4;
+        if (buf) {
+            if (attalign >= 4) *(int32_t *)buf = x;
+            else xb_store(buf, &x, 4);
+        }
+        break;
+    }
     case XB_LD_INT8:
-    case XB_LD_FLT8: { nbytes = 8; if (buf) xb_store(buf, &v, 8); break; }
+    case XB_LD_FLT8:
+        nbytes = 8;
+        if (buf) {
+            if (attalign >= 8) *(uint64_t *)buf = v;
+            else xb_store(buf, &v, 8);
+        }
+        break;
     case XB_LD_TEXT: {
         nbytes = 4 + aux;
         if (buf) {
             const uint32_t hdr = nbytes << 2;               /* SET_VARSIZE */
-            xb_store(buf, &hdr, 4);
-            xb_store(buf + 4, (const void *)v, aux);
+            if (attalign >= 4) {
+                *(uint32_t *)buf = hdr;
+                xb_copy_words(buf + 4, (const uint8_t *)v, aux);
+            } else {
+                xb_store(buf, &hdr, 4);
+                xb_store(buf + 4, (const void *)v, aux);
+            }
         }
         infomask |= HEAP_HASVARWIDTH;
         break;
@@ -1201,7 +1252,10 @@ xb_proj_attr(char *base, uint32_t t, int attalign, int ld, uint64_t v, uint32_t 
     case XB_LD_NUMERIC: {
         const uint8_t *vl = (const uint8_t *)v;
         nbytes = xb_numeric_varsize(vl);
-        if (buf) xb_store(buf, vl, nbytes);
+        if (buf) {
+            if (attalign >= 4) xb_copy_words(buf, vl, nbytes);
+            else xb_store(buf, vl, nbytes);
+        }
         infomask |= HEAP_HASVARWIDTH;
         break;
     }
@@ -1211,30 +1265,30 @@ xb_proj_attr(char *base, uint32_t t, int attalign, int ld, uint64_t v, uint32_t 
     return t_next + nbytes;
 }
 
-/* zero the header and set t_infomask2 / t_hoff / the NULL bitmap */
+/* the header of a tuple at base, 8-byte aligned: its words, the NULL bitmap
+ * from byte 15 on (nulls: bit j set when attribute j is NULL) */
 __device__ __forceinline__ void
-xb_proj_head(char *base, uint32_t nattrs, uint32_t hoff, uint32_t nulls)
+xb_proj_head(char *base, uint32_t nattrs, uint32_t hoff, uint32_t nulls, uint32_t t_len, uint32_t hash, uint16_t infomask)
 {
-    for (uint32_t i = 0; i < hoff; i++)
-        base[i] = 0;
-    const uint16_t im2 = (uint16_t)(nattrs & HEAP_NATTS_MASK);
-    const uint8_t th = (uint8_t)(hoff + MINIMAL_TUPLE_OFFSET);
-    xb_store(base + offsetof(kern_tupitem, t_infomask2), &im2, 2);
-    xb_store(base + offsetof(kern_tupitem, t_hoff), &th, 1);
-    if (nulls) {
-        for (uint32_t j = 0; j < nattrs; j++)
-            if (!((nulls >> j) & 1u))
-                base[offsetof(kern_tupitem, t_bits) + (j >> 3)] |= (char)(1 << (j & 7));
-    }
+    uint64_t bits = 0;
+    if (nulls)
+        bits = ~(uint64_t)nulls & ((1ULL << nattrs) - 1);
+    ((uint64_t *)base)[0] = ((uint64_t)hash << 32) | t_len;
+    ((uint64_t *)base)[1] = ((uint64_t)(nattrs & HEAP_NATTS_MASK) << 16) | ((uint64_t)infomask << 32) |
+                            ((uint64_t)((hoff + MINIMAL_TUPLE_OFFSET) & 0xff) << 48) | (bits << 56);
+    bits >>= 8;
+    for (uint32_t w = 2; w < hoff / 8; w++, bits = 0)
+        ((uint64_t *)base)[w] = bits;
 }
 
-/* t_len, t_infomask and the trailing row id */
+/* the trailing row id */
 __device__ __forceinline__ void
-xb_proj_tail(char *base, uint32_t t_len, uint16_t infomask, uint32_t rowid)
+xb_proj_tail(char *base, uint32_t t_len, uint32_t rowid)
 {
-    xb_store(base + offsetof(kern_tupitem, t_infomask), &infomask, 2);
-    xb_store(base, &t_len, 4);
-    xb_store(base + t_len - ROWID_SIZE, &rowid, 4);
+    if ((t_len & 3) == 0)
+        *(uint32_t *)(base + t_len - ROWID_SIZE) = rowid;
+    else
+        xb_store(base + t_len - ROWID_SIZE, &rowid, 4);
 }
 
 /* kds_dst bytes one row of tuple length t_len takes (the reference's
@@ -1340,14 +1394,12 @@ xb_proj_emit(const xb_plan *plan, char *dst, uint64_t dst_len,
     if (!ip)
         return;
     char *tp = ip + item;
-    xb_proj_head(tp, n, hoff, nulls);
-    if (item)
-        xb_store(tp + offsetof(kern_tupitem, hash), &hash, 4);
+    xb_proj_head(tp, n, hoff, nulls, t_len, item ? hash : 0, im);
     t = hoff;
     for (uint32_t j = 0; j < n; j++)
         if (!((nulls >> j) & 1u))
             t = xb_proj_attr(tp, t, plan->proj[j].attalign, plan->proj[j].ld, vals[j], auxs[j], im);
-    xb_proj_tail(tp, t_len, im, rowid);
+    xb_proj_tail(tp, t_len, rowid);
     if (item) {
         uint64_t *slots = (uint64_t *)(dst + head) - plan->proj_nslots;
         const unsigned long long next =

@@ -1506,11 +1506,10 @@ struct Gen {
           << i2 << "char *tp = xb_proj_claim(E.dst, E.dst_len, " << p->proj_head_len << "ULL, xb_proj_rowsz(tl, "
           << p->proj_margin << "u), E.st, &rowid);\n"
           << i2 << "if (tp) {\n"
-          << i2 << "    xb_proj_head(tp, " << n << "u, hoff, pn);\n"
-          << i2 << "    t = hoff;\n"
-          << i2 << "    im = pn ? HEAP_HASNULL : 0;\n";
+          << i2 << "    xb_proj_head(tp, " << n << "u, hoff, pn, tl, 0, im);\n"
+          << i2 << "    t = hoff;\n";
         attrs("tp");
-        o << i2 << "    xb_proj_tail(tp, tl, im, rowid);\n"
+        o << i2 << "    xb_proj_tail(tp, tl, rowid);\n"
           << i2 << "    xb_proj_index(E.dst, E.dst_len, " << p->proj_head_len << "ULL, rowid, tp);\n"
           << i2 << "}\n"
           << ind << "}\n";
