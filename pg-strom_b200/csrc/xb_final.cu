@@ -229,11 +229,29 @@ struct XbFinalRun {
         ta.tile_slots = (uint32_t)slots;
         ta.ntiles = (uint32_t)((ta.cap + slots - 1) / slots);
         const uint64_t n = pset * ta.ntiles;
-        if (!alloc(n * 4, (void **)&ta.count) || !alloc(n * 8, (void **)&ta.bytes) ||
-            !alloc(n * 4, (void **)&ta.count_scan) || !alloc(n * 8, (void **)&ta.bytes_scan) ||
-            !alloc(16ULL * nparts, (void **)&d_totals) || !alloc(xb_scan_temp_bytes<uint64_t>(n), &d_temp))
+        /* the work arrays in one piece */
+        const uint64_t tb = 16ULL * nparts;
+        char *w = nullptr;
+        if (!alloc(24 * n + tb + xb_scan_temp_bytes<uint64_t>(n) + 256, (void **)&w))
             return XB_ERR(err, ERRCODE_DEVICE_FATAL, "out of device memory in Final");
+        ta.bytes = (uint64_t *)w;
+        ta.bytes_scan = ta.bytes + n;
+        d_totals = ta.bytes + 2 * n;
+        ta.count = (uint32_t *)(w + 16 * n + tb);
+        ta.count_scan = ta.count + n;
+        d_temp = (void *)(((uintptr_t)(ta.count + 2 * n) + 255) & ~(uintptr_t)255);
         totals.assign(2 * (size_t)nparts, 0);
+        if (nparts == 1 && ta.cap <= XB_FINAL_SMALL) {
+            ta.pset = 1;
+            xb_final_count_small<<<1, 1024, 0, st>>>(ta, s->pinned->totals);
+            cudaError_t rc = cudaGetLastError();
+            if (rc != cudaSuccess || (rc = cudaStreamSynchronize(st)) != cudaSuccess)
+                return XB_ERR(err, ERRCODE_DEVICE_FATAL, "Final: %s", cudaGetErrorString(rc));
+            totals[0] = s->pinned->totals[0];
+            totals[1] = s->pinned->totals[1];
+            set0 = 0;
+            return 0;
+        }
         for (uint32_t p = 0; p < nparts; p += XB_FINAL_PARTS)
             if (!count(p))
                 return XB_ERR(err, ERRCODE_DEVICE_FATAL, "Final: %s", cudaGetErrorString(cudaGetLastError()));
@@ -257,22 +275,33 @@ struct XbFinalRun {
         cudaStream_t st = s->stream;
         const kern_session_info *session = (const kern_session_info *)s->h_session.data();
         XbFinalPart *d_parts = nullptr;
-        uint64_t *d_head = nullptr;
-        if (!alloc(sizeof(XbFinalPart) * parts.size(), (void **)&d_parts) || !alloc(head_len, (void **)&d_head))
-            return XB_ERR(err, ERRCODE_DEVICE_FATAL, "out of device memory in Final");
-        XB_CUDA(cudaMemcpyAsync(d_parts, parts.data(), sizeof(XbFinalPart) * parts.size(), cudaMemcpyHostToDevice, st), err);
-        XB_CUDA(cudaMemcpyAsync(d_head, s->d_session + session->groupby_kds_final, head_len,
-                                cudaMemcpyDeviceToDevice, st), err);
+        const char *head = s->d_session + session->groupby_kds_final;
+        if (((uintptr_t)head & 7) != 0) {
+            char *copy = nullptr;
+            if (!alloc(head_len, (void **)&copy))
+                return XB_ERR(err, ERRCODE_DEVICE_FATAL, "out of device memory in Final");
+            XB_CUDA(cudaMemcpyAsync(copy, head, head_len, cudaMemcpyDeviceToDevice, st), err);
+            head = copy;
+        }
+        if (ta.nparts > 1) {
+            if (!alloc(sizeof(XbFinalPart) * parts.size(), (void **)&d_parts))
+                return XB_ERR(err, ERRCODE_DEVICE_FATAL, "out of device memory in Final");
+            XB_CUDA(cudaMemcpyAsync(d_parts, parts.data(), sizeof(XbFinalPart) * parts.size(),
+                                    cudaMemcpyHostToDevice, st), err);
+        }
+        ta.head = (const uint64_t *)head;
+        ta.head_len = (uint32_t)head_len;
+        ta.only = parts[0];
         ta.out = out;
         for (uint32_t p0 = 0; p0 < ta.nparts; p0 += XB_FINAL_PARTS) {
             if (set0 != p0 && !count(p0))
                 return XB_ERR(err, ERRCODE_DEVICE_FATAL, "Final: %s", cudaGetErrorString(cudaGetLastError()));
-            ta.part = d_parts + p0;
+            ta.part = d_parts ? d_parts + p0 : nullptr;
             uint64_t most = 0;
             for (uint32_t p = p0; p < p0 + ta.pset; p++)
                 most = std::max<uint64_t>(most, parts[p].nslots);
             const unsigned gx = (unsigned)std::min<uint64_t>((head_len / 8 + most + 255) / 256, 1024);
-            xb_final_heads<<<dim3(gx, ta.pset), 256, 0, st>>>(out, ta.part, d_head, (uint32_t)head_len, ta.row_format);
+            xb_final_heads<<<dim3(gx, ta.pset), 256, 0, st>>>(ta);
             xb_final_fill<<<grid(), XB_FINAL_TILE, ta.nparts > 1 ? 16 * ta.pset : 0, st>>>(ta);
         }
         cudaError_t rc = cudaGetLastError();

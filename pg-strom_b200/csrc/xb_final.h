@@ -52,6 +52,7 @@ struct XbFinalPart {
 /* kds_final by tiles of the group table: the groups and item bytes of
  * every (part, tile), then the tuples (xb_final_tiles, xb_final_fill) */
 #define XB_FINAL_TILE   256
+#define XB_FINAL_SMALL  16384       /* slots of a table that one CTA counts */
 #define XB_FINAL_PARTS  1024        /* parts of one launch (their counters are in shared memory) */
 struct XbTileArgs {
     const xb_plan  *plan;
@@ -68,7 +69,10 @@ struct XbTileArgs {
     const uint32_t *count_scan;     /* exclusive prefixes of the two, over all parts */
     const uint64_t *bytes_scan;
     char           *out;
-    const XbFinalPart *part;
+    const XbFinalPart *part;        /* nullptr: the one part 'only' */
+    XbFinalPart     only;
+    const uint64_t *head;           /* the session's kds_final definition */
+    uint32_t        head_len;
     const uint32_t *list;           /* the entries to write, in order (cap of them), or
                                      * nullptr: every group, in table order */
     XbFinalProg     prog;
@@ -148,9 +152,9 @@ struct XbRebuildArgs {
 __global__ void __launch_bounds__(XB_FINAL_TILE) xb_final_tiles(const __grid_constant__ XbTileArgs a);
 __global__ void __launch_bounds__(XB_FINAL_TILE) xb_final_scan_small(XbTileArgs a, uint32_t *count_scan,
                                                                       uint64_t *bytes_scan, uint32_t n);
+__global__ void __launch_bounds__(1024) xb_final_count_small(const __grid_constant__ XbTileArgs a, uint64_t *totals);
 __global__ void xb_final_totals(XbTileArgs a, uint64_t *totals);
-__global__ void xb_final_heads(char *out, const XbFinalPart *part, const uint64_t *head, uint32_t head_len,
-                               uint32_t row_format);
+__global__ void xb_final_heads(const __grid_constant__ XbTileArgs a);
 __global__ void __launch_bounds__(XB_FINAL_TILE) xb_final_fill(const __grid_constant__ XbTileArgs a);
 __global__ void __launch_bounds__(XB_FINAL_TILE) xb_final_ents(const __grid_constant__ XbTileArgs a, uint32_t *ents);
 __global__ void xb_top_hist(XbTopArgs a, uint32_t digit);

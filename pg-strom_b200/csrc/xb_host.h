@@ -30,6 +30,7 @@
 struct xb_pinned {
     xb_status       st;
     xb_gtable       gt;
+    uint64_t        totals[2];      /* of a small kds_final: groups, item bytes */
 };
 
 /* pinned memory (mapped on the GPU) that one fetch of chunk headers uses:
