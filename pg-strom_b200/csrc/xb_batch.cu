@@ -148,6 +148,7 @@ static void xb_reset_groups(xpuB200Session *s)
         s->h_gt.grow = 0;
         s->h_gt.dump_used = 0;
         s->h_gt.soft_cap = (s->h_gt.cap_mask + 1) / 2;
+        cudaMemsetAsync(s->d_gt, 0, XB_GT_BYTES, st);
         cudaMemcpyAsync(s->d_gt, &s->h_gt, sizeof(xb_gtable), cudaMemcpyHostToDevice, st);
     }
     cudaMemsetAsync(s->d_status, 0, sizeof(xb_status), st);

@@ -2698,10 +2698,7 @@ const char *xb_msg_text(uint32_t id)
 }
 
 static_assert(XBJ_WARPS_PER_CTA == XB_WARPS, "specialised kernels assume the executor's CTA size");
-/* the specialised kernels fetch bytes 48..63 of the group table (16-byte
- * aligned) for its 'grow' word, the second word there */
-static_assert(offsetof(xb_gtable, grow) == 52 && offsetof(xb_gtable, overflow) == 48,
-              "the group table's grow word moved");
+static_assert(sizeof(xb_gtable) <= XB_GROW_OFF, "the copies of the growth request follow the header");
 /* xb_proj_head composes a tuple's header by words */
 static_assert(offsetof(kern_tupitem, t_infomask2) == 10 && offsetof(kern_tupitem, t_infomask) == 12 &&
               offsetof(kern_tupitem, t_hoff) == 14 && offsetof(kern_tupitem, t_bits) == 15, "kern_tupitem");
@@ -3024,7 +3021,8 @@ xpuB200OpenSession(xpuB200Device *dev, const kern_session_info *session, uint64_
         DALLOC(cap * plan->gent_size, &s->h_gt.entries);
         DALLOC(arena, &s->h_gt.arena);
         cudaMemsetAsync(s->h_gt.entries, 0, cap * plan->gent_size, st);
-        DALLOC(sizeof(xb_gtable), &s->d_gt);
+        DALLOC(XB_GT_BYTES, &s->d_gt);
+        cudaMemsetAsync(s->d_gt, 0, XB_GT_BYTES, st);
         cudaMemcpyAsync(s->d_gt, &s->h_gt, sizeof(xb_gtable), cudaMemcpyHostToDevice, st);
         s->sm_cap = xb_sm_cap_for(est, plan->gent_size);
     }
@@ -3730,6 +3728,7 @@ int xb_gt_grow(xpuB200Session *s, uint64_t min_entries, kern_errorbuf *err)
     ng.grow = 0;
     ng.soft_cap = new_cap / 2;
     ng.dump_used = 0;
+    XB_CUDA(cudaMemsetAsync(s->d_gt, 0, XB_GT_BYTES, st), err);
     XB_CUDA(cudaMemcpyAsync(s->d_gt, &ng, sizeof(xb_gtable), cudaMemcpyHostToDevice, st), err);
     XB_CUDA(cudaMemsetAsync(s->d_status, 0, sizeof(xb_status), st), err);
     XbGrowArgs ga;

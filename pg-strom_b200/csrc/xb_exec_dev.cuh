@@ -134,17 +134,20 @@ __device__ __forceinline__ uint32_t xb_ld_relaxed(const uint32_t *p)
  * ================================================================ */
 __device__ __forceinline__ void xb_gt_want_grow(xb_gtable *gt)
 {
-    if (*(volatile uint32_t *)&gt->grow == 0)
-        atomicExch(&gt->grow, 1u);
+    if (*(volatile uint32_t *)&gt->grow == 0 && atomicExch(&gt->grow, 1u) == 0) {
+        for (uint32_t i = 0; i < XB_GROW_COPIES; i++)
+            *(volatile uint32_t *)((char *)gt + XB_GROW_OFF + i * XB_GROW_STRIDE) = 1;
+    }
 }
 
 /* new global entries a warp of a specialised kernel may leave uncounted
  * between 32-row batches */
 #define XB_UNCOUNTED    31
 /* rows a warp may still apply after the table asked to grow: the 32 it is
- * applying, 32 more if its look at the request came just before, and the
- * rows that wait in its queue (31) */
-#define XB_INFLIGHT     95
+ * applying, 32 more if its look at the request came just before (and 32 if
+ * its copy of the request was still to be written), and the rows that wait
+ * in its queue (31) */
+#define XB_INFLIGHT     127
 
 /* count new entries of the global table; once soft_cap entries are in use
  * the table asks to grow */
@@ -704,8 +707,8 @@ struct alignas(16) XbSrc {
     uint32_t item;                  /* next item of the unit */
     uint32_t nitems;                /* items of the unit */
     uint32_t newg;                  /* specialised kernels: new global groups not yet counted */
-    uint32_t grow_buf[4];           /* specialised kernels, lane 0: bytes 48..63 of the
-                                     * group table (its 'grow' word), fetched asynchronously */
+    uint32_t grow_buf[4];           /* specialised kernels, lane 0: the CTA's copy of the group
+                                     * table's growth request, fetched asynchronously */
 };
 
 /* chunk owning global unit 'unit' (tasks are sorted by unit_base) */

@@ -229,13 +229,14 @@ __device__ __forceinline__ bool xbj_stage_wait(uint64_t *mbar, uint32_t parity)
 }
 #endif
 
-/* 16 bytes of the group table holding its 'grow' word, copied into shared
- * memory through L2 (cp.async.cg: no L1 copy that could be stale) */
+/* the CTA's copy of the group table's growth request into shared memory,
+ * through L2 (cp.async.cg: no L1 copy that could be stale) */
 __device__ __forceinline__ void xbj_grow_fetch(uint32_t *buf, const xb_gtable *gt)
 {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n\t"
                  "cp.async.commit_group;"
-                 :: "r"((uint32_t)__cvta_generic_to_shared(buf)), "l"((const char *)gt + 48) : "memory");
+                 :: "r"((uint32_t)__cvta_generic_to_shared(buf)), "l"((const char *)gt + XB_GROW_OFF +
+                    (blockIdx.x % XB_GROW_COPIES) * XB_GROW_STRIDE) : "memory");
 }
 
 /* new groups of a warp from which on it counts them: half of the rows it
@@ -261,7 +262,7 @@ __device__ __forceinline__ uint32_t xbj_grow_seen(const uint32_t *buf, uint32_t 
     if (lane != 0)
         return 0;
     asm volatile("cp.async.wait_all;" ::: "memory");
-    return *(volatile const uint32_t *)&buf[1];
+    return *(volatile const uint32_t *)&buf[0];
 }
 
 /* add *newg new groups to the table's count (one thread; nobody is
@@ -433,9 +434,7 @@ xbj_body(const XbExecArgs &args, char *smem)
 #else
                 break;
 #endif
-#ifndef XBJ_COMPACT
             XBJ_GROW_FETCH();
-#endif
             const uint32_t idx = item + lane;
             uint32_t lp = 0;
 #ifdef XBJ_ACOLS
@@ -498,16 +497,13 @@ xbj_body(const XbExecArgs &args, char *smem)
             qn += __popc(passed);
             __syncwarp();
 #endif
-#ifndef XBJ_COMPACT
             if (XBJ_GROW_SEEN())
                 stop = true;
-#endif
         }
 #ifdef XBJ_COMPACT
         else {
             if (qn == 0)
                 break;
-            XBJ_GROW_FETCH();
             const uint32_t n = qn < 32 ? qn : 32;
             qn -= n;
             if (lane < n) {
@@ -517,8 +513,6 @@ xbj_body(const XbExecArgs &args, char *smem)
                 xbj_after_quals(R, E, C, failed);
             }
             __syncwarp();
-            if (XBJ_GROW_SEEN())
-                stop = true;
         }
 #endif
         uint32_t big = C.out | C.in | C.raw;
