@@ -3548,7 +3548,7 @@ static int xb_launch_tasks(xpuB200Session *s, const xb_task *d_tasks, uint32_t n
  * enough for the slices the replay's CTAs work on together to stay in L2.
  * Rows past a full bucket are updated in place, so any bucket size is
  * correct.  Used by
- * prepared batches whose table is several times L2 (the records of a batch
+ * prepared batches whose table is beyond L2 (the records of a batch
  * take device memory in proportion to its rows, which the serving path's
  * admission does not budget); XPU_B200_PARTITION=1 uses it for every
  * launch on the session's stream over a table above 64 MB, =0 never;
@@ -3573,7 +3573,17 @@ static bool xb_part_prepare(xpuB200Session *s, uint64_t nunits, uint32_t format,
     const uint32_t rec = xb_jit_part_rec_size(plan, format);
     const uint64_t cap = s->h_gt.cap_mask + 1;
     const uint64_t table = cap * plan->gent_size;
-    if (rec == 0 || table <= (force ? (64ULL << 20) : (512ULL << 20)))
+    if (rec == 0)
+        return false;
+    /* The replay passes over the whole table, in place a row costs requests
+     * to a table beyond L2.  Arrow rows into 448 MB of table: 1M rows 154 us
+     * in place and 228 deferred, 2M 245 and 260, 4M 335 and 284, 20M 941 and
+     * 614; into 224 MB: 1M 159 and 187, 4M 286 and 234; into 112 MB: 4M 225
+     * and 220, 20M 570 and 521; heap rows into 448 MB: 1M 324 and 399, 5M 885
+     * and 739.  So from 192 MB on, with half as many rows as slots (about
+     * 100 rows a heap page); above 512 MB always */
+    const uint64_t rows_about = nunits * (format == KDS_FORMAT_BLOCK ? 100ULL : (uint64_t)XB_ROWS_UNIT);
+    if (table <= (force ? 64ULL << 20 : rows_about * 2 >= cap ? 192ULL << 20 : 512ULL << 20))
         return false;
     /* one bucket per slice of the table that a replay CTA's shared table
      * covers: at the table's load its groups fit in shared memory */
