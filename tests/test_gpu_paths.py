@@ -226,3 +226,40 @@ def test_limit(device, ngroups, limit, keys):
     if keys[-1][0] == "VREF" and keys[-1][1] == 11:             # a total order: the very groups
         assert list(got) == [x[0] for _, x in want]
     assert F.compare_groups(got, {k: expect[k] for k in got}) == []
+
+
+# ---- replay on slices of the table: probes that leave a slice (256 slots of
+# 288 bytes, half full), chunks replayed on an empty and on a filled table
+@pytest.mark.parametrize("est,groups", [(64_000, 40), (64_000, 20_000), (64_000, 120_000)])
+def test_replay_slices(device, monkeypatch, est, groups):
+    monkeypatch.setenv("XPU_B200_PARTITION", "1")
+    tbl, _, _, expect, _ = C.wide_groupby(nrows=200_000, seed_config=66, ngroups=groups)
+    sess = C.wide_groupby_session(ngroups=est)
+    chunks = tbl.block_chunks(pages_per_chunk=700)
+    assert len(chunks) >= 3
+    s = xpu_b200.Session(device, sess)
+    try:
+        for ch in chunks:
+            s.exec(ch)
+        assert s.info()["partition_used"], s.info()
+        got = F.decode_kds_final(s.final()[0], sess)
+    finally:
+        s.close()
+    assert F.compare_groups(got, expect) == []
+
+
+# ---- kds_final counted by one CTA (16384 slots at most) or by tiles
+@pytest.mark.parametrize("est,slots", [(1, 2048), (3_840, 16_384), (3_841, 32_768)])
+@pytest.mark.parametrize("groups", [1, 33, 3_000])
+def test_final_of_small_tables(device, est, slots, groups):
+    tbl, _, _, expect, _ = C.scan_groupby(nrows=12_000, seed_config=67, a_limit=700, ngroups=groups)
+    sess = C.scan_groupby_session(700, est)
+    s = xpu_b200.Session(device, sess)
+    try:
+        assert s.info()["gtable_cap"] == slots
+        for ch in tbl.block_chunks(pages_per_chunk=300):
+            s.exec(ch)
+        got = F.decode_kds_final(s.final()[0], sess)
+    finally:
+        s.close()
+    assert F.compare_groups(got, _truth(expect)) == []
