@@ -229,6 +229,41 @@ __device__ __forceinline__ void xb_atomic_add_f64c_g(double *hi, double *lo, dou
         xb_red_g_add_f64(lo, e);
 }
 
+/* the two in halves, for updates that add several sums before they look at
+ * an old value: the addition, and what follows from the value it found */
+__device__ __forceinline__ uint64_t xb_atom_g_add_u64(void *p, uint64_t v)
+{
+    uint64_t old;
+    asm volatile("atom.relaxed.gpu.global.add.u64 %0, [%1], %2;"
+                 : "=l"(old) : "l"(__cvta_generic_to_global(p)), "l"(v) : "memory");
+    return old;
+}
+
+__device__ __forceinline__ double xb_atom_g_add_f64(void *p, double v)
+{
+    double old;
+    asm volatile("atom.relaxed.gpu.global.add.f64 %0, [%1], %2;"
+                 : "=d"(old) : "l"(__cvta_generic_to_global(p)), "d"(v) : "memory");
+    return old;
+}
+
+__device__ __forceinline__ void xb_i128_carry_g(void *hi_word, uint64_t old, xb_i128 v)
+{
+    const uint64_t lo = (uint64_t)v;
+    const uint64_t hi = (uint64_t)((unsigned __int128)v >> 64) + (old + lo < old ? 1 : 0);
+    if (hi)
+        xb_red_g_add_u64(hi_word, hi);
+}
+
+__device__ __forceinline__ void xb_f64c_err_g(void *lo, double old, double x)
+{
+    const double s = __dadd_rn(old, x);
+    const double bp = __dsub_rn(s, old);
+    const double e = __dadd_rn(__dsub_rn(old, __dsub_rn(s, bp)), __dsub_rn(x, bp));
+    if (e != 0.0)
+        xb_red_g_add_f64(lo, e);
+}
+
 __device__ __forceinline__ double xb_reg_f64(uint64_t v, int rk)
 {
     return rk == XB_RK_FLT ? __longlong_as_double(v) : (double)(int64_t)v;

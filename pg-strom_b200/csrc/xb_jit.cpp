@@ -761,7 +761,10 @@ struct Gen {
         /* state updates of the global table's entries: the lanes are spread
          * over many entries (combining them per entry would run once per
          * distinct entry with the other lanes idle), so each lane updates
-         * its entry directly */
+         * its entry directly.  The sums whose old value is needed are all
+         * added before the first of these values is looked at: a lane waits
+         * for the table once, not once a sum (2M rows, every statistic, 3000\n         * groups: 972 -> 958 us a query) */
+        std::ostringstream late;
         o << "__device__ __forceinline__ void xbj_update(char *e, const XbjRegs &R, const XbjEnv &E)\n{\n"
              "    (void)E;\n" << numeric_args();
         for (uint32_t i = 0; i < p->naggs; i++) {
@@ -770,13 +773,71 @@ struct Gen {
                 continue;
             const AggExpr x = agg_expr(a);
             const std::string S = "(e + " + std::to_string(a.state_off) + ")";
+            if (returning_update(a, i, S, x.c, x.xd, x.yd, late))
+                continue;
             o << "    { /* aggregate " << i << ": action " << a.action << " */\n";
-            if (!direct_update(a, S, x.f, x.c, x.xd))
-                helper_update(a, S, x.c, x.xd, x.yd);
+            direct_update(a, S, x.f, x.c, x.xd);
             o << "    }\n";
         }
-        o << "}\n\n";
+        o << late.str() << "}\n\n";
         shared_form();
+    }
+
+    /* per-lane update of an action whose sums need the value that the
+     * addition found (the rounding error of a float sum, the carry of a
+     * 128-bit one): the additions to o, what follows from the old values to
+     * late; false for other actions */
+    bool returning_update(const xb_agg &a, uint32_t i, const std::string &S, std::string c, const std::string &xd,
+                          const std::string &yd, std::ostringstream &late)
+    {
+        const std::string I = std::to_string(i);
+        std::vector<std::string> sums;      /* float sums, 16 bytes apart from byte 8 */
+        switch (a.action) {
+        case KAGG_ACTION__PSUM_FP: case KAGG_ACTION__PAVG_FP:
+            sums = {xd};
+            break;
+        case KAGG_ACTION__STDDEV:
+            sums = {xd, xd + " * " + xd};
+            break;
+        case KAGG_ACTION__COVAR:
+            sums = {xd, xd + " * " + xd, yd, yd + " * " + yd, xd + " * " + yd};
+            c += " && !" + N(a.arg1);
+            break;
+        case KAGG_ACTION__PSUM_INT64: case KAGG_ACTION__PAVG_INT64:
+        case KAGG_ACTION__PSUM_NUMERIC: case KAGG_ACTION__PAVG_NUMERIC: {
+            const bool num = is_numeric_sum(a);
+            const std::string v = num ? "x" + num_id(a) : "(xb_i128)(int64_t)" + V(a.arg0);
+            const std::string put = num ? "k" + num_id(a) + " == XB_NUM_VALID" : "true";
+            o << "    uint64_t o" << I << " = 0; /* aggregate " << i << ": action " << a.action << " */\n"
+              << "    if (" << c << ") {\n"
+              << "        if (" << put << ") {\n"
+              << "            xb_red_g_add_u64(" << S << ", 1ULL);\n"
+              << "            o" << I << " = xb_atom_g_add_u64(" << S << " + 8, (uint64_t)(" << v << "));\n"
+              << "        }";
+            if (num)
+                o << " else {\n            xb_red_g_or_u32(" << S << " + 24, xb_numeric_special(k" << num_id(a) << "));\n"
+                     "        }";
+            o << "\n    }\n";
+            late << "    if (" << c << " && " << put << ") xb_i128_carry_g(" << S << " + 16, o" << I << ", " << v << ");\n";
+            return true;
+        }
+        default:
+            return false;
+        }
+        o << "    double";
+        for (size_t k = 0; k < sums.size(); k++)
+            o << (k ? ", o" : " o") << I << "_" << k << " = 0.0";
+        o << "; /* aggregate " << i << ": action " << a.action << " */\n"
+          << "    if (" << c << ") {\n"
+          << "        xb_red_g_add_u64(" << S << ", 1ULL);\n";
+        late << "    if (" << c << ") {\n";
+        for (size_t k = 0; k < sums.size(); k++) {
+            o << "        o" << I << "_" << k << " = xb_atom_g_add_f64(" << S << " + " << 8 + 16 * k << ", " << sums[k] << ");\n";
+            late << "        xb_f64c_err_g(" << S << " + " << 16 + 16 * k << ", o" << I << "_" << k << ", " << sums[k] << ");\n";
+        }
+        o << "    }\n";
+        late << "    }\n";
+        return true;
     }
 
     /* an update's numeric arguments, each decoded once per scale however
@@ -1233,18 +1294,6 @@ struct Gen {
             o << "        if (" << c << ") {\n"
                  "            xb_red_g_add_u64(" << S << ", 1ULL);\n"
                  "            xb_red_g_add_u64(" << S << " + 8, (unsigned long long)" << V(a.arg0) << ");\n"
-                 "        }\n";
-            return true;
-        case KAGG_ACTION__PSUM_INT64: case KAGG_ACTION__PAVG_INT64:
-            o << "        if (" << c << ") {\n"
-                 "            xb_red_g_add_u64(" << S << ", 1ULL);\n"
-                 "            xb_atomic_add_i128_g((uint64_t *)(" << S << " + 8), (xb_i128)(int64_t)" << V(a.arg0) << ");\n"
-                 "        }\n";
-            return true;
-        case KAGG_ACTION__PSUM_FP: case KAGG_ACTION__PAVG_FP:
-            o << "        if (" << c << ") {\n"
-                 "            xb_red_g_add_u64(" << S << ", 1ULL);\n"
-                 "            xb_atomic_add_f64c_g((double *)(" << S << " + 8), (double *)(" << S << " + 16), " << xd << ");\n"
                  "        }\n";
             return true;
         default:
