@@ -229,6 +229,13 @@ __device__ __forceinline__ void xb_atomic_add_f64c_g(double *hi, double *lo, dou
         xb_red_g_add_f64(lo, e);
 }
 
+__device__ __forceinline__ uint64_t xb_ld_relaxed_u64(const void *p)
+{
+    uint64_t v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(__cvta_generic_to_global(p)) : "memory");
+    return v;
+}
+
 /* the two in halves, for updates that add several sums before they look at
  * an old value: the addition, and what follows from the value it found */
 __device__ __forceinline__ uint64_t xb_atom_g_add_u64(void *p, uint64_t v)
@@ -297,18 +304,6 @@ xb_agg_numeric_add(char *s, const uint8_t *vl, int16_t weight, xb_status *st)
         XB_RAISE(st, ERRCODE_DEVICE_ERROR, XB_MSG_NUMERIC_CORRUPT);
     else
         xb_agg_numeric_put(s, kind, v);
-}
-
-/* xb_agg_numeric_put for an entry of the global table (global reductions) */
-__device__ __forceinline__ void
-xb_agg_numeric_put_g(char *s, uint8_t kind, xb_i128 v)
-{
-    if (kind == XB_NUM_VALID) {
-        xb_red_g_add_u64(s, 1ULL);
-        xb_atomic_add_i128_g((uint64_t *)(s + 8), v);
-    } else {
-        xb_red_g_or_u32(s + 24, xb_numeric_special(kind));
-    }
 }
 
 /* xb_agg_numeric_put for an entry of a shared-memory group table (shared

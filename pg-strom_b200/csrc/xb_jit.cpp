@@ -763,7 +763,7 @@ struct Gen {
          * distinct entry with the other lanes idle), so each lane updates
          * its entry directly.  The sums whose old value is needed are all
          * added before the first of these values is looked at: a lane waits
-         * for the table once, not once a sum (2M rows, every statistic, 3000\n         * groups: 972 -> 958 us a query) */
+         * for the table once, not once a sum (2M rows, every statistic, 3000\n         * groups: 972 -> 958 us a query, 933 with the minima and maxima below) */
         std::ostringstream late;
         o << "__device__ __forceinline__ void xbj_update(char *e, const XbjRegs &R, const XbjEnv &E)\n{\n"
              "    (void)E;\n" << numeric_args();
@@ -776,7 +776,7 @@ struct Gen {
             if (returning_update(a, i, S, x.c, x.xd, x.yd, late))
                 continue;
             o << "    { /* aggregate " << i << ": action " << a.action << " */\n";
-            direct_update(a, S, x.f, x.c, x.xd);
+            direct_update(a, S, x.f, x.c);
             o << "    }\n";
         }
         o << late.str() << "}\n\n";
@@ -793,6 +793,25 @@ struct Gen {
         const std::string I = std::to_string(i);
         std::vector<std::string> sums;      /* float sums, 16 bytes apart from byte 8 */
         switch (a.action) {
+        case KAGG_ACTION__PMIN_INT32: case KAGG_ACTION__PMIN_INT64: case KAGG_ACTION__PMIN_FP64:
+        case KAGG_ACTION__PMAX_INT32: case KAGG_ACTION__PMAX_INT64: case KAGG_ACTION__PMAX_FP64: {
+            /* a relaxed read of the value, and a reduction only where the
+             * row changes it (a value read too early only costs one).  The
+             * flag belongs to the first row: as long as the value is what a
+             * group starts with */
+            const bool is_min = a.action == KAGG_ACTION__PMIN_INT32 || a.action == KAGG_ACTION__PMIN_INT64 ||
+                                a.action == KAGG_ACTION__PMIN_FP64;
+            const bool fp = a.action == KAGG_ACTION__PMIN_FP64 || a.action == KAGG_ACTION__PMAX_FP64;
+            const std::string val = fp ? "(long long)xb_f64_ordered(" + xd + ")" : "(long long)" + V(a.arg0);
+            o << "    long long o" << I << " = 0; /* aggregate " << i << ": action " << a.action << " */\n"
+              << "    if (" << c << ") o" << I << " = (long long)xb_ld_relaxed_u64(" << S << ");\n";
+            late << "    if (" << c << ") {\n"
+                    "        if (o" << I << " == " << (is_min ? "INT64_MAX" : "INT64_MIN") << ") xb_red_g_or_u32(" << S << " + 8, 1u);\n"
+                    "        if (" << val << (is_min ? " < o" : " > o") << I << ") "
+                 << (is_min ? "xb_red_g_min_s64" : "xb_red_g_max_s64") << "(" << S << ", " << val << ");\n"
+                    "    }\n";
+            return true;
+        }
         case KAGG_ACTION__PSUM_FP: case KAGG_ACTION__PAVG_FP:
             sums = {xd};
             break;
@@ -1242,16 +1261,12 @@ struct Gen {
         o << "}\n\n";
     }
 
-    /* per-lane update of the actions kept in helpers (numeric, stddev,
-     * covariance): the standard form */
+    /* per-lane update of the actions kept in helpers (stddev, covariance):
+     * the standard form */
     void helper_update(const xb_agg &a, const std::string &S, const std::string &c, const std::string &xd,
                        const std::string &yd)
     {
         switch (a.action) {
-        case KAGG_ACTION__PSUM_NUMERIC: case KAGG_ACTION__PAVG_NUMERIC:
-            o << "        if (" << c << ") xb_agg_numeric_put_g(" << S << ", k" << num_id(a) << ", x" << num_id(a)
-              << ");\n";
-            break;
         case KAGG_ACTION__STDDEV:
             o << "        if (" << c << ") xb_agg_stddev_add(" << S << ", " << xd << ");\n";
             break;
@@ -1264,40 +1279,26 @@ struct Gen {
         }
     }
 
-    /* per-lane update of one combinable action into an entry of the
-     * global table (keyed groups: e is global memory, so every update
-     * whose old value is not needed is a fire-and-forget reduction);
-     * false if not combinable */
-    bool direct_update(const xb_agg &a, const std::string &S, const std::string &f,
-                       const std::string &c, const std::string &xd)
+    /* per-lane update of a count or an integer sum of an entry of the global
+     * table (keyed groups: e is global memory, the updates are
+     * fire-and-forget reductions) */
+    void direct_update(const xb_agg &a, const std::string &S, const std::string &f, const std::string &c)
     {
         switch (a.action) {
         case KAGG_ACTION__NROWS_ANY:
             o << "        if (" << f << ") xb_red_g_add_u64(" << S << ", 1ULL);\n";
-            return true;
+            break;
         case KAGG_ACTION__NROWS_COND:
             o << "        if (" << c << ") xb_red_g_add_u64(" << S << ", 1ULL);\n";
-            return true;
-        case KAGG_ACTION__PMIN_INT32: case KAGG_ACTION__PMIN_INT64: case KAGG_ACTION__PMIN_FP64:
-        case KAGG_ACTION__PMAX_INT32: case KAGG_ACTION__PMAX_INT64: case KAGG_ACTION__PMAX_FP64: {
-            const bool is_min = a.action == KAGG_ACTION__PMIN_INT32 || a.action == KAGG_ACTION__PMIN_INT64 ||
-                                a.action == KAGG_ACTION__PMIN_FP64;
-            const bool fp = a.action == KAGG_ACTION__PMIN_FP64 || a.action == KAGG_ACTION__PMAX_FP64;
-            const std::string val = fp ? "(long long)xb_f64_ordered(" + xd + ")" : "(long long)" + V(a.arg0);
-            o << "        if (" << c << ") {\n"
-                 "            xb_red_g_or_u32(" << S << " + 8, 1u);\n"
-                 "            " << (is_min ? "xb_red_g_min_s64" : "xb_red_g_max_s64") << "(" << S << ", " << val << ");\n"
-                 "        }\n";
-            return true;
-        }
+            break;
         case KAGG_ACTION__PSUM_INT: case KAGG_ACTION__PAVG_INT:
             o << "        if (" << c << ") {\n"
                  "            xb_red_g_add_u64(" << S << ", 1ULL);\n"
                  "            xb_red_g_add_u64(" << S << " + 8, (unsigned long long)" << V(a.arg0) << ");\n"
                  "        }\n";
-            return true;
+            break;
         default:
-            return false;
+            break;
         }
     }
 
