@@ -4321,10 +4321,10 @@ xpuB200ExecTaskDst(xpuB200Session *s, const kern_data_store *kds_src, int kds_sr
     if (rc) return rc;
     const xb_status *hs = s->h_status;
     const uint64_t nitems = hs->proj_nitems, usage = hs->proj_usage;
-    const uint64_t required = head_len + hs->proj_need;
+    const uint64_t required = head_len + 8 * nitems + usage;
     if (p_required)
         *p_required = required;
-    if (hs->proj_overflow)
+    if (required > len)
         return XB_ERR(err, ERRCODE_SUSPEND_NO_SPACE, "kds_dst needs %llu bytes (buffer %llu)",
                       (unsigned long long)required, (unsigned long long)len);
     /* the header: the session's kds_dst definition with this chunk's rows

@@ -436,15 +436,13 @@ typedef struct xb_status {
      * claim lands here, away from the error word every warp polls */
     uint64_t    unit_cursor;
     uint64_t    __pad2[15];
-    /* projection output: proj_need counts the row index and tuple bytes
-     * of every claim, including those past the end of kds_dst (so that
-     * the host learns the size needed); proj_usage / proj_nitems place
-     * only the claims that fit */
-    uint64_t    proj_need;
+    /* projection output: tuple bytes and rows of every claim, including
+     * those past the end of kds_dst (so that the host learns the size
+     * needed), each alone in its line: every emitting warp adds to both */
     uint64_t    proj_usage;
-    uint32_t    proj_nitems;
-    uint32_t    proj_overflow;
-    uint64_t    __pad3[13];
+    uint64_t    __pad3[15];
+    uint64_t    proj_nitems;
+    uint64_t    __pad4[15];
 } xb_status;
 
 /* error message ids reported by device code */
