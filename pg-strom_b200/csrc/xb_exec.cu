@@ -2718,6 +2718,9 @@ const char *xb_msg_text(uint32_t id)
 }
 
 static_assert(XBJ_WARPS_PER_CTA == XB_WARPS, "specialised kernels assume the executor's CTA size");
+/* the specialised kernels fetch bytes 48..63 of the header for its 'grow' word */
+static_assert(offsetof(xb_gtable, grow) == 52 && offsetof(xb_gtable, overflow) == 48,
+              "the group table's grow word moved");
 static_assert(sizeof(xb_gtable) <= XB_GROW_OFF, "the copies of the growth request follow the header");
 /* xb_proj_head composes a tuple's header by words */
 static_assert(offsetof(kern_tupitem, t_infomask2) == 10 && offsetof(kern_tupitem, t_infomask) == 12 &&
@@ -3656,10 +3659,12 @@ static bool xb_part_prepare(xpuB200Session *s, uint64_t nunits, uint32_t format,
  * when the table's free half is smaller than twice those.  The entries are
  * cleared as they are taken (xb_dump_slot): clearing the region was 45 MB a
  * query */
-static int xb_dump_ensure(xpuB200Session *s, int grid, uint32_t sm_cap, cudaStream_t st, kern_errorbuf *err)
+static int xb_dump_ensure(xpuB200Session *s, uint32_t format, int grid, uint32_t sm_cap, cudaStream_t st,
+                          kern_errorbuf *err)
 {
     const uint64_t cap = s->h_gt.cap_mask + 1;
-    const uint64_t inflight = (uint64_t)grid * XB_WARPS * (XB_INFLIGHT + XB_UNCOUNTED);
+    const uint64_t inflight = (uint64_t)grid * XB_WARPS *
+        ((format == KDS_FORMAT_ARROW ? XB_INFLIGHT_ARROW : XB_INFLIGHT) + XB_UNCOUNTED);
     uint64_t need = (uint64_t)grid * sm_cap;
     if (cap / 2 < 2 * inflight)
         need += inflight;
@@ -3875,7 +3880,7 @@ int xb_launch_on(xpuB200Session *s, const xb_task *d_tasks, uint32_t ntasks,
             const uint64_t warps = (uint64_t)grid * XB_WARPS;
             s->run_static_base0 = format == KDS_FORMAT_BLOCK ? ((nunits * 3 / 5) / warps) * warps : 0;
         }
-        if (xb_dump_ensure(s, grid, s->sm_cap, stream, err) != 0)
+        if (xb_dump_ensure(s, format, grid, s->sm_cap, stream, err) != 0)
             return err ? err->errcode : ERRCODE_DEVICE_FATAL;
     }
     if (format < 256)

@@ -144,10 +144,11 @@ __device__ __forceinline__ void xb_gt_want_grow(xb_gtable *gt)
  * between 32-row batches */
 #define XB_UNCOUNTED    31
 /* rows a warp may still apply after the table asked to grow: the 32 it is
- * applying, 32 more if its look at the request came just before (and 32 if
- * its copy of the request was still to be written), and the rows that wait
- * in its queue (31) */
-#define XB_INFLIGHT     127
+ * applying and 32 more if its look at the request came just before; where
+ * Arrow rows are compacted also 32 if its copy of the request was still to
+ * be written, and the rows that wait in its queue (31) */
+#define XB_INFLIGHT         64
+#define XB_INFLIGHT_ARROW   127
 
 /* count new entries of the global table; once soft_cap entries are in use
  * the table asks to grow */

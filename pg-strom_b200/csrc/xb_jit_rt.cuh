@@ -229,14 +229,22 @@ __device__ __forceinline__ bool xbj_stage_wait(uint64_t *mbar, uint32_t parity)
 }
 #endif
 
-/* the CTA's copy of the group table's growth request into shared memory,
- * through L2 (cp.async.cg: no L1 copy that could be stale) */
+/* the group table's growth request into shared memory, through L2
+ * (cp.async.cg: no L1 copy that could be stale): the CTA's copy of it where
+ * rows are compacted, else the 16 bytes of the header that hold it (with a
+ * row's decode between two looks they do not wait for one another) */
+#ifdef XBJ_COMPACT
+#define XBJ_GROW_AT     (XB_GROW_OFF + (blockIdx.x % XB_GROW_COPIES) * XB_GROW_STRIDE)
+#define XBJ_GROW_WORD   0
+#else
+#define XBJ_GROW_AT     48
+#define XBJ_GROW_WORD   1
+#endif
 __device__ __forceinline__ void xbj_grow_fetch(uint32_t *buf, const xb_gtable *gt)
 {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n\t"
                  "cp.async.commit_group;"
-                 :: "r"((uint32_t)__cvta_generic_to_shared(buf)), "l"((const char *)gt + XB_GROW_OFF +
-                    (blockIdx.x % XB_GROW_COPIES) * XB_GROW_STRIDE) : "memory");
+                 :: "r"((uint32_t)__cvta_generic_to_shared(buf)), "l"((const char *)gt + XBJ_GROW_AT) : "memory");
 }
 
 /* new groups of a warp from which on it counts them: half of the rows it
@@ -262,7 +270,7 @@ __device__ __forceinline__ uint32_t xbj_grow_seen(const uint32_t *buf, uint32_t 
     if (lane != 0)
         return 0;
     asm volatile("cp.async.wait_all;" ::: "memory");
-    return *(volatile const uint32_t *)&buf[0];
+    return *(volatile const uint32_t *)&buf[XBJ_GROW_WORD];
 }
 
 /* add *newg new groups to the table's count (one thread; nobody is
@@ -527,7 +535,7 @@ xbj_body(const XbExecArgs &args, char *smem)
         }
         /* (at most XB_UNCOUNTED groups of a warp stay uncounted between
          * batches, which the growth's dump region allows for) */
-        if (lane == 0 && *(volatile uint32_t *)E.newg > XBJ_UNCOUNTED)
+        if (args.left_out && lane == 0 && *(volatile uint32_t *)E.newg > XBJ_UNCOUNTED)
             xbj_count_flush(args.gt, E.newg);
     }
     if (stop)
