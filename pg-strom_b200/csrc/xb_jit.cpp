@@ -2485,7 +2485,13 @@ xb_jit_prepare(void *func, int block, size_t smem, int *p_per_sm)
     std::lock_guard<std::mutex> guard(g_lock);
     if (!g_drv.ok)
         return -1;
-    if (g_drv.setattr((CUfunction)func, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, (int)smem) != CUDA_SUCCESS)
+    /* the limit is the function's, which sessions of one plan shape share
+     * with shared tables of their own sizes: it is only ever raised */
+    int cur = 0;
+    if (g_drv.getattr(&cur, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, (CUfunction)func) != CUDA_SUCCESS)
+        cur = 0;
+    if ((size_t)cur < smem &&
+        g_drv.setattr((CUfunction)func, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, (int)smem) != CUDA_SUCCESS)
         return -1;
     int per_sm = 0;
     if (g_drv.occupancy(&per_sm, (CUfunction)func, block, smem) != CUDA_SUCCESS || per_sm < 1)

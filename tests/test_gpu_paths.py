@@ -263,3 +263,22 @@ def test_final_of_small_tables(device, est, slots, groups):
     finally:
         s.close()
     assert F.compare_groups(got, _truth(expect)) == []
+
+
+# ---- sessions of one plan shape share a kernel: a session with a small shared
+# table opened after one with a large table must not take its shared memory
+def test_shared_kernel_of_two_table_sizes(device):
+    tbl, _, _, expect, _ = C.scan_groupby(nrows=20_000, seed_config=68, a_limit=600, ngroups=200)
+    chunks = tbl.block_chunks(pages_per_chunk=100)
+    large, small = C.scan_groupby_session(600, 200), C.scan_groupby_session(600, 1)
+    a, b = xpu_b200.Session(device, large), xpu_b200.Session(device, small)
+    try:
+        for ch in chunks:
+            a.exec(ch)
+            b.exec(ch)
+        assert a.info()["smem_bytes"] > b.info()["smem_bytes"]
+        for s, sess in ((a, large), (b, small)):
+            assert F.compare_groups(F.decode_kds_final(s.final()[0], sess), _truth(expect)) == []
+    finally:
+        a.close()
+        b.close()
