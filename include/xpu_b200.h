@@ -189,7 +189,10 @@ void xpuB200CloseSession(xpuB200Session *sess);
  * returns its statistics in *results, or its error; a ticket is reported
  * done once.  Groups accumulate in the session as with xpuB200ExecTask;
  * xpuB200Final and xpuB200CloseSession first wait for the session's
- * submitted commands.  xpuB200ServeConfig sets the admission budget in
+ * submitted commands, and so do the calls that may move or rewrite its
+ * group table (ExecTask and BatchExec of a session whose table can grow,
+ * MergeFinal, FinalParts); commands submitted during such a call start when
+ * it is done.  xpuB200ServeConfig sets the admission budget in
  * bytes and alone_units (0 keeps a value).  The default budget,
  * XPU_B200_ADMIT_FREE_HBM, admits by the device's free memory: a launch is
  * admitted while the staging bytes of its commands fit the GPU's free HBM

@@ -106,6 +106,7 @@ xpuB200BatchExec(xpuB200Batch *b, kern_exec_results *results, kern_errorbuf *err
     if (!b)
         return XB_ERR(err, ERRCODE_DEVICE_ERROR, "invalid batch");
     xpuB200Session *s = b->sess;
+    xb_table_hold hold(s, xb_table_moves(s));
     std::lock_guard<std::mutex> g(s->lock);
     XB_CUDA(cudaSetDevice(s->dev->dindex), err);
     s->in_batch = true;
@@ -119,6 +120,7 @@ xpuB200BatchTime(xpuB200Batch *b, int niters, double *p_msec, kern_errorbuf *err
 {
     xb_clear_error(err);
     xpuB200Session *s = b->sess;
+    xb_table_hold hold(s, xb_table_moves(s));
     std::lock_guard<std::mutex> g(s->lock);
     XB_CUDA(cudaSetDevice(s->dev->dindex), err);
     float total = 0.0f;
@@ -165,7 +167,7 @@ xpuB200BatchTune(xpuB200Batch *b, uint32_t flags, char *report, size_t report_le
     if (!b || flags != 0)
         return XB_ERR(err, ERRCODE_DEVICE_ERROR, "invalid BatchTune arguments");
     xpuB200Session *s = b->sess;
-    xb_sched_drain_session(s);
+    xb_table_hold hold(s);
     std::lock_guard<std::mutex> g(s->lock);
     if (s->total_raw != 0)
         return XB_ERR(err, ERRCODE_DEVICE_ERROR, "tune a session before it executes chunks");

@@ -4121,6 +4121,15 @@ static bool xb_groups_may_grow(const xpuB200Session *s)
     return true;
 }
 
+/* can a run on the session's stream move or rewrite its group table (it
+ * grows, or rows are replayed on slices of it)?  Then launches that update
+ * the table in place stay away meanwhile (xb_table_hold) */
+bool xb_table_moves(xpuB200Session *s)
+{
+    std::lock_guard<std::mutex> g(s->lock);
+    return xb_groups_may_grow(s);
+}
+
 int xb_run(xpuB200Session *s, const xb_task *d_tasks, uint32_t ntasks, uint64_t nunits,
                   uint32_t format, kern_exec_results *results, kern_errorbuf *err, bool timed)
 {
@@ -4212,6 +4221,7 @@ xpuB200ExecTask(xpuB200Session *s, const kern_data_store *kds_src, int kds_src_o
     xb_clear_error(err);
     if (!s || !kds_src)
         return XB_ERR(err, ERRCODE_DEVICE_ERROR, "invalid ExecTask arguments");
+    xb_table_hold hold(s, xb_table_moves(s));
     std::lock_guard<std::mutex> g(s->lock);
     if (s->h_plan->has_proj)
         return XB_ERR(err, ERRCODE_DEVICE_ERROR,
@@ -4363,6 +4373,7 @@ xpuB200TimeExecTask(xpuB200Session *s, const kern_data_store *kds_src_dev, int n
                     double *p_msec, kern_errorbuf *err)
 {
     xb_clear_error(err);
+    xb_table_hold hold(s, xb_table_moves(s));
     std::lock_guard<std::mutex> g(s->lock);
     XB_CUDA(cudaSetDevice(s->dev->dindex), err);
     kern_data_store head;

@@ -487,7 +487,7 @@ xpuB200FinalNoAlloc(xpuB200Session *s, void *kds_final_dev, uint64_t buf_sz, uin
     xb_clear_error(err);
     if (!s)
         return XB_ERR(err, ERRCODE_DEVICE_ERROR, "invalid FinalNoAlloc arguments");
-    xb_sched_drain_session(s);
+    xb_table_hold hold(s);
     std::lock_guard<std::mutex> g(s->lock);
     const int dindex = s->dev->dindex;
     if (dindex < 0 || dindex >= XB_FINAL_SCRATCH_DEVS)
@@ -574,7 +574,7 @@ xpuB200Final(xpuB200Session *s, void *kds_final_buf, uint64_t buf_sz, uint64_t *
     xb_clear_error(err);
     if (!s)
         return XB_ERR(err, ERRCODE_DEVICE_ERROR, "invalid Final arguments");
-    xb_sched_drain_session(s);
+    xb_table_hold hold(s);
     std::lock_guard<std::mutex> g(s->lock);
     XB_CUDA(cudaSetDevice(s->dev->dindex), err);
     cudaStream_t st = s->stream;
@@ -643,7 +643,7 @@ xpuB200MergeFinal(xpuB200Session *s, const kern_data_store *kds_final, int kds_f
     xb_clear_error(err);
     if (!s || !kds_final)
         return XB_ERR(err, ERRCODE_DEVICE_ERROR, "invalid MergeFinal arguments");
-    xb_sched_drain_session(s);
+    xb_table_hold hold(s);
     std::lock_guard<std::mutex> g(s->lock);
     const xb_plan *plan = s->h_plan;
     if (!plan->has_groupby)
@@ -723,7 +723,7 @@ xpuB200FinalParts(xpuB200Session *s, uint32_t nparts, void *parts_dev, uint64_t 
     xb_clear_error(err);
     if (!s || nparts < 1 || nparts > 4096 || !part_offsets)
         return XB_ERR(err, ERRCODE_DEVICE_ERROR, "invalid FinalParts arguments");
-    xb_sched_drain_session(s);
+    xb_table_hold hold(s);
     std::lock_guard<std::mutex> g(s->lock);
     XB_CUDA(cudaSetDevice(s->dev->dindex), err);
     const xb_plan *plan = s->h_plan;

@@ -13,6 +13,7 @@
 #define XB_HOST_H
 
 #include <cuda_runtime.h>
+#include <atomic>
 #include <map>
 #include <mutex>
 #include <string>
@@ -48,7 +49,7 @@ struct xpuB200Device {
     uint64_t        hbm_budget;
     size_t          smem_optin;     /* dynamic shared memory a CTA may opt in to */
     cudaStream_t    stream;
-    struct xb_sched *sched = nullptr; /* asynchronous commands (created by the first submit) */
+    std::atomic<struct xb_sched *> sched{nullptr}; /* asynchronous commands (created by the first submit) */
     /* recycled per-session resources: creating a stream or pinning host
      * memory costs far more than a query's own host work */
     std::mutex      pool_lock;
@@ -137,6 +138,8 @@ struct xpuB200Session {
     void           *jit_job[256] = {nullptr};      /* a background build of it, pending */
     char            ran_kind[256] = {0};   /* 'j' / 'v': kernel last launched per format */
     uint32_t        sched_refs = 0;        /* submitted commands not yet finished */
+    std::atomic<bool> held{false};         /* its submitted commands wait (xb_table_hold) */
+    std::mutex      table_lock;            /* the holder's */
     /* device projection: staging buffer for host kds_dst, and the buffer of
      * the launch in progress */
     char           *d_dst = nullptr;
@@ -261,6 +264,20 @@ int xb_mix_launch(const xb_mix_group &g, const XbMixArgs &ma, cudaStream_t strea
 
 /* the scheduler's, which the core calls (xb_serve.cu) */
 void xb_sched_drain_session(xpuB200Session *s);
+
+/* keeps submitted commands off a session's group table while a call moves
+ * or rewrites it (growth, the replay on slices, a merge, kds_final): waits
+ * for those launched before and holds back those submitted meanwhile.
+ * Taken before the session's lock, which the scheduler takes under its own */
+class xb_table_hold {
+    xpuB200Session *s;
+public:
+    explicit xb_table_hold(xpuB200Session *sess, bool on = true);
+    ~xb_table_hold();
+    xb_table_hold(const xb_table_hold &) = delete;
+    xb_table_hold &operator=(const xb_table_hold &) = delete;
+};
+bool xb_table_moves(xpuB200Session *s);
 void xb_sched_destroy(xpuB200Device *dev);
 
 /* the interpreting kernel of mixed launches (xb_exec.cu) */

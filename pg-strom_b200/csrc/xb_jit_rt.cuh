@@ -677,6 +677,9 @@ __device__ __forceinline__ void xbj_rec_leave(char *rec, xb_status *st)
  * at work, is put on the spill list, replayed on the whole table by the
  * launch after this one (xbj_replay); when the list is full the record is
  * left as one that found the table full is.
+ * The entries are written back whole, by plain stores: no other launch may
+ * update the table meanwhile.  Those of the session's stream come before or
+ * after; served ones are held back (xb_table_hold).
  */
 extern "C" __global__ void __launch_bounds__(XB_SLICE_BLOCK, 2)
 xbj_replay_slice(const __grid_constant__ XbReplayArgs args)

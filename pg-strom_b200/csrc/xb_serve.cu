@@ -17,6 +17,8 @@
 #include <thread>
 #include <unordered_map>
 #include <vector>
+#include <chrono>
+#include <condition_variable>
 #include <cstdio>
 #include <cstring>
 #include "xb_host.h"
@@ -35,6 +37,9 @@
  * admitted as slots and memory free up, so their work overlaps on the
  * device.  A finished command's statistics are added to its session and
  * kept for xpuB200Poll; its groups are in the session's group table.
+ * Commands of a session whose table another call is about to move or rewrite
+ * (a batch or task that may grow it or replay rows on slices of it, Final,
+ * a merge) stay queued until that call is done; others pass them.
  */
 /* the device's free and total memory, and the reserve admission keeps */
 static void xb_mem_info(xpuB200Device *dev, uint64_t *p_free, uint64_t *p_total, uint64_t *p_reserve)
@@ -101,6 +106,7 @@ struct xb_sched {
     uint64_t        admit_bytes = 0;
     uint64_t        inflight_bytes = 0;
     uint32_t        alone_units = XB_ALONE_UNITS;
+    std::condition_variable released;   /* a session is no longer held */
     int             mix_grid_per_sm[2] = {0, 0};
 };
 
@@ -123,6 +129,9 @@ static void xb_slot_free(xb_slot &sl)
 
 static int xb_sched_init(xpuB200Device *dev, kern_errorbuf *err)
 {
+    if (dev->sched)
+        return 0;
+    std::lock_guard<std::mutex> g(dev->pool_lock);      /* (first submits of two threads) */
     if (dev->sched)
         return 0;
     xb_sched *q = new xb_sched();
@@ -217,6 +226,12 @@ static int xb_sched_launch(xpuB200Device *dev, xb_sched *q, xb_slot &sl, kern_er
 {
     std::vector<xb_cmd> take;
     uint64_t bytes = 0;
+    /* commands of held sessions wait, the others pass them */
+    size_t at = 0;
+    while (at < q->pending.size() && q->pending[at].s->held)
+        at++;
+    if (at == q->pending.size())
+        return 0;
     /* admission: by the device's free memory (the slot's staging buffer
      * is reusable), or against a fixed budget for the bytes in flight */
     uint64_t room;
@@ -227,11 +242,15 @@ static int xb_sched_launch(xpuB200Device *dev, xb_sched *q, xb_slot &sl, kern_er
     } else {
         room = q->admit_bytes > q->inflight_bytes ? q->admit_bytes - q->inflight_bytes : 0;
     }
-    const xb_cmd &f = q->pending.front();
+    const xb_cmd f = q->pending[at];
     const bool alone = f.units >= q->alone_units && f.s->jit_enabled;
     void *kern = alone ? nullptr : xb_mix_kernel_of(f.s, f.format, false);
-    while (!q->pending.empty() && take.size() < (alone ? 1u : (size_t)XB_SLOT_CMDS)) {
-        const xb_cmd &c = q->pending.front();
+    while (at < q->pending.size() && take.size() < (alone ? 1u : (size_t)XB_SLOT_CMDS)) {
+        const xb_cmd &c = q->pending[at];
+        if (c.s->held) {
+            at++;
+            continue;
+        }
         if (!alone && c.units >= q->alone_units && c.s->jit_enabled)
             break;                      /* a large one runs alone, in a later launch */
         if (!alone && xb_mix_kernel_of(c.s, c.format, false) != kern)
@@ -241,7 +260,7 @@ static int xb_sched_launch(xpuB200Device *dev, xb_sched *q, xb_slot &sl, kern_er
             break;                      /* admission: wait for memory to free up */
         bytes += b;
         take.push_back(c);
-        q->pending.pop_front();
+        q->pending.erase(q->pending.begin() + at);
     }
     if (take.empty())
         return 0;
@@ -380,8 +399,11 @@ static void xb_sched_wait_one(xb_sched *q, std::unique_lock<std::mutex> &lk, con
     for (int i = 0; i < XB_SLOTS && pick < 0; i++)
         if (q->slot[i].busy)
             pick = i;
-    if (pick < 0)
+    if (pick < 0) {
+        /* what is pending belongs to held sessions */
+        q->released.wait_for(lk, std::chrono::microseconds(200));
         return;
+    }
     cudaEvent_t ev = q->slot[pick].done;
     lk.unlock();
     cudaEventSynchronize(ev);
@@ -402,6 +424,45 @@ void xb_sched_drain_session(xpuB200Session *s)
             break;
         xb_sched_wait_one(q, lk, s);
     }
+}
+
+xb_table_hold::xb_table_hold(xpuB200Session *sess, bool on) : s(on ? sess : nullptr)
+{
+    if (!s)
+        return;
+    s->table_lock.lock();
+    xb_sched *q;
+    while (!(q = s->dev->sched)) {
+        s->held = true;
+        if (!s->dev->sched)
+            return;                 /* a scheduler that comes later finds it held */
+        s->held = false;
+    }
+    cudaSetDevice(s->dev->dindex);
+    std::unique_lock<std::mutex> lk(q->lock);
+    for (;;) {
+        xb_sched_progress(s->dev, q);
+        if (s->sched_refs == 0)
+            break;
+        xb_sched_wait_one(q, lk, s);
+    }
+    s->held = true;
+}
+
+xb_table_hold::~xb_table_hold()
+{
+    if (!s)
+        return;
+    s->held = false;
+    if (xb_sched *q = s->dev->sched) {
+        std::lock_guard<std::mutex> g(q->lock);
+        if (!q->pending.empty()) {
+            cudaSetDevice(s->dev->dindex);
+            xb_sched_progress(s->dev, q);
+            q->released.notify_all();
+        }
+    }
+    s->table_lock.unlock();
 }
 
 void xb_sched_destroy(xpuB200Device *dev)
@@ -444,11 +505,12 @@ xpuB200ServeConfig(xpuB200Device *dev, uint64_t admit_bytes, uint32_t alone_unit
     XB_CUDA(cudaSetDevice(dev->dindex), err);
     int rc = xb_sched_init(dev, err);
     if (rc) return rc;
-    std::lock_guard<std::mutex> g(dev->sched->lock);
+    xb_sched *q = dev->sched;
+    std::lock_guard<std::mutex> g(q->lock);
     if (admit_bytes)
-        dev->sched->admit_bytes = admit_bytes;
+        q->admit_bytes = admit_bytes;
     if (alone_units)
-        dev->sched->alone_units = alone_units;
+        q->alone_units = alone_units;
     return 0;
 }
 

@@ -149,3 +149,46 @@ def test_staged_pages_do_not_defer_text_keys(device, monkeypatch):
     want = F.decode_kds_final(o.final(), sess)
     o.close()
     assert F.compare_groups(F.decode_kds_final(final, sess), want) == []
+
+
+@pytest.mark.parametrize("threads", [False, True])
+def test_served_commands_beside_a_replay(device, monkeypatch, threads):
+    # chunks submitted to the session whose batch rewrites slices of the
+    # group table: in flight when the batch starts, or submitted by another
+    # thread while it runs; nothing that either adds may be lost
+    import threading
+    monkeypatch.delenv("XPU_B200_PARTITION", raising=False)
+    chunks, _, expect, meta = C.arrow_groupby(nrows=3_000_000, nkeys=1_000_000, rows_per_chunk=500_000,
+                                              seed_config=88)
+    sess = C.arrow_groupby_session(ngroups_estimate=10_000_000.0)
+    ups = [device.upload(c) for c in chunks]
+    try:
+        for rep in range(3):
+            s = xpu_b200.Session(device, sess)
+            batches = [s.batch([p for _, p in ups[:2]]), s.batch([p for _, p in ups[2:4]])]
+            tickets = []
+
+            def submit():
+                tickets.append(device.submit(s, chunks[4]))
+                tickets.append(device.submit(s, ups[5][1], on_device=True))
+            if threads:
+                t = threading.Thread(target=lambda: [b.exec() for b in batches])
+                t.start()
+                submit()
+                t.join()
+            else:
+                submit()
+                for b in batches:
+                    b.exec()
+            for k in tickets:
+                device.poll(k)
+            for b in batches:
+                b.close()
+            final, res = s.final()
+            info = s.info()
+            s.close()
+            assert info["partition_used"], info
+            assert F.compare_groups(F.decode_kds_final(final, sess), expect) == [], rep
+    finally:
+        for base, _ in ups:
+            device.free(base)
