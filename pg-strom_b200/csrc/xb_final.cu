@@ -311,6 +311,44 @@ struct XbFinalRun {
     }
 };
 
+/* what is wrong with a caller's output buffer at addr, memory of the given
+ * kind (and device, and device address) for a call on GPU dindex: it must be
+ * memory that this GPU's kernels can write, 8-byte aligned (kds_final is
+ * written in words).  own: no other GPU's memory either.  nullptr: nothing */
+static const char *xb_out_buffer_fault(const cudaPointerAttributes &pa, uint64_t addr, int dindex, bool own)
+{
+    if (pa.type == cudaMemoryTypeUnregistered)
+        return "is not CUDA memory";
+    if (own && !((pa.type == cudaMemoryTypeDevice && pa.device == dindex) || pa.type == cudaMemoryTypeManaged ||
+                 (pa.type == cudaMemoryTypeHost && (uint64_t)pa.devicePointer == addr)))
+        return "must be memory of the session's GPU (or mapped host memory)";
+    if ((addr & 7) != 0)
+        return "is not 8-byte aligned";
+    return nullptr;
+}
+
+/* the same decision for tests, without a GPU */
+extern "C" const char *xb_out_buffer_fault_of(int type, int device, uint64_t devptr, uint64_t addr, int dindex, int own)
+{
+    cudaPointerAttributes pa;
+    memset(&pa, 0, sizeof(pa));
+    pa.type = (cudaMemoryType)type;
+    pa.device = device;
+    pa.devicePointer = (void *)devptr;
+    return xb_out_buffer_fault(pa, addr, dindex, own != 0);
+}
+
+static int xb_check_out_buffer(const char *func, const char *name, const void *p, int dindex, bool own, kern_errorbuf *err)
+{
+    cudaPointerAttributes pa;
+    const char *why = "is not CUDA memory";
+    if (cudaPointerGetAttributes(&pa, p) == cudaSuccess)
+        why = xb_out_buffer_fault(pa, (uint64_t)p, dindex, own);
+    else
+        cudaGetLastError();
+    return why ? XB_ERR(err, ERRCODE_DEVICE_ERROR, "%s: %s %s (GPU %d)", func, name, why, dindex) : 0;
+}
+
 /* GPU-Sort of the session's groups: the entries of those kept by LIMIT or
  * the window rank, in order, in *p_list (work memory of run; *p_n of them).
  * run has counted the groups of the whole table.  Returns 0, or -1. */
@@ -542,10 +580,12 @@ xpuB200FinalNoAlloc(xpuB200Session *s, void *kds_final_dev, uint64_t buf_sz, uin
                       "point's fixed work space of %llu bytes serves; use xpuB200Final",
                       (unsigned long long)cap, (unsigned long long)XB_FINAL_SCRATCH_SLOTS,
                       (unsigned long long)XB_FINAL_SCRATCH_BYTES);
+    int rc = kds_final_dev ? xb_check_out_buffer("FinalNoAlloc", "kds_final_dev", kds_final_dev, dindex, true, err) : 0;
+    if (rc) return rc;
     XbFinalRun run(s);
     run.scratch = scratch;
     run.scratch_left = XB_FINAL_SCRATCH_BYTES;
-    int rc = run.plan(1, err);
+    rc = run.plan(1, err);
     if (rc) return rc;
     const XbFinalPart P = run.part(0, 0);
     if (p_required) *p_required = P.length;
@@ -731,7 +771,10 @@ xpuB200FinalParts(xpuB200Session *s, uint32_t nparts, void *parts_dev, uint64_t 
         return XB_ERR(err, ERRCODE_DEVICE_ERROR, "FinalParts needs a session with GROUP BY keys");
     if (plan->nsort)
         return XB_ERR(err, ERRCODE_DEVICE_ERROR, "GPU-Sort applies to the merged groups, not to their parts");
-    int rc = xb_gt_settle(s, err);
+    /* (another GPU's memory will do where the caller made it accessible) */
+    int rc = parts_dev ? xb_check_out_buffer("FinalParts", "parts_dev", parts_dev, s->dev->dindex, false, err) : 0;
+    if (rc) return rc;
+    rc = xb_gt_settle(s, err);
     if (rc) return rc;
     XbFinalRun run(s);
     rc = run.plan(nparts, err);

@@ -111,3 +111,24 @@ def test_chunk_checks_row_index_inside_the_chunk():
     assert _kds_check(buf)[0] == ord("E")
     for ch in tbl.row_chunks(rows_per_chunk=30):                  # chunks of the ROW producer
         assert _kds_check(ch) == (0, "")
+
+
+def test_output_buffers_of_other_memory_are_refused():
+    # the decision of FinalNoAlloc (own) and FinalParts on a caller's output
+    # buffer: kinds 0 unregistered, 1 pinned host, 2 device, 3 managed memory
+    L = ctypes.CDLL(xpu_b200.LIB_PATH)
+    fn = L.xb_out_buffer_fault_of
+    fn.restype = ctypes.c_char_p
+    fn.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_uint64, ctypes.c_uint64, ctypes.c_int, ctypes.c_int]
+    a = 0x7f0000001000
+    for own in (0, 1):
+        assert b"not CUDA memory" in fn(0, -2, 0, a, 0, own)
+        assert fn(2, 0, a, a, 0, own) is None
+        assert fn(3, 0, a, a, 0, own) is None
+        assert fn(1, 0, a, a, 0, own) is None
+        for odd in (1, 2, 4, 7):
+            assert b"aligned" in fn(2, 0, a + odd, a + odd, 0, own)
+    # another GPU's memory, host memory that is not mapped at its address
+    assert b"session's GPU" in fn(2, 1, a, a, 0, 1)
+    assert b"session's GPU" in fn(1, 0, 0, a, 0, 1)
+    assert fn(2, 1, a, a, 0, 0) is None

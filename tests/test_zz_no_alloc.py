@@ -139,3 +139,23 @@ def test_final_without_allocation_rejects_large_group_tables(device):
         assert "use xpuB200Final" in msg
     finally:
         s.close()
+
+
+def test_final_without_allocation_refuses_memory_it_cannot_write(device):
+    # pageable memory and a misaligned place are refused before anything
+    # runs; the next call serves as ever
+    torch = pytest.importorskip("torch")
+    s, sess, truth = _open(device, "scan")
+    try:
+        _, need, _, _ = _final_no_alloc(s, 0, 0)
+        host = np.zeros(need + 64, dtype=np.uint8)
+        rc, _, _, msg = _final_no_alloc(s, host.ctypes.data, need)
+        assert rc == ord("E") and "not CUDA memory" in msg
+        out = torch.zeros(need + 64, dtype=torch.uint8, device="cuda:0")
+        rc, _, _, msg = _final_no_alloc(s, out.data_ptr() + 4, need)
+        assert rc == ord("E") and "aligned" in msg
+        assert not host.any() and not out.cpu().numpy().any()
+        got, _ = _no_alloc_final_bytes(s)
+        assert F.compare_groups(F.decode_kds_final(got, sess), truth) == []
+    finally:
+        s.close()
