@@ -273,17 +273,14 @@ __device__ __forceinline__ uint32_t xbj_grow_seen(const uint32_t *buf, uint32_t 
     return *(volatile const uint32_t *)&buf[XBJ_GROW_WORD];
 }
 
-/* add *newg new groups to the table's count (one thread; nobody is
- * creating groups against newg meanwhile) */
+/* add *newg new groups to the table's count (one thread).  Taken by an
+ * exchange: other lanes may already be creating groups of their next rows */
 __device__ __forceinline__ void xbj_count_flush(xb_gtable *gt, uint32_t *newg)
 {
-    const uint32_t n = *(volatile uint32_t *)newg;
-    if (n) {
-        *(volatile uint32_t *)newg = 0;
+    const uint32_t n = atomicExch(newg, 0u);
+    if (n)
         xb_gt_count_new(gt, n);
-    }
 }
-
 
 /* one launch's (or one mixed-launch command's) work for this CTA; ends
  * with the counters and the shared group table flushed, without a final
