@@ -2016,10 +2016,21 @@ struct Gen {
      * read are loaded for rows that passed only.  20M rows into
      * 1.7M groups 2314 -> 1772 us a query, 500M rows into 10M groups 23.8 ->
      * 22.2 ms.  Heap rows, which would be decoded twice, lost 3 to 14% by
-     * it, and an aggregate without keys has too little to do per row. */
+     * it, and an aggregate without keys has too little to do per row.  Not
+     * where the quals save a value into a slot (SaveExpr), which later
+     * programs may read: a row taken from the queue is decoded again, the
+     * quals are not evaluated again. */
     bool compact() const
     {
-        return format == KDS_FORMAT_ARROW && p->scan_quals.count && p->has_groupby == 1;
+        if (format != KDS_FORMAT_ARROW || !p->scan_quals.count || p->has_groupby != 1)
+            return false;
+        for (uint32_t i = 0; i < p->scan_quals.count; i++) {
+            const xb_insn &in = p->insns[p->scan_quals.start + i];
+            const bool writes = in.op != XB_OP_MASK_PUSH && in.op != XB_OP_MASK_NARROW && in.op != XB_OP_MASK_POP;
+            if (writes && in.dst < p->nslots)
+                return false;
+        }
+        return true;
     }
 
     void pipeline()

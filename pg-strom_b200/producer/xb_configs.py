@@ -582,6 +582,38 @@ def arrow_groupby(nrows=500_000_000, nkeys=10_000_000, seed_config=2, rows_per_c
     return chunks, session, expect, meta
 
 
+def arrow_saved_qual_session(saved):
+    """WHERE v1 + 5 < 0 GROUP BY k -> count(*), sum(v1 + 5) over the Arrow
+    group-by's chunks; saved: the qual saves v1 + 5 into a slot (SaveExpr)
+    that the aggregate reads, else both evaluate it."""
+    class SavingBuilder(SessionBuilder):
+        def emit(self, buf, e, depth, flags=0):
+            if isinstance(e, tuple) and e[0] == "save":
+                self.emit_save(buf, e[1], depth)
+            elif isinstance(e, SavedSlot):
+                super().emit(buf, Var(-1, self._temp(e.expr, depth).slot, e.typ), depth, flags)
+            else:
+                super().emit(buf, e, depth, flags)
+
+        def _lookup_var(self, v, curr_depth):
+            return self.kvdefs[v.resno] if v.depth == -1 else super()._lookup_var(v, curr_depth)
+
+    class SavedSlot:
+        def __init__(self, expr):
+            self.expr, self.typ = expr, expr.typ
+
+        def __eq__(self, o):
+            return isinstance(o, SavedSlot) and o.expr == self.expr
+
+    v = Func("int4pl", [Var(0, 2, "int4"), Const("int4", 5)], "int4")
+    arg = SavedSlot(v) if saved else v
+    return SavingBuilder(0, DEVTASK_PREAGG | DEVKIND_GPU).build(
+        scan_quals=Func("int4lt", [("save", v) if saved else v, Const("int4", 0)], "bool"),
+        groupby_keys=[Var(0, 1, "int8")],
+        aggs=[Agg("NROWS_ANY"), Agg("PSUM_INT", Func("int4_to_int8", [arg], "int8"))],
+        ngroups_estimate=1e6)
+
+
 def _validity(valid: np.ndarray) -> np.ndarray:
     """Arrow validity bitmap (bit i set: row i has a value, least significant
     bit first)"""

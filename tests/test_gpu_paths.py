@@ -112,6 +112,17 @@ def test_compaction_arrow_units(device, nrows, batch):
     assert F.compare_groups(got, expect) == []
 
 
+def test_value_saved_by_the_quals(device):
+    # a SaveExpr in the scan quals whose slot an aggregate reads
+    chunks, _, _, _ = C.arrow_groupby(nrows=20_000, nkeys=500, rows_per_chunk=3_001, seed_config=65, with_expect=False)
+    for saved in (False, True):
+        sess = C.arrow_saved_qual_session(saved)
+        want = _oracle(sess, chunks)
+        assert len(want) == 500
+        got, _ = _run(device, sess, chunks)
+        assert F.compare_groups(got, want) == []
+
+
 # ---- chunk headers: more chunks than one fetch takes, a header larger than
 # its slot (30 columns)
 def test_many_chunks_in_a_batch(device):

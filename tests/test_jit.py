@@ -130,3 +130,24 @@ def test_generated_source_names_the_plan():
     # two join depths, a group-by and no interpreter loop
     assert "/* depth 1 */" in src and "/* depth 2 */" in src and "/* depth 3 */" not in src
     assert "xbj_group_get<true>" in src and "xb_vm_exec" not in src
+
+
+def _source(L, sess, km, fmt):
+    plan = _translate(L, sess, km)
+    n = ctypes.c_size_t(0)
+    buf = ctypes.create_string_buffer(1 << 21)
+    assert L.xb_jit_source(plan, ctypes.c_uint32(ord(fmt)), buf, ctypes.c_size_t(len(buf)), ctypes.byref(n)) == 0
+    return buf.value.decode()
+
+
+def test_quals_that_save_a_slot_are_not_compacted():
+    # a row taken from the queue is decoded again, and what the quals saved
+    # for later programs would be gone; And / Or in the quals and the same
+    # expression evaluated by the aggregates again do not matter
+    L = _lib()
+    for saved in (False, True):
+        src = _source(L, C.arrow_saved_qual_session(saved), None, "a")
+        assert ("#define XBJ_COMPACT 1" in src) == (not saved)
+    for case in ("arrow_groupby", "arrow_nulls"):
+        sess, km, _ = _session(case)
+        assert "#define XBJ_COMPACT 1" in _source(L, sess, km, "a"), case
