@@ -134,10 +134,12 @@ __device__ __forceinline__ void
 xbj_after_quals(XbjRegs &R, const XbjEnv &E, XbjCnt &C, bool &failed);
 
 #ifdef XBJ_ACC
-/* generated: a lane's aggregate, empty at first; all lanes of a warp added
- * to the one group's entry */
-__device__ __forceinline__ void xbj_acc_init(XbjAcc &A);
-__device__ __forceinline__ void xbj_acc_flush(XbjAcc &A, const XbjEnv &E);
+/* generated: a lane's aggregate, empty at first; its row counts moved to
+ * carried (XBJ_ACC words); all lanes of a warp added to the one group's
+ * entry */
+__device__ __forceinline__ void xbj_acc_init(XbjAcc &A, volatile unsigned long long *carried);
+__device__ __forceinline__ void xbj_acc_carry(XbjAcc &A, volatile unsigned long long *carried);
+__device__ __forceinline__ void xbj_acc_flush(XbjAcc &A, volatile unsigned long long *carried, const XbjEnv &E);
 
 /* s + c += x, the rounding error of the sum kept in c (TwoSum) */
 __device__ __forceinline__ void xbj_two_sum(double &s, double &c, double x)
@@ -337,7 +339,8 @@ xbj_body(const XbExecArgs &args, char *smem)
     C.raw = C.in = C.out = 0;
     C.gready = 0;
 #ifdef XBJ_ACC
-    xbj_acc_init(C.acc);
+    volatile unsigned long long carried[XBJ_ACC];
+    xbj_acc_init(C.acc, carried);
 #endif
 #pragma unroll
     for (int d = 0; d <= XB_MAX_DEPTH; d++)
@@ -524,8 +527,12 @@ xbj_body(const XbExecArgs &args, char *smem)
 #pragma unroll
         for (int d = 1; d <= XBJ_NRELS; d++)
             big |= C.depth[d];
-        if (big & 0x80000000u)
+        if (big & 0x80000000u) {
             xbj_flush_cnt(C, args.st);
+#ifdef XBJ_ACC
+            xbj_acc_carry(C.acc, carried);
+#endif
+        }
         if (__any_sync(XB_FULL, failed)) {
             stop = false;
             break;
@@ -546,7 +553,7 @@ xbj_body(const XbExecArgs &args, char *smem)
 #endif
     __syncwarp();
 #ifdef XBJ_ACC
-    xbj_acc_flush(C.acc, E);
+    xbj_acc_flush(C.acc, carried, E);
     __syncwarp();
 #endif
     if (lane == 0 && args.gt)

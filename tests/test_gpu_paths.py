@@ -93,6 +93,26 @@ def test_no_group_by_state_forms(device, nrows, limit):
     assert F.compare_groups(got, {(): want}) == []
 
 
+def test_no_group_by_over_a_join(device):
+    # joined rows counted and summed in the lanes' registers
+    fact, _, km, _, meta = C.join_groupby(nfact=30_000, ndim1=100, ndim2=10, seed_config=66)
+    k1, k2 = Var(0, 1, "int4"), Var(0, 2, "int4")
+    sess = SessionBuilder(2, C.DEVTASK_PREAGG | C.DEVKIND_GPU).build(
+        joins=[([k1], [Func("int4eq", [k1, Var(1, 1, "int4")], "bool")], []),
+               ([k2], [Func("int4eq", [k2, Var(2, 1, "int4")], "bool")], [])],
+        aggs=[Agg("NROWS_ANY"), Agg("PSUM_INT", Func("int4_to_int8", [k1], "int8")),
+              Agg("PMAX_INT32", Var(1, 1, "int4")), Agg("PMIN_INT32", k2)],
+        ngroups_estimate=1.0)
+    chunks = fact.block_chunks(pages_per_chunk=100)
+    o = O.Oracle(sess, km)
+    for ch in chunks:
+        o.exec(ch)
+    want = F.decode_kds_final(o.final(), sess)
+    o.close()
+    got, _ = _run(device, sess, chunks, km, 2)
+    assert want and F.compare_groups(got, want) == []
+
+
 # ---- rows compacted between the quals and the rest: none, few, all pass;
 # pages and units of a few rows; a filtered projection
 @pytest.mark.parametrize("limit", [0, 1, 500, 1000])

@@ -151,3 +151,28 @@ def test_quals_that_save_a_slot_are_not_compacted():
     for case in ("arrow_groupby", "arrow_nulls"):
         sess, km, _ = _session(case)
         assert "#define XBJ_COMPACT 1" in _source(L, sess, km, "a"), case
+
+
+def test_counts_without_group_by_are_64_bit():
+    # a lane counts its rows in registers over the whole launch: in 64 bits
+    # behind a join, else carried into 64 bits where the statistics are
+    # flushed; aggregates that count the same rows share a counter
+    from xb_producer import Agg, Const, Func, SessionBuilder, Var
+    L = _lib()
+    scan, _, _ = _session("scan_nogroup")
+    _, _, km, _, _ = C.join_groupby(nfact=1000, ndim1=100, ndim2=10)
+    join = SessionBuilder(2, C.DEVTASK_PREAGG | C.DEVKIND_GPU).build(
+        joins=[([Var(0, 1, "int4")], [Func("int4eq", [Var(0, 1, "int4"), Var(1, 1, "int4")], "bool")], []),
+               ([Var(0, 2, "int4")], [Func("int4eq", [Var(0, 2, "int4"), Var(2, 1, "int4")], "bool")], [])],
+        aggs=[Agg("NROWS_ANY"), Agg("PSUM_INT", Func("int4_to_int8", [Var(1, 1, "int4")], "int8"))],
+        ngroups_estimate=1.0)
+    for sess, k, typ in ((scan, None, ["uint32_t"]), (join, km, ["unsigned", "long", "long"])):
+        src = _source(L, sess, k, "b")
+        acc = src[src.index("struct XbjAcc {"):]
+        counts = [ln.split() for ln in acc[:acc.index("};")].splitlines() if ln.split()[-1].startswith("n")]
+        assert counts and all(c[:-1] == typ for c in counts)
+        for i, c in enumerate(counts):
+            n = c[-1][:-1]
+            assert src.count("A.%s++" % n) == 1
+            assert "carried[%d] += A.%s; A.%s = 0;" % (i, n, n) in src
+            assert "xbj_warp_sum(carried[%d] + A.%s)" % (i, n) in src
