@@ -302,7 +302,7 @@ xb_update_states_warp(const xb_plan *plan, char *e, const XbRegs &R, uint32_t la
         case KAGG_ACTION__PSUM_FP: case KAGG_ACTION__PAVG_FP:
             atomicAdd((unsigned long long *)s, cnt);
             xb_atomic_add_f64c((double *)(s + 8), (double *)(s + 16), fs);
-            if (fc != 0.0)
+            if (fabs(fc) > 0.0)
                 atomicAdd((double *)(s + 16), fc);
             break;
         default:

@@ -196,14 +196,16 @@ __device__ __forceinline__ void xb_atomic_add_i128(uint64_t *p, xb_i128 v)
 }
 
 /* compensated atomic sum: hi accumulates the rounded sum, lo the exact
- * rounding error of each addition (TwoSum on the value atomicAdd saw) */
+ * rounding error of each addition (TwoSum on the value atomicAdd saw).  Of a
+ * sum that is no longer finite the error is NaN: it is left out, hi alone is
+ * the infinity or NaN that a plain sum gives */
 __device__ __forceinline__ void xb_atomic_add_f64c(double *hi, double *lo, double x)
 {
     double old = atomicAdd(hi, x);
     double s = __dadd_rn(old, x);
     double bp = __dsub_rn(s, old);
     double e = __dadd_rn(__dsub_rn(old, __dsub_rn(s, bp)), __dsub_rn(x, bp));
-    if (e != 0.0)
+    if (fabs(e) > 0.0)
         atomicAdd(lo, e);
 }
 
@@ -226,7 +228,7 @@ __device__ __forceinline__ void xb_atomic_add_f64c_g(double *hi, double *lo, dou
     double s = __dadd_rn(old, x);
     double bp = __dsub_rn(s, old);
     double e = __dadd_rn(__dsub_rn(old, __dsub_rn(s, bp)), __dsub_rn(x, bp));
-    if (e != 0.0)
+    if (fabs(e) > 0.0)
         xb_red_g_add_f64(lo, e);
 }
 
@@ -268,7 +270,7 @@ __device__ __forceinline__ void xb_f64c_err_g(void *lo, double old, double x)
     const double s = __dadd_rn(old, x);
     const double bp = __dsub_rn(s, old);
     const double e = __dadd_rn(__dsub_rn(old, __dsub_rn(s, bp)), __dsub_rn(x, bp));
-    if (e != 0.0)
+    if (fabs(e) > 0.0)
         xb_red_g_add_f64(lo, e);
 }
 
@@ -427,7 +429,7 @@ static __device__ __noinline__ void xb_merge_states(const xb_plan *plan, char *d
                     xb_atomic_add_f64c((double *)(d + k), (double *)(d + k + 8),
                                        *(const double *)(s + k));
                     double lo = *(const double *)(s + k + 8);
-                    if (lo != 0.0)
+                    if (fabs(lo) > 0.0)
                         atomicAdd((double *)(d + k + 8), lo);
                 }
             }

@@ -1046,7 +1046,7 @@ struct Gen {
                            "        if (leader && " << n << ") {\n"
                            "            xb_atomic_add_f64c((double *)(" << S << " + " << 8 + 16 * k << "), (double *)(" << S
                         << " + " << 16 + 16 * k << "), A.s" << K << ");\n"
-                           "            if (A.c" << K << " != 0.0) atomicAdd((double *)(" << S << " + " << 16 + 16 * k
+                           "            if (fabs(A.c" << K << ") > 0.0) atomicAdd((double *)(" << S << " + " << 16 + 16 * k
                         << "), A.c" << K << ");\n"
                            "        }\n";
                 }
@@ -1278,7 +1278,7 @@ struct Gen {
                 for (uint32_t k = 8; k + 16 <= a.state_sz; k += 16)
                     o << "            xb_atomic_add_f64c_g((double *)(" << D << " + " << k << "), (double *)(" << D << " + "
                       << k + 8 << "), *(const double *)(" << S << " + " << k << "));\n"
-                         "            if (*(const double *)(" << S << " + " << k + 8 << ") != 0.0) xb_red_g_add_f64("
+                         "            if (fabs(*(const double *)(" << S << " + " << k + 8 << ")) > 0.0) xb_red_g_add_f64("
                       << D << " + " << k + 8 << ", *(const double *)(" << S << " + " << k + 8 << "));\n";
                 o << "        }\n";
                 break;

@@ -113,6 +113,65 @@ def test_no_group_by_over_a_join(device):
     assert want and F.compare_groups(got, want) == []
 
 
+# ---- infinities, NaN and the ends of int8 in every form of the updates: the
+# groups' states start at INT64_MAX / INT64_MIN, which values may equal
+def _extreme_table(nrows):
+    r = np.random.default_rng(67)
+    g = (np.arange(nrows) % 8).astype(np.int32)
+    b = r.integers(-1000, 1000, nrows).astype(np.float64)       # finite sums are exact
+    pick = (np.arange(nrows) // 8) % 5
+    b[(g == 1) & (pick == 2)] = np.inf
+    b[(g == 2) & (pick == 3)] = -np.inf
+    b[(g == 3) & (pick == 1)] = np.inf
+    b[(g == 3) & (pick == 4)] = -np.inf
+    b[(g == 4) & (pick == 0)] = np.nan
+    b[g == 6] = np.inf
+    b[g == 7] = -np.inf
+    top, low = np.iinfo(np.int64).max, np.iinfo(np.int64).min
+    w = r.integers(-5, 6, nrows, dtype=np.int64)
+    w[g == 0], w[g == 1] = top, low
+    w[(g == 2) & (pick == 1)], w[(g == 2) & (pick == 2)] = top, low
+    return Table("t", [Column("w", "int8", values=w), Column("b", "float8", values=b, nulls=(g == 5)),
+                       Column("g", "int4", values=g)], nrows)
+
+
+def _plain(groups):
+    """decoded groups with floats as comparable texts, undefined values left out"""
+    one = lambda v: repr(float(v)) if isinstance(v, (float, np.floating)) else v        # noqa: E731
+    return {k: [tuple(one(x) for x in (s[:1] if s[0] == 0 else s)) if isinstance(s, tuple) else one(s) for s in v]
+            for k, v in groups.items()}
+
+
+@pytest.mark.parametrize("path", ["vm", "shared", "global", "slices", "none"])
+def test_extreme_values(device, monkeypatch, path):
+    monkeypatch.setenv("XPU_B200_JIT", "0" if path == "vm" else "1")
+    monkeypatch.setenv("XPU_B200_PARTITION", "1" if path == "slices" else "0")
+    vw, vb, vg = Var(0, 1, "int8"), Var(0, 2, "float8"), Var(0, 3, "int4")
+    aggs = [Agg("NROWS_ANY"), Agg("PMIN_INT64", vw), Agg("PMAX_INT64", vw), Agg("PMIN_FP64", vb), Agg("PMAX_FP64", vb),
+            Agg("PSUM_FP", vb), Agg("PAVG_INT64", vw), Agg("STDDEV", vb), Agg("COVAR", vb, arg1=vb)]
+    chunks = _extreme_table(6_000).block_chunks(pages_per_chunk=20)
+    flags = C.DEVTASK_PREAGG | C.DEVKIND_GPU
+    if path == "none":
+        sessions = [SessionBuilder(0, flags).build(scan_quals=Func("int4eq", [vg, Const("int4", i)], "bool"), aggs=aggs,
+                                                   ngroups_estimate=1.0) for i in range(8)]
+    else:
+        est = {"global": 20_000.0, "slices": 1_000_000.0}.get(path, 8.0)
+        sessions = [SessionBuilder(0, flags).build(groupby_keys=[vg], aggs=aggs, ngroups_estimate=est)]
+    for sess in sessions:
+        want = _plain(_oracle(sess, chunks))
+        s = xpu_b200.Session(device, sess)
+        try:
+            for ch in chunks:
+                s.exec(ch)
+            got = _plain(F.decode_kds_final(s.final()[0], sess))
+            info = s.info()
+        finally:
+            s.close()
+        assert info["kernels"] == {"b": "vm" if path == "vm" else "jit"}, info
+        assert info["partition_used"] == (path == "slices"), info
+        assert got == want
+
+
 # ---- rows compacted between the quals and the rest: none, few, all pass;
 # pages and units of a few rows; a filtered projection
 @pytest.mark.parametrize("limit", [0, 1, 500, 1000])
