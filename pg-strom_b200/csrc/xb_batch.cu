@@ -54,7 +54,7 @@ xpuB200BatchCreate(xpuB200Session *s, const kern_data_store *const *kds_dev, uin
         if (((uintptr_t)kds_dev[i] & 7) != 0)
             return XB_ERR(err, ERRCODE_DEVICE_ERROR, "chunk %u is not 8-byte aligned", i);
     std::vector<std::vector<char>> heads;
-    int rc = xb_fetch_heads(s->dev, s->stream, kds_dev, nchunks, heads, err);
+    int rc = xb_fetch_heads(s->dev, kds_dev, nchunks, heads, err);
     if (rc) return rc;
     for (uint32_t i = 0; i < nchunks; i++) {
         const kern_data_store *h = (const kern_data_store *)heads[i].data();
@@ -418,7 +418,7 @@ xpuB200MixCreate(xpuB200Device *dev, uint32_t ncmds, xpuB200Session *const *sess
         if (((uintptr_t)kds_dev[i] & 7) != 0)
             return XB_ERR(err, ERRCODE_DEVICE_ERROR, "command %u: chunk is not 8-byte aligned", i);
     }
-    int hrc = xb_fetch_heads(dev, dev->stream, kds_dev, ncmds, heads, err);
+    int hrc = xb_fetch_heads(dev, kds_dev, ncmds, heads, err);
     if (hrc) return hrc;
     for (uint32_t i = 0; i < ncmds; i++) {
         xpuB200Session *s = sess[i];

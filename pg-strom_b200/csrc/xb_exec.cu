@@ -2592,13 +2592,16 @@ static uint64_t xb_device_room(int dindex, const void *p)
 /*
  * One kernel gathers up to XB_HEADS headers into pinned memory and one wait
  * ends the fetch (two synchronous copies per chunk took 30 us each: 2.3 ms
- * of a 4.2 ms query over 78 chunks).  Pointers that are not plainly this
- * device's memory, and headers that do not fit a slot, are copied by
- * themselves, so that a bad pointer is the copy's error as before.  A
- * synchronous copy is ordered after the legacy stream's work; so is the
- * kernel.
+ * of a 4.2 ms query over 78 chunks).  A single header is copied: the kernel
+ * waits for a free place on an SM, which the launches of other sessions fill
+ * (Submit beside a session whose launches take 4.5 ms: 3.0 ms with the
+ * kernel, 0.12 ms with the copy, as on an idle GPU).  Pointers that are not
+ * plainly this device's memory, and headers that do not fit a slot, are
+ * copied by themselves, so that a bad pointer is the copy's error as before.
+ * A synchronous copy is ordered after the legacy stream's work; so is the
+ * fetch, on a stream of its own that waits for nothing else.
  */
-int xb_fetch_heads(xpuB200Device *dev, cudaStream_t st, const kern_data_store *const *kds, uint32_t n,
+int xb_fetch_heads(xpuB200Device *dev, const kern_data_store *const *kds, uint32_t n,
                    std::vector<std::vector<char>> &heads, kern_errorbuf *err)
 {
     const size_t head0 = offsetof(kern_data_store, colmeta);
@@ -2614,11 +2617,14 @@ int xb_fetch_heads(xpuB200Device *dev, cudaStream_t st, const kern_data_store *c
     if (!sc.mem) {
         if (cudaMallocHost((void **)&sc.mem, XB_HEADS * (sizeof(XbHeadReq) + XB_HEAD_SLOT)) != cudaSuccess)
             sc.mem = nullptr;
-        else if (cudaEventCreateWithFlags(&sc.ev, cudaEventDisableTiming) != cudaSuccess) {
+        else if (cudaEventCreateWithFlags(&sc.ev, cudaEventDisableTiming) != cudaSuccess ||
+                 cudaStreamCreateWithFlags(&sc.st, cudaStreamNonBlocking) != cudaSuccess) {
+            if (sc.ev) cudaEventDestroy(sc.ev);
             cudaFreeHost(sc.mem);
-            sc.mem = nullptr;
+            sc = xb_head_scratch();
         }
     }
+    const cudaStream_t st = sc.st;
     cudaError_t rc = sc.mem ? cudaSuccess : cudaErrorMemoryAllocation;
     if (rc == cudaSuccess && (rc = cudaEventRecord(sc.ev, cudaStreamLegacy)) == cudaSuccess)
         rc = cudaStreamWaitEvent(st, sc.ev, 0);
@@ -2637,8 +2643,14 @@ int xb_fetch_heads(xpuB200Device *dev, cudaStream_t st, const kern_data_store *c
         }
         if (!k)
             continue;
-        xb_gather_heads<<<k, 128, 0, st>>>(req, slots);
-        if ((rc = cudaGetLastError()) == cudaSuccess)
+        if (n == 1) {
+            rc = cudaMemcpyAsync(slots, req[0].kds, req[0].avail < XB_HEAD_SLOT ? req[0].avail : XB_HEAD_SLOT,
+                                 cudaMemcpyDeviceToHost, st);
+        } else {
+            xb_gather_heads<<<k, 128, 0, st>>>(req, slots);
+            rc = cudaGetLastError();
+        }
+        if (rc == cudaSuccess)
             rc = cudaStreamSynchronize(st);
         for (uint32_t j = 0; rc == cudaSuccess && j < k; j++) {
             const kern_data_store *h = (const kern_data_store *)(slots + (size_t)j * XB_HEAD_SLOT);
@@ -2826,6 +2838,7 @@ xpuB200Shutdown(xpuB200Device *dev)
     for (xb_head_scratch &sc : dev->free_heads) {
         cudaFreeHost(sc.mem);
         cudaEventDestroy(sc.ev);
+        cudaStreamDestroy(sc.st);
     }
     delete dev;
 }
@@ -4252,7 +4265,7 @@ static int xb_place_src(xpuB200Session *s, const kern_data_store *kds_src, int k
         if (((uintptr_t)kds_src & 7) != 0)
             return XB_ERR(err, ERRCODE_DEVICE_ERROR, "device chunk is not 8-byte aligned");
         std::vector<std::vector<char>> hb;
-        int rc = xb_fetch_heads(s->dev, st, &kds_src, 1, hb, err);
+        int rc = xb_fetch_heads(s->dev, &kds_src, 1, hb, err);
         if (rc) return rc;
         hbuf.swap(hb[0]);
         memcpy(&head, hbuf.data(), offsetof(kern_data_store, colmeta));

@@ -41,6 +41,7 @@ struct xb_pinned {
 struct xb_head_scratch {
     char           *mem = nullptr;
     cudaEvent_t     ev = nullptr;
+    cudaStream_t    st = nullptr;           /* the fetch's own: no session's work to wait for */
 };
 
 struct xpuB200Device {
@@ -220,7 +221,7 @@ void xb_account_status(xpuB200Session *s, const xb_status *hs, kern_exec_results
 int xb_check_kds(const kern_data_store *kds, kern_errorbuf *err);
 /* the headers of n chunks in this device's memory (each 8-byte aligned),
  * copied to the host */
-int xb_fetch_heads(xpuB200Device *dev, cudaStream_t st, const kern_data_store *const *kds, uint32_t n,
+int xb_fetch_heads(xpuB200Device *dev, const kern_data_store *const *kds, uint32_t n,
                    std::vector<std::vector<char>> &heads, kern_errorbuf *err);
 uint32_t xb_chunk_units(const kern_data_store *head);
 void xb_fill_results(const xb_status *hs, uint32_t nrels, kern_exec_results *results);

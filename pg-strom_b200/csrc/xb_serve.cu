@@ -535,7 +535,7 @@ xpuB200Submit(xpuB200Session *s, const kern_data_store *kds_src, int kds_src_on_
         if (((uintptr_t)kds_src & 7) != 0)
             return XB_ERR(err, ERRCODE_DEVICE_ERROR, "device chunk is not 8-byte aligned");
         std::vector<std::vector<char>> heads;
-        rc = xb_fetch_heads(dev, s->stream, &kds_src, 1, heads, err);
+        rc = xb_fetch_heads(dev, &kds_src, 1, heads, err);
         if (rc) return rc;
         hb.swap(heads[0]);
     } else {

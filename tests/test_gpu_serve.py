@@ -166,3 +166,49 @@ def test_new_plan_shape_served_while_its_kernel_builds(device, alone):
     want = F.decode_kds_final(o.final(), sess)
     o.close()
     assert F.compare_groups(F.decode_kds_final(final, sess), want) == []
+
+
+def test_submit_does_not_wait_for_other_launches(device, monkeypatch):
+    """Submit of a device chunk reads its header at once, while launches of
+    another session fill the GPU."""
+    import threading
+    import time
+    monkeypatch.setenv("XPU_B200_JIT", "0")
+    tbl, sess, _, _, _ = C.scan_groupby(nrows=1_000_000, seed_config=92)
+    ups = [device.upload(c) for c in tbl.block_chunks(pages_per_chunk=4000)]
+    busy = xpu_b200.Session(device, sess)
+    b = busy.batch([p for _, p in ups] * 64)
+    monkeypatch.setenv("XPU_B200_JIT", "1")
+    small, ssess, _, expect, _ = C.scan_groupby(nrows=900, seed_config=93)
+    chunk, = small.block_chunks()
+    base, p = device.upload(chunk)
+    s = xpu_b200.Session(device, ssess)
+    try:
+        launch_ms = b.time(1)
+        s.exec(p, on_device=True)                   # its kernel is built
+        stop = threading.Event()
+
+        def loop():
+            while not stop.is_set():
+                b.time(1)
+        t = threading.Thread(target=loop)
+        t.start()
+        took = []
+        for _ in range(20):
+            t0 = time.perf_counter()
+            ticket = device.submit(s, p, on_device=True)
+            took.append((time.perf_counter() - t0) * 1e3)
+            device.poll(ticket)
+        stop.set()
+        t.join()
+        assert launch_ms > 4.0, launch_ms           # a launch long enough to tell
+        assert float(np.median(took)) < launch_ms / 4, (took, launch_ms)
+        got = F.decode_kds_final(s.final()[0], ssess)
+        assert {k: v[0] for k, v in got.items()} == {k: 21 * v["nrows"] for k, v in expect.items()}
+    finally:
+        b.close()
+        busy.close()
+        s.close()
+        for x, _ in ups:
+            device.free(x)
+        device.free(base)
