@@ -2442,6 +2442,11 @@ struct JitJob {
 };
 std::atomic<int> g_jobs_running{0};
 std::atomic<bool> g_exiting{false};
+/* the builds under way, by GPU and source: sessions of one plan shape that
+ * open meanwhile wait for the same one (a build each was hundreds of threads
+ * compiling the same source when clients opened sessions quickly) */
+std::mutex g_jobs_lock;
+std::map<std::pair<int, std::string>, std::shared_ptr<JitJob>> g_jobs;
 
 void jobs_at_exit()
 {
@@ -2457,14 +2462,24 @@ xb_jit_build_async(const xb_plan *plan, uint32_t format, int dindex, int min_blo
 {
     static std::once_flag once;
     std::call_once(once, [] { std::atexit(jobs_at_exit); });
+    Gen g;
+    g.p = plan;
+    g.format = format;
+    g.minb = (min_blocks >= 1 && min_blocks <= 8) ? min_blocks : 0;
+    const auto key = std::make_pair(dindex, g.run());
+    std::lock_guard<std::mutex> jobs(g_jobs_lock);
+    auto it = g_jobs.find(key);
+    if (it != g_jobs.end())
+        return new std::shared_ptr<JitJob>(it->second);
     auto job = std::make_shared<JitJob>();
     memcpy(&job->plan, plan, sizeof(xb_plan));
     job->format = format;
     job->dindex = dindex;
     job->minb = min_blocks;
+    g_jobs[key] = job;
     g_jobs_running++;
     try {
-        std::thread([job]() {
+        std::thread([job, key]() {
             if (!g_exiting) {
                 cudaSetDevice(job->dindex);
                 const int rc = jit_build(&job->plan, job->format, job->dindex, job->minb, false, &job->fn,
@@ -2474,13 +2489,24 @@ xb_jit_build_async(const xb_plan *plan, uint32_t format, int dindex, int min_blo
                 snprintf(job->msg, sizeof(job->msg), "process exiting");
                 job->state = -1;
             }
+            {
+                std::lock_guard<std::mutex> done(g_jobs_lock);
+                g_jobs.erase(key);
+            }
             g_jobs_running--;
         }).detach();
     } catch (...) {
+        g_jobs.erase(key);
         g_jobs_running--;
         return nullptr;
     }
     return new std::shared_ptr<JitJob>(job);
+}
+
+/* for tests: builds under way */
+extern "C" int xb_jit_jobs_running(void)
+{
+    return g_jobs_running.load();
 }
 
 extern "C" int

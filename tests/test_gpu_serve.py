@@ -168,6 +168,37 @@ def test_new_plan_shape_served_while_its_kernel_builds(device, alone):
     assert F.compare_groups(F.decode_kds_final(final, sess), want) == []
 
 
+def test_sessions_of_a_new_shape_share_one_build(device):
+    """Commands of many sessions of a plan shape without a kernel: one
+    background build serves them all."""
+    import ctypes
+    import time
+    running = ctypes.CDLL(xpu_b200.LIB_PATH).xb_jit_jobs_running
+    tbl, _, _, _, _ = C.scan_groupby(nrows=20_000, seed_config=94)
+    chunk = tbl.block_chunks(pages_per_chunk=60)[0]
+    sess = _rare_shape_session(variant=2)
+    deadline = time.perf_counter() + 60.0
+    while running() and time.perf_counter() < deadline:     # earlier tests'
+        time.sleep(0.01)
+    sessions = [xpu_b200.Session(device, sess) for _ in range(24)]
+    try:
+        tickets = [device.submit(s, chunk) for s in sessions]
+        seen = running()
+        for k in tickets:
+            device.poll(k)
+        assert seen <= 1, seen
+        got = [F.decode_kds_final(s.final()[0], sess) for s in sessions]
+        for g in got[1:]:
+            assert F.compare_groups(g, got[0]) == []
+        while running() and time.perf_counter() < deadline:
+            time.sleep(0.01)
+        device.poll(device.submit(sessions[0], chunk))
+        assert sessions[0].info()["kernels"] == {"b": "jit"}
+    finally:
+        for s in sessions:
+            s.close()
+
+
 def test_submit_does_not_wait_for_other_launches(device, monkeypatch):
     """Submit of a device chunk reads its header at once, while launches of
     another session fill the GPU."""
