@@ -41,6 +41,8 @@ typedef struct xpuB200Session xpuB200Session;
  */
 int  xpuB200Init(int cuda_dindex, uint64_t hbm_budget,
                  xpuB200Device **p_dev, kern_errorbuf *err);
+/* (waits for specialised kernels still being built in the background: a
+ * process calls it before it ends) */
 void xpuB200Shutdown(xpuB200Device *dev);
 
 /*

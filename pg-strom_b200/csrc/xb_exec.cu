@@ -2821,6 +2821,7 @@ extern "C" void
 xpuB200Shutdown(xpuB200Device *dev)
 {
     if (!dev) return;
+    xb_jit_wait_builds(0);
     cudaSetDevice(dev->dindex);
     xb_sched_destroy(dev);
     for (xb_inner_entry *e : dev->inner_cache)

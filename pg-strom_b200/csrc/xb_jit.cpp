@@ -2448,14 +2448,27 @@ std::atomic<bool> g_exiting{false};
 std::mutex g_jobs_lock;
 std::map<std::pair<int, std::string>, std::shared_ptr<JitJob>> g_jobs;
 
+void wait_for_jobs()
+{
+    for (int i = 0; i < 3000 && g_jobs_running.load() > 0; i++)
+        std::this_thread::sleep_for(std::chrono::milliseconds(10));
+}
+
 void jobs_at_exit()
 {
     /* builds still running may not outlive the objects they use */
     g_exiting = true;
-    for (int i = 0; i < 3000 && g_jobs_running.load() > 0; i++)
-        std::this_thread::sleep_for(std::chrono::milliseconds(10));
+    wait_for_jobs();
 }
 }   /* namespace */
+
+extern "C" void
+xb_jit_wait_builds(int exiting)
+{
+    if (exiting)
+        g_exiting = true;
+    wait_for_jobs();
+}
 
 extern "C" void *
 xb_jit_build_async(const xb_plan *plan, uint32_t format, int dindex, int min_blocks)

@@ -54,6 +54,10 @@ void *xb_jit_build_async(const xb_plan *plan, uint32_t format, int dindex, int m
 int   xb_jit_job_poll(void *job, void **p_func, void **p_mixfn, void **p_replay, double *p_compile_ms,
                       char *errbuf, size_t errlen);
 void  xb_jit_job_release(void *job);
+/* wait for the builds under way; exiting: those not begun stay unbuilt.  To
+ * be called before exit(): the compiler's own exit handlers, registered
+ * after the library's, take its tables away from a build that runs */
+void  xb_jit_wait_builds(int exiting);
 
 /* bytes of one deferred-row record of partitioned aggregation for plan
  * and source format (0: its kernel does not defer group updates); the replay kernel is

@@ -5,6 +5,7 @@ The product is libxpu_b200.so; this module only marshals buffers for tests
 and the benchmark.  Loading fails loudly when the library is missing: there
 is no fallback implementation.
 """
+import atexit
 import ctypes
 import os
 import struct
@@ -40,6 +41,10 @@ def lib():
         if not os.path.exists(LIB_PATH):
             raise RuntimeError(f"{LIB_PATH} is missing: build it with pg-strom_b200/build.py")
         L = ctypes.CDLL(LIB_PATH)
+        # background kernel builds end before the compiler's exit handlers run
+        L.xb_jit_wait_builds.argtypes = [ctypes.c_int]
+        L.xb_jit_wait_builds.restype = None
+        atexit.register(L.xb_jit_wait_builds, 1)
         P, U64, I = ctypes.c_void_p, ctypes.c_uint64, ctypes.c_int
         EB = ctypes.POINTER(KernErrorbuf)
         L.xpuB200Init.argtypes = [I, U64, ctypes.POINTER(P), EB]

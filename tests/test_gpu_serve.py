@@ -243,3 +243,30 @@ def test_submit_does_not_wait_for_other_launches(device, monkeypatch):
         for x, _ in ups:
             device.free(x)
         device.free(base)
+
+
+_EXIT_DURING_BUILD = """
+import sys, time
+sys.path[:0] = %r
+import xb_configs as C, xpu_b200
+from test_gpu_serve import _rare_shape_session
+dev = xpu_b200.Device(0)
+tbl, _, _, _, _ = C.scan_groupby(nrows=5_000, seed_config=95)
+s = xpu_b200.Session(dev, _rare_shape_session(variant=3))
+dev.poll(dev.submit(s, tbl.block_chunks()[0]))
+time.sleep(%f)
+"""
+
+
+@pytest.mark.parametrize("wait", [0.3, 0.6, 1.0])
+def test_process_that_ends_during_a_build(device, wait):
+    """Python ends while the specialised kernel is compiled in the
+    background: the process ends normally."""
+    import os
+    import subprocess
+    import sys
+    here = os.path.dirname(os.path.abspath(__file__))
+    paths = [here] + [p for p in sys.path if p]
+    p = subprocess.run([sys.executable, "-c", _EXIT_DURING_BUILD % (paths, wait)], capture_output=True, text=True,
+                       timeout=120)
+    assert p.returncode == 0, (p.returncode, p.stderr[-2000:])
