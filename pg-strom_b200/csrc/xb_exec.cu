@@ -3186,10 +3186,11 @@ xpuB200OpenSession(xpuB200Device *dev, const kern_session_info *session, uint64_
         const uint64_t limit = (uint64_t)in->nitems * 4 > 4096 ? (uint64_t)in->nitems * 4 : 4096;
         if (range > limit || range > (1ULL << 28)) {
             /* found through the index: the live columns packed per row, one
-             * or a few 16-byte loads in place of a load per column */
+             * or a few 16-byte loads in place of a load per column (without
+             * the memory for them, the columns as they are) */
             const uint32_t rs = xb_drec_layout(in, s->h_plan->rk, -1, nullptr, nullptr, nullptr);
-            if (in->live && !(in->live >> 31) && in->nitems > 0 && rs <= 64) {
-                DALLOC((size_t)in->nitems * rs, &in->dpay);
+            if (in->live && !(in->live >> 31) && in->nitems > 0 && rs <= 64 &&
+                xb_dalloc(s, (size_t)in->nitems * rs, (void **)&in->dpay, nullptr) == 0) {
                 in->drec_size = rs;
                 cudaMemcpyAsync(&s->d_plan->inner[d], in, sizeof(xb_inner), cudaMemcpyHostToDevice, st);
                 int grid = (int)((in->cap_mask + 1ULL + XB_BLOCK - 1) / XB_BLOCK);
