@@ -26,6 +26,8 @@
  * ---------------------------------------------------------------- */
 struct xpuB200Batch {
     xpuB200Session *sess;
+    int             dindex;         /* the session's GPU and stream, to free d_tasks by: the */
+    cudaStream_t    stream;         /* session may be closed first (streams are pooled) */
     xb_task        *d_tasks;
     uint32_t        ntasks;
     uint64_t        nunits;
@@ -81,6 +83,8 @@ xpuB200BatchCreate(xpuB200Session *s, const kern_data_store *const *kds_dev, uin
     }
     xpuB200Batch *b = new xpuB200Batch();
     b->sess = s;
+    b->dindex = s->dev->dindex;
+    b->stream = s->stream;
     b->ntasks = nchunks;
     b->nunits = base;
     b->format = format;
@@ -268,8 +272,8 @@ extern "C" void
 xpuB200BatchDestroy(xpuB200Batch *b)
 {
     if (!b) return;
-    cudaSetDevice(b->sess->dev->dindex);
-    cudaFreeAsync(b->d_tasks, b->sess->stream);
+    cudaSetDevice(b->dindex);
+    cudaFreeAsync(b->d_tasks, b->stream);
     delete b;
 }
 

@@ -222,6 +222,25 @@ def test_many_chunks_in_a_batch(device):
     assert F.compare_groups(F.decode_kds_final(final, sess), _truth(expect)) == []
 
 
+def test_batch_closed_after_its_session(device):
+    tbl, sess, _, expect, meta = C.scan_groupby(nrows=5_000, seed_config=68)
+    ups = [device.upload(c) for c in tbl.block_chunks(pages_per_chunk=20)]
+    try:
+        for _ in range(3):
+            s = xpu_b200.Session(device, sess)
+            b = s.batch([p for _, p in ups])
+            assert b.exec()["nitems_in"] == meta["nitems_in"]
+            got = F.decode_kds_final(s.final()[0], sess)
+            s.close()
+            other = xpu_b200.Session(device, sess)      # takes the pooled stream
+            b.close()
+            other.close()
+            assert F.compare_groups(got, _truth(expect)) == []
+    finally:
+        for base, _ in ups:
+            device.free(base)
+
+
 def test_chunk_header_of_many_columns(device):
     n, r = 3_000, np.random.default_rng(64)
     k, v = r.integers(0, 50, n, dtype=np.int32), r.integers(-1000, 1000, n, dtype=np.int32)
