@@ -484,6 +484,7 @@ xpuB200MixCreate(xpuB200Device *dev, uint32_t ncmds, xpuB200Session *const *sess
         a.nunits = tasks[i].nunits;
         a.format = tasks[i].format;
         a.sm_cap = s->sm_cap;
+        a.sm_trial = s->sm_trial;
         a.warp_bytes = s->warp_bytes;
         a.gt = s->d_gt;
         a.st = m->d_status + i;

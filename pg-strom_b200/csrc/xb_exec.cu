@@ -604,6 +604,8 @@ xb_exec_body(const XbExecArgs &args, char *smem)
         ((uint32_t *)sm_entries)[i] = 0;
     for (size_t i = lane; i < XB_WARP_HEAD / 4; i += 32)
         ((uint32_t *)ws)[i] = 0;
+    if (threadIdx.x == 0)
+        meta->sm_on = args.sm_cap;
     __syncthreads();
 
     const XbRegs R = xb_regs_setup(wbase + XB_WARP_HEAD + sizeof(XbCursor) * nrels_arg, plan->nregs);
@@ -614,7 +616,7 @@ xb_exec_body(const XbExecArgs &args, char *smem)
             cursors[d].live = 0;
     __syncwarp();
 
-    char *const sm_tab = args.sm_cap ? sm_entries : nullptr;
+    char *sm_tab = args.sm_cap ? sm_entries : nullptr;
     const uint32_t sm_mask = args.sm_cap ? args.sm_cap - 1 : 0;
     xb_gtable *const gt = args.gt;
     xb_status *const st = args.st;
@@ -714,6 +716,8 @@ xb_exec_body(const XbExecArgs &args, char *smem)
                     if (sm_tab)
                         e = xb_group_get<true>(plan, R, lane, sm_tab, sm_mask, hash, nullptr, st, &full);
                     if (!e) {
+                        if (sm_tab && args.sm_trial)
+                            *(volatile uint32_t *)&meta->sm_on = 0;
                         full = false;
                         e = xb_group_get<false>(plan, R, lane, gt->entries, gt->cap_mask, hash, gt, st, &full);
                         if (!e && full) {
@@ -734,6 +738,8 @@ xb_exec_body(const XbExecArgs &args, char *smem)
                 if (__any_sync(XB_FULL, bad))
                     break;
                 xb_update_states_warp(plan, e, R, lane, st);
+                if (sm_tab && args.sm_trial && !__shfl_sync(XB_FULL, *(volatile uint32_t *)&meta->sm_on, 0))
+                    sm_tab = nullptr;
                 d = nrels;
                 stage = nrels ? XB_ST_PROBE : XB_ST_FETCH;
             } else {
@@ -2903,21 +2909,33 @@ static uint64_t xb_next_pow2(uint64_t x)
 /*
  * Entries of the per-CTA shared group table for est groups: a load of at
  * most 1/4 where 48 KB hold that (four CTAs share an SM), up to 7/8 where
- * they do not, and none beyond: most rows would search a crowded table and
- * go to the global one all the same, whose entries are many enough by then
- * for the L2's atomics (2M rows, 300 groups: 2.27 ms a query through a table
- * of 256 entries, 1.35 ms without one).  Large entries count too: three
- * groups of 288 bytes take 10.1 ms in the global table, 1.43 ms here.
+ * they do not.  Beyond, most rows would search a crowded table and go to
+ * the global one all the same, whose entries are many enough by then for the
+ * L2's atomics (1M rows, 60% of them kept, 300 groups: 1.97 ms a pass when
+ * every row searched 256 entries, 155 us without a table).
+ * But the estimate may be far too high, and a few groups in the global table
+ * are lines of L2 that all rows queue at (3 groups 1.64 ms, 64 groups 300 us;
+ * 84 and 81 us in a shared table).  So up to 2048 estimated groups a table of
+ * 128 entries is there on trial: a CTA that finds it full goes on without
+ * it.  A pass estimated at 1000 groups: 85 us with 3, 86 us with 64, and 137
+ * us (117 without the trial) with 1000.
  */
-static uint32_t xb_sm_cap_for(double est, uint32_t gent_size)
+static uint32_t xb_sm_cap_for(double est, uint32_t gent_size, bool *trial)
 {
     const uint64_t room = (48 * 1024) / xb_jit_sm_stride(gent_size);
-    if (est > (double)room)
-        return 0;
-    uint64_t cap = xb_next_pow2((uint64_t)(est * 4) + 16);
-    while (cap > room && cap > 8)
+    *trial = false;
+    if (est <= (double)room) {
+        uint64_t cap = xb_next_pow2((uint64_t)(est * 4) + 16);
+        while (cap > room && cap > 8)
+            cap >>= 1;
+        if (cap <= room && est * 8 <= (double)cap * 7)
+            return (uint32_t)cap;
+    }
+    uint64_t cap = 128;
+    while (cap > room)
         cap >>= 1;
-    return cap <= room && est * 8 <= (double)cap * 7 ? (uint32_t)cap : 0;
+    *trial = est <= 2048 && cap >= 16;
+    return *trial ? (uint32_t)cap : 0;
 }
 
 extern "C" int
@@ -3061,7 +3079,7 @@ xpuB200OpenSession(xpuB200Device *dev, const kern_session_info *session, uint64_
         DALLOC(XB_GT_BYTES, &s->d_gt);
         cudaMemsetAsync(s->d_gt, 0, XB_GT_BYTES, st);
         cudaMemcpyAsync(s->d_gt, &s->h_gt, sizeof(xb_gtable), cudaMemcpyHostToDevice, st);
-        s->sm_cap = xb_sm_cap_for(est, plan->gent_size);
+        s->sm_cap = xb_sm_cap_for(est, plan->gent_size, &s->sm_trial);
     }
     /* test hooks, inert unless set: XPU_B200_WAIT_LIMIT shortens the
      * bounded wait on a BUSY group entry; XPU_B200_TEST_BUSY_GROUPS=1 marks
@@ -3137,8 +3155,11 @@ xpuB200OpenSession(xpuB200Device *dev, const kern_session_info *session, uint64_
      * relation; the specialised kernels then index the shared-memory group
      * table by id.  Needs the shared table to hold every id. */
     const size_t ia2 = s->d_allocs.size();
-    if (hit && hit->gid_cap && s->sm_cap < hit->gid_cap)
-        s->sm_cap = hit->gid_cap;
+    if (hit && hit->gid_cap) {
+        s->sm_trial = false;
+        if (s->sm_cap < hit->gid_cap)
+            s->sm_cap = hit->gid_cap;
+    }
     if (!hit && s->h_plan->gid_depth >= 1 && s->h_plan->gid_depth <= plan->nrels && plan->gent_size > 0) {
         const uint32_t d = s->h_plan->gid_depth;
         xb_inner *in = &s->h_plan->inner[d];
@@ -3171,6 +3192,7 @@ xpuB200OpenSession(xpuB200Device *dev, const kern_session_info *session, uint64_
             if (ngids >= 1 && ngids <= limit && (size_t)cap * plan->gent_size <= 48 * 1024) {
                 in->gid_on = 1;
                 in->ngids = ngids;
+                s->sm_trial = false;
                 if (s->sm_cap < cap)
                     s->sm_cap = cap;
                 cudaMemcpyAsync(&s->d_plan->inner[d], in, sizeof(xb_inner), cudaMemcpyHostToDevice, st);
@@ -3586,7 +3608,7 @@ static bool xb_part_prepare(xpuB200Session *s, uint64_t nunits, uint32_t format,
     if (stream != s->stream)
         return false;
     const xb_plan *plan = s->h_plan;
-    if (plan->has_groupby != 1 || s->sm_cap != 0)
+    if (plan->has_groupby != 1 || (s->sm_cap != 0 && !s->sm_trial))
         return false;
     const uint32_t rec = xb_jit_part_rec_size(plan, format);
     const uint64_t cap = s->h_gt.cap_mask + 1;
@@ -3868,6 +3890,7 @@ int xb_launch_on(xpuB200Session *s, const xb_task *d_tasks, uint32_t ntasks,
     void *fn = xb_session_jit(s, format, stream == s->stream);
     /* (the first launch may adopt a tuned table size) */
     a.sm_cap = s->sm_cap;
+    a.sm_trial = s->sm_trial;
     int grid = fn ? s->jit_grid[format] : s->grid;
     /* a warp per unit, up to the resident warps: a heap page takes a warp
      * about 20 us whatever runs beside it (dependent loads), so a launch of
@@ -3906,6 +3929,7 @@ int xb_launch_on(xpuB200Session *s, const xb_task *d_tasks, uint32_t ntasks,
         a.part_cnt = s->part_cnt;
         a.part_cap = s->part_cap;
         a.part_shift = s->part_shift;
+        a.sm_cap = 0;
         cudaMemsetAsync(s->part_cnt, 0, sizeof(uint32_t) * XB_PART_CNT_STRIDE * (s->nparts + 1), stream);
         s->part_used = true;
     }

@@ -601,6 +601,7 @@ struct XbExecArgs {
     uint64_t        nunits;         /* total units over all tasks */
     uint32_t        format;         /* common KDS format of the tasks */
     uint32_t        sm_cap;         /* shared-memory group table entries (0: none) */
+    uint32_t        sm_trial;       /* a CTA that finds it full goes on without it */
     uint32_t        warp_bytes;     /* shared memory of one warp: counters, cursors, registers */
     char           *dst;            /* projection: device kds_dst buffer, or nullptr */
     uint64_t        dst_len;
@@ -691,7 +692,7 @@ struct XbSrcMeta {
     int32_t  ncols;
     uint32_t fixed;                 /* 1: every depth-0 load is fixed-width at a cached offset */
     uint32_t fixed_end;             /* payload bytes those loads span */
-    uint32_t __pad;
+    uint32_t sm_on;                 /* rows look into the CTA's shared group table */
 };
 
 #define XB_WARP_HEAD    ((sizeof(XbWarpState) + 15) & ~(size_t)15)

@@ -121,6 +121,7 @@ struct xpuB200Session {
     xb_task        *d_tasks = nullptr;      /* work queue of single-chunk launches */
     uint32_t        d_tasks_cap = 0;
     uint32_t        sm_cap = 0;
+    bool            sm_trial = false;       /* the table is for fewer groups than estimated */
     uint32_t        warp_bytes = 0;
     uint32_t        plan_bytes = 0;
     size_t          smem_bytes = 0;

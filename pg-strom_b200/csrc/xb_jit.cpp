@@ -722,15 +722,16 @@ struct Gen {
         /* find or create */
         o << "template <bool SMEM>\n__device__ __forceinline__ char *\n"
              "xbj_group_get(const XbjRegs &R, const XbjEnv &E, char *entries, uint64_t cap_mask, uint32_t hash, bool *full)\n{\n"
-             "    uint64_t pos = hash & cap_mask;\n"
-             "    const uint64_t bound = SMEM ? XB_SM_PROBES - 1 : XB_PROBE_LIMIT;\n"
-             "    const uint64_t limit = cap_mask < bound ? cap_mask : bound;\n"
-             "    for (uint64_t probe = 0; probe <= limit; probe++) {\n"
-             "        char *e = entries + pos * (SMEM ? XBJ_SM_STRIDE : XBJ_GENT_SIZE);\n"
+             "    const uint32_t mask = (uint32_t)cap_mask;   /* (tables have below 2^31 slots) */\n"
+             "    uint32_t pos = hash & mask;\n"
+             "    const uint32_t bound = SMEM ? XB_SM_PROBES - 1 : XB_PROBE_LIMIT;\n"
+             "    const uint32_t limit = mask < bound ? mask : bound;\n"
+             "    for (uint32_t probe = 0; probe <= limit; probe++) {\n"
+             "        char *e = SMEM ? entries + pos * XBJ_SM_STRIDE : entries + (uint64_t)pos * XBJ_GENT_SIZE;\n"
              "        xb_gent_head *h = (xb_gent_head *)e;\n"
              "        uint32_t s = SMEM ? xb_ld_acquire_cta(&h->state) : xb_ld_acquire(&h->state);\n"
              "        if (s == XB_GSTATE_EMPTY) {\n"
-             "            const int rc = xbj_group_claim(e, hash, SMEM ? nullptr : E.gt, E.st, E.newg";
+             "            const int rc = xbj_group_claim(e, hash, SMEM ? nullptr : E.gt, E.st, xbj_counter(E)";
         for (uint32_t k = 0; k < p->nkeys; k++) {
             const int r = p->keys[k].reg;
             o << ", " << V(r) << ", " << A(r) << ", " << N(r);
@@ -749,7 +750,7 @@ struct Gen {
              "            s = SMEM ? xb_ld_acquire_cta(&h->state) : xb_ld_acquire(&h->state);\n"
              "        }\n"
              "        if (h->hash == hash && xbj_key_match(e, R))\n            return e;\n"
-             "        pos = (pos + 1) & cap_mask;\n"
+             "        pos = (pos + 1) & mask;\n"
              "    }\n"
              "    *full = true;\n    return nullptr;\n}\n\n";
 
@@ -1532,8 +1533,10 @@ struct Gen {
              "xbj_group_row(XbjRegs &R, const XbjEnv &E, const uint32_t ghash, bool &failed)\n{\n"
              "    char *e = nullptr;\n"
              "    bool full = false;\n"
-             "    if (E.sm_tab)\n"
+             "    if (E.sm_tab && *(volatile uint32_t *)E.sm_on) {\n"
              "        e = xbj_group_get<true>(R, E, E.sm_tab, E.sm_mask, ghash, &full);\n"
+             "        if (!e && E.sm_trial) *(volatile uint32_t *)E.sm_on = 0;\n"
+             "    }\n"
              "    const bool in_sm = e != nullptr;\n"
              "    if (!e) {\n"
              "        full = false;\n"
@@ -1542,7 +1545,12 @@ struct Gen {
              "            char *slot_ = xb_dump_slot(E.gt, XBJ_GENT_SIZE);\n"
              "            if (slot_) {\n"
              "                full = false;\n"
-             "                e = xbj_group_get<false>(R, E, slot_, 0, ghash, &full);\n"
+             "                e = xbj_group_claim(slot_, ghash, E.gt, E.st, xbj_counter(E)";
+        for (uint32_t k = 0; k < p->nkeys; k++) {
+            const int r = p->keys[k].reg;
+            o << ", " << V(r) << ", " << A(r) << ", " << N(r);
+        }
+        o << ") == 1 ? slot_ : nullptr;\n"
              "            }\n"
              "        }\n"
              "        if (!e && full) {\n"
@@ -1636,7 +1644,7 @@ struct Gen {
             program(p->gb_keyhash, i2);
             o << i2 << "if (failed) return;\n"
               << i2 << "const uint32_t ghash = (uint32_t)" << V(p->gb_keyhash.result) << ";\n"
-              << i2 << "if (gs == XB_GSTATE_EMPTY && xbj_group_claim(e, ghash, nullptr, E.st, E.newg";
+              << i2 << "if (gs == XB_GSTATE_EMPTY && xbj_group_claim(e, ghash, nullptr, E.st, nullptr";
             for (uint32_t k = 0; k < p->nkeys; k++) {
                 const int r = p->keys[k].reg;
                 o << ", " << V(r) << ", " << A(r) << ", " << N(r);

@@ -39,6 +39,8 @@ struct XbjEnv {
     uint64_t        gt_mask;
     char           *sm_tab;         /* shared-memory group table, or nullptr */
     uint32_t        sm_mask;
+    uint32_t       *sm_on;          /* shared memory: rows look there */
+    uint32_t        sm_trial;       /* until the CTA finds it full */
     uint32_t        lane;
     char           *dst;            /* projection: kds_dst and its length */
     uint64_t        dst_len;
@@ -48,8 +50,26 @@ struct XbjEnv {
     uint32_t        part_cap;
     uint32_t        part_shift;
     uint32_t        replay;         /* in the replay: a full table leaves the record for later */
-    uint32_t       *newg;           /* shared memory: new global groups not yet counted in the table */
+    uint32_t       *newg;           /* shared memory: new global groups not yet counted in the
+                                     * table (nullptr: xbj_newg) */
 };
+
+/* the warps' work-distribution state, at the start of the main kernels'
+ * dynamic shared memory after the source's metadata; the warp's count of
+ * new global groups in it */
+#define XBJ_WSRC_AT     ((sizeof(XbSrcMeta) + 15) & ~(size_t)15)
+__device__ __forceinline__ uint32_t *xbj_newg()
+{
+    extern __shared__ __align__(16) char smem[];
+    return &((XbSrc *)(smem + XBJ_WSRC_AT))[threadIdx.x >> 5].newg;
+}
+
+/* where a new global group is counted: the address is worked out at each
+ * use, not kept in registers over the main loop */
+__device__ __forceinline__ uint32_t *xbj_counter(const XbjEnv &E)
+{
+    return E.newg ? E.newg : xbj_newg();
+}
 
 /* per-thread counters, 32-bit to spare registers; flushed into the launch
  * totals whenever one passes 2^31 (checked once per batch) */
@@ -294,13 +314,15 @@ xbj_body(const XbExecArgs &args, char *smem)
     XbSrcMeta *meta = (XbSrcMeta *)smem;
     /* warp-uniform work-distribution state lives in shared memory, not in
      * registers (read once per unit) */
-    XbSrc *wsrc = (XbSrc *)(smem + ((sizeof(XbSrcMeta) + 15) & ~(size_t)15));
+    XbSrc *wsrc = (XbSrc *)(smem + XBJ_WSRC_AT);
     char *sm_entries = (char *)(wsrc + XB_WARPS);
     const size_t sm_bytes = (size_t)args.sm_cap * XBJ_SM_STRIDE;
 
     xb_setup_meta(args, meta);
     for (size_t i = threadIdx.x; i < sm_bytes / 4; i += blockDim.x)
         ((uint32_t *)sm_entries)[i] = 0;
+    if (threadIdx.x == 0)
+        meta->sm_on = args.sm_cap;
     /* after the group table: the existence bitmaps of filter depths */
     uint32_t *sbits = (uint32_t *)(((uintptr_t)(sm_entries + sm_bytes) + 15) & ~(uintptr_t)15);
 #ifdef XBJ_BITS
@@ -323,6 +345,8 @@ xbj_body(const XbExecArgs &args, char *smem)
     E.gt_mask = args.gt ? args.gt->cap_mask : 0;
     E.sm_tab = args.sm_cap ? sm_entries : nullptr;
     E.sm_mask = args.sm_cap ? args.sm_cap - 1 : 0;
+    E.sm_on = &meta->sm_on;
+    E.sm_trial = args.sm_trial;
     E.lane = lane;
     E.dst = args.dst;
     E.dst_len = args.dst_len;
@@ -332,9 +356,9 @@ xbj_body(const XbExecArgs &args, char *smem)
     E.part_cap = args.part_cap;
     E.part_shift = args.part_shift;
     E.replay = 0;
-    E.newg = &wsrc[threadIdx.x >> 5].newg;
+    E.newg = nullptr;
     if (lane == 0)
-        *E.newg = 0;
+        *xbj_newg() = 0;
     XbjCnt C;
     C.raw = C.in = C.out = 0;
     C.gready = 0;
@@ -539,8 +563,8 @@ xbj_body(const XbExecArgs &args, char *smem)
         }
         /* (at most XB_UNCOUNTED groups of a warp stay uncounted between
          * batches, which the growth's dump region allows for) */
-        if (args.left_out && lane == 0 && *(volatile uint32_t *)E.newg > XBJ_UNCOUNTED)
-            xbj_count_flush(args.gt, E.newg);
+        if (args.left_out && lane == 0 && *(volatile uint32_t *)xbj_newg() > XBJ_UNCOUNTED)
+            xbj_count_flush(args.gt, xbj_newg());
     }
     if (stop)
         xb_src_leave(args, src, lane, item, nitems);
@@ -557,7 +581,7 @@ xbj_body(const XbExecArgs &args, char *smem)
     __syncwarp();
 #endif
     if (lane == 0 && args.gt)
-        xbj_count_flush(args.gt, E.newg);
+        xbj_count_flush(args.gt, xbj_newg());
     /* statistics */
     {
         const unsigned long long raw = xbj_warp_sum(C.raw);
@@ -646,6 +670,8 @@ __device__ __forceinline__ void xbj_replay_env(XbjEnv &E, const XbReplayArgs &ar
     E.gt_mask = args.gt->cap_mask;
     E.sm_tab = nullptr;
     E.sm_mask = 0;
+    E.sm_on = nullptr;
+    E.sm_trial = 0;
     E.lane = threadIdx.x & 31;
     E.dst = nullptr;
     E.dst_len = 0;

@@ -327,6 +327,7 @@ static int xb_sched_launch(xpuB200Device *dev, xb_sched *q, xb_slot &sl, kern_er
                 a.nunits = sl.cmds[i].units;
                 a.format = sl.cmds[i].format;
                 a.sm_cap = s->sm_cap;
+                a.sm_trial = s->sm_trial;
                 a.warp_bytes = s->warp_bytes;
                 a.gt = s->d_gt;
                 a.st = sl.d_status + i;

@@ -44,7 +44,8 @@ def _oracle(sess, chunks):
 # ---- shared group tables: the capacity follows the estimate, the groups
 # may be more or fewer (est entries of 112 + 8 bytes: 256 entries at most)
 @pytest.mark.parametrize("est,groups", [(1, 1), (1, 700), (3, 3), (60, 64), (64, 900), (200, 200), (224, 230),
-                                        (225, 225), (400, 390), (410, 3000)])
+                                        (225, 225), (400, 390), (410, 3000), (300, 1), (2048, 3), (2049, 3), (1000, 90),
+                                        (1000, 127), (1000, 129), (2000, 256)])
 def test_shared_table_estimates(device, est, groups):
     tbl, _, _, expect, meta = C.scan_groupby(nrows=40_000, seed_config=60 + est % 7, a_limit=600, ngroups=groups)
     got, res = _run(device, C.scan_groupby_session(600, est), tbl.block_chunks(pages_per_chunk=300))
@@ -52,11 +53,35 @@ def test_shared_table_estimates(device, est, groups):
     assert F.compare_groups(got, _truth(expect)) == []
 
 
-@pytest.mark.parametrize("est,groups", [(1, 2), (3, 3), (100, 112), (113, 150)])
+@pytest.mark.parametrize("est,groups", [(1, 2), (3, 3), (100, 112), (113, 150), (500, 3), (2000, 70)])
 def test_shared_table_of_large_entries(device, est, groups):
     tbl, _, _, expect, _ = C.wide_groupby(nrows=30_000, seed_config=70, ngroups=groups)
     got, _ = _run(device, C.wide_groupby_session(ngroups=est), tbl.block_chunks(pages_per_chunk=300))
     assert F.compare_groups(got, expect) == []
+
+
+def test_estimate_far_above_the_groups(device, monkeypatch):
+    # a few groups take about as long under a high estimate as under the right
+    # one, on both kernels (20 times as long in the global table)
+    tbl, _, _, expect, _ = C.scan_groupby(nrows=1_000_000, seed_config=71, a_limit=600, ngroups=3)
+    ups = [device.upload(c) for c in tbl.block_chunks(pages_per_chunk=4000)]
+    try:
+        for jit in ("1", "0"):
+            monkeypatch.setenv("XPU_B200_JIT", jit)
+            ms = {}
+            for est in (3, 1000):
+                s = xpu_b200.Session(device, C.scan_groupby_session(600, est))
+                b = s.batch([p for _, p in ups])
+                b.exec()
+                got = F.decode_kds_final(s.final()[0], C.scan_groupby_session(600, est))
+                assert F.compare_groups(got, _truth(expect)) == []
+                ms[est] = min(b.time(3) for _ in range(5))
+                b.close()
+                s.close()
+            assert ms[1000] < 3 * ms[3], (jit, ms)
+    finally:
+        for base, _ in ups:
+            device.free(base)
 
 
 # ---- no GROUP BY: every state form from the lanes' registers
