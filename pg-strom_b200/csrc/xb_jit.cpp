@@ -2124,6 +2124,15 @@ struct Gen {
             o << "#define XBJ_PART 1\n#define XBJ_REC_SIZE " << part_rec_size() << "\n";
         if (compact())
             o << "#define XBJ_COMPACT 1\n";
+        /* rows create groups in the global table (or the one group there
+         * is): the warp counts them.  Where the groups are numbered they
+         * come with the merge at the end, and the count, its reset and its
+         * look after every batch are left out (100M rows joined, a pass:
+         * 1270 us with them, 1245 without) */
+        if (p->has_groupby == 1 && !gid_mode())
+            o << "#define XBJ_KEYED 1\n";
+        if ((p->has_groupby == 1 && !gid_mode()) || p->has_groupby == 2)
+            o << "#define XBJ_NEWG 1\n";
         if (format == KDS_FORMAT_ARROW && p->nload0 > 0)
             o << "#define XBJ_ACOLS " << p->nload0 << "\n";
         o << "struct XbjRegs {\n"
