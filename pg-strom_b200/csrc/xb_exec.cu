@@ -3681,8 +3681,9 @@ static bool xb_part_prepare(xpuB200Session *s, uint64_t nunits, uint32_t format,
  * (gpu_service.c:2418-2470, :3872-3879; resume at cuda_gpujoin.cu:
  * 1098-1103).  Here the table asks to grow before it is full: once half of
  * its slots are in use (or half of the key arena), every warp of a launch
- * on the session's stream stops after its current 32-row batch and records
- * the work it held (XbLeft ranges).  Groups that meanwhile find the table
+ * on the session's stream stops after its current 32-row batch (where Arrow
+ * rows are compacted: after the batch it filters and the rows that wait in
+ * its queue) and records the work it held (XbLeft ranges).  Groups that meanwhile find the table
  * without room take an entry of the dump region.  The host then rehashes
  * the live entries into a table at least twice as large, merges the dump
  * entries in, and a resume launch processes the recorded ranges and the

@@ -22,8 +22,7 @@
 #define XB_SM_PROBES    32          /* max probes in a CTA's shared group table: a group that
                                      * finds no entry in reach goes to the global table (with
                                      * the whole table searched, every row of such a group
-                                     * read all of it: a query over 2M rows with 1000 groups
-                                     * took 2.41 ms, 1.30 ms now) */
+                                     * read all of it) */
 
 /*
  * Hide a pointer's address space from the compiler.  Group-state atomics
@@ -143,10 +142,12 @@ __device__ __forceinline__ void xb_gt_want_grow(xb_gtable *gt)
 /* new global entries a warp of a specialised kernel may leave uncounted
  * between 32-row batches */
 #define XB_UNCOUNTED    31
-/* rows a warp may still apply after the table asked to grow: the 32 it is
- * applying and 32 more if its look at the request came just before; where
- * Arrow rows are compacted also 32 if its copy of the request was still to
- * be written, and the rows that wait in its queue (31) */
+/* source rows a warp may still apply after the table asked to grow: the 32
+ * it is applying and 32 more if its look at the request came just before;
+ * where Arrow rows are compacted also 32 if its copy of the request was still
+ * to be written, and the rows that wait in its queue (31).  Groups at most,
+ * if no source row joins to several rows; where it does, a table without
+ * room and a full dump region are reported as such (SUSPEND_NO_SPACE) */
 #define XB_INFLIGHT         64
 #define XB_INFLIGHT_ARROW   127
 

@@ -31,6 +31,10 @@ static void xb_final_program(const xb_plan *plan, bool row_fmt, XbFinalProg *pg)
 {
     pg->nunits = 0;
     pg->item = 0;
+    /* test hook, inert unless set: every tuple by the general writer */
+    const char *off = getenv("XPU_B200_TEST_NO_FINAL_PROGRAM");
+    if (off && off[0] == '1')
+        return;
     uint8_t img[XB_FINAL_UNITS * 4] = {0};
     uint16_t op[XB_FINAL_UNITS] = {0}, src[XB_FINAL_UNITS] = {0};
     const uint32_t n = plan->naggs;

@@ -764,7 +764,8 @@ struct Gen {
          * distinct entry with the other lanes idle), so each lane updates
          * its entry directly.  The sums whose old value is needed are all
          * added before the first of these values is looked at: a lane waits
-         * for the table once, not once a sum (2M rows, every statistic, 3000\n         * groups: 972 -> 958 us a query, 933 with the minima and maxima below) */
+         * for the table once, not once a sum (2M rows, every statistic, 3000
+         * groups: 972 -> 958 us a query, 933 with the minima and maxima below) */
         std::ostringstream late;
         o << "__device__ __forceinline__ void xbj_update(char *e, const XbjRegs &R, const XbjEnv &E)\n{\n"
              "    (void)E;\n" << numeric_args();

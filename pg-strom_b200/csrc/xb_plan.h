@@ -409,9 +409,9 @@ typedef struct xb_gtable {
 /* The growth request for the CTAs of a specialised kernel: copies of 'grow'
  * behind the table's header, each in a line of its own, one for every
  * XB_GROW_COPIES-th CTA.  Where Arrow rows are compacted every warp looks at
- * the request once per 32 rows that it filters; at the one word in the header, next to the count of the groups, these
- * looks waited for one another (20M Arrow rows into 1.7M groups 2.46 ms a
- * query, 1.78 ms with the copies). */
+ * the request once per 32 rows that it filters; at the one word in the
+ * header, next to the count of the groups, these looks waited for one another
+ * (20M Arrow rows into 1.7M groups 2.46 ms a query, 1.78 ms with the copies). */
 #define XB_GROW_COPIES  64
 #define XB_GROW_STRIDE  128
 #define XB_GROW_OFF     256

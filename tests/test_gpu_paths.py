@@ -197,11 +197,10 @@ def test_extreme_values(device, monkeypatch, path):
         assert got == want
 
 
-# ---- rows compacted between the quals and the rest: none, few, all pass;
-# pages and units of a few rows; a filtered projection
+# ---- filters that none, few and all rows of a page pass
 @pytest.mark.parametrize("limit", [0, 1, 500, 1000])
 @pytest.mark.parametrize("nrows", [1, 31, 130, 20_000])
-def test_compaction_selectivities(device, nrows, limit):
+def test_filter_selectivities(device, nrows, limit):
     tbl, sess, _, expect, meta = C.scan_groupby(nrows=nrows, seed_config=62, a_limit=limit, ngroups=2_000)
     got, res = _run(device, sess, tbl.block_chunks(pages_per_chunk=7))
     assert (res["nitems_raw"], res["nitems_in"]) == (meta["nitems_raw"], meta["nitems_in"])
@@ -214,6 +213,22 @@ def test_compaction_arrow_units(device, nrows, batch):
     got, res = _run(device, sess, chunks)
     assert res["nitems_in"] == meta["nitems_in"]
     assert F.compare_groups(got, expect) == []
+
+
+# ---- Arrow rows compacted between the quals and the rest: none, few and all
+# of a unit's rows wait in the queue
+@pytest.mark.parametrize("lo,hi", [(30_000, 30_001), (16_436, 16_437), (17_532, 18_262), (0, 30_000)])
+@pytest.mark.parametrize("nrows,batch", [(1, 1), (33, 33), (1_024, 1_024), (20_000, 3_001)])
+def test_compaction_arrow_selectivities(device, nrows, batch, lo, hi):
+    chunks, _, _, _ = C.arrow_groupby(nrows=nrows, nkeys=300, rows_per_chunk=batch, seed_config=69, with_expect=False)
+    sess = C.arrow_groupby_session(lo, hi, ngroups_estimate=300.0)
+    want = _oracle(sess, chunks)
+    got, res = _run(device, sess, chunks)
+    assert res["nitems_raw"] == nrows
+    assert res["nitems_in"] == sum(v[0] for v in want.values())
+    if lo == 30_000 or hi == 30_000:
+        assert res["nitems_in"] == (nrows if hi == 30_000 else 0)
+    assert F.compare_groups(got, want) == []
 
 
 def test_value_saved_by_the_quals(device):

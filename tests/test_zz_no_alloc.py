@@ -159,3 +159,56 @@ def test_final_without_allocation_refuses_memory_it_cannot_write(device):
         assert F.compare_groups(F.decode_kds_final(got, sess), truth) == []
     finally:
         s.close()
+
+
+def _program_item(sess):
+    """item bytes of the session's fixed tuple (0: none)"""
+    L = ctypes.CDLL(xpu_b200.LIB_PATH)
+    plan, err = ctypes.create_string_buffer(1 << 20), ctypes.create_string_buffer(1024)
+    rc = L.xb_compile_session(bytes(sess), ctypes.c_size_t(len(sess)), ctypes.c_uint64(1 << 32), None, plan, err,
+                              ctypes.c_size_t(len(err)))
+    assert rc == 0, err.value
+    return L.xb_final_program_item(plan)
+
+
+@pytest.mark.parametrize("case", ["every_state", "keys", "text_key", "null_key", "no_key"])
+def test_fixed_tuples_equal_the_general_writers(device, monkeypatch, case):
+    """kds_final word by word from the plan's program, and by the general
+    tuple writer: the same bytes, header bits and padding included, whatever
+    the buffer held before."""
+    torch = pytest.importorskip("torch")
+    from test_gpu_paths import _extreme_table
+    from xb_producer import Agg, Column, SessionBuilder, Table, Var, encode_text_from_dict
+    tbl = _extreme_table(4_000)                 # group 5: no value but NULLs in b
+    vw, vb, vg = Var(0, 1, "int8"), Var(0, 2, "float8"), Var(0, 3, "int4")
+    aggs = [Agg("NROWS_ANY"), Agg("NROWS_COND", vb), Agg("PMIN_INT64", vw), Agg("PMAX_INT64", vw), Agg("PMIN_FP64", vb),
+            Agg("PMAX_FP64", vb), Agg("PSUM_FP", vb), Agg("PAVG_INT64", vw), Agg("STDDEV", vb), Agg("COVAR", vb, arg1=vb),
+            Agg("PMIN_INT32", vg), Agg("PSUM_INT", vw)]
+    keys = {"every_state": [vg], "keys": [vg, Var(0, 4, "date"), vw], "text_key": [Var(0, 5, "text"), vg],
+            "null_key": [Var(0, 4, "date")], "no_key": []}[case]
+    n = 4_000
+    tbl = Table("t", tbl.columns + [
+        Column("d", "date", values=(np.arange(n) % 11).astype(np.int32), nulls=(np.arange(n) % 3 == 0) if case == "null_key" else None),
+        Column("s", "text", values=encode_text_from_dict(np.arange(n) % 7, ["key%d" % i for i in range(7)]))], n)
+    sess = SessionBuilder(0, C.DEVTASK_PREAGG | C.DEVKIND_GPU).build(groupby_keys=keys, aggs=aggs, ngroups_estimate=100.0)
+    assert (_program_item(sess) > 0) == (case != "text_key")
+    s = xpu_b200.Session(device, sess)
+    try:
+        for ch in tbl.block_chunks(pages_per_chunk=20):
+            s.exec(ch)
+        got = []
+        for off, fill in (("0", 0xA5), ("1", 0x5A)):
+            monkeypatch.setenv("XPU_B200_TEST_NO_FINAL_PROGRAM", off)
+            _, need, _, _ = _final_no_alloc(s, 0, 0)
+            out = torch.full((need,), fill, dtype=torch.uint8, device="cuda:0")
+            torch.cuda.synchronize()
+            rc, _, _, msg = _final_no_alloc(s, out.data_ptr(), need)
+            assert rc == 0, msg
+            got.append(out.cpu().numpy())
+    finally:
+        s.close()
+    assert F.decode_kds_final(got[0], sess)
+    if case == "no_key":
+        assert got[0].tobytes() == got[1].tobytes()
+    else:
+        assert _layout(got[0]) == _layout(got[1])
