@@ -3428,7 +3428,9 @@ std::map<std::pair<int, uint64_t>, int> g_tune_minb;
 
 std::tuple<int, uint64_t, uint32_t> xb_tune_key(xpuB200Session *s, uint32_t format)
 {
-    return std::make_tuple(s->dev->dindex, xb_jit_shape_key(s->h_plan, format), s->sm_cap_default);
+    /* (a table on trial is not the shape of one that the estimate fits) */
+    return std::make_tuple(s->dev->dindex, xb_jit_shape_key(s->h_plan, format),
+                           s->sm_cap_default | (s->sm_trial ? 0x80000000u : 0u));
 }
 
 static bool xb_tune_lookup(xpuB200Session *s, uint32_t format, xb_tune_choice *c)

@@ -94,3 +94,28 @@ def test_tune_after_exec_is_rejected(device):
         s.close()
         for x in bases:
             device.free(x)
+
+
+def test_tuned_trial_table_is_not_adopted_by_a_right_estimate(device):
+    # tables of 128 entries by default, of a plan that estimates 1000 groups
+    # (on trial) and of one that estimates 20: two shapes for the tuner
+    tbl, _, _, expect, _ = C.scan_groupby(nrows=300_000, seed_config=24, a_limit=900, ngroups=1000)
+    bases, ptrs = _upload(device, tbl.block_chunks(pages_per_chunk=1000))
+    try:
+        s = xpu_b200.Session(device, C.scan_groupby_session(900, 1000))
+        b = s.batch(ptrs)
+        rep = b.tune()
+        b.exec()
+        got = F.decode_kds_final(s.final()[0], C.scan_groupby_session(900, 1000))
+        assert F.compare_groups(got, {k: [v["nrows"], v["sum_a"], v["sum_c"], v["avg_b"]] for k, v in expect.items()}) == []
+        assert rep["default_sm_groups"] == 128
+        b.close()
+        s.close()
+        s = xpu_b200.Session(device, C.scan_groupby_session(900, 20))
+        s.exec(ptrs[0], on_device=True)
+        info = s.info()
+        s.close()
+        assert info["sm_cap"] == info["sm_cap_default"] == 128, info
+    finally:
+        for x in bases:
+            device.free(x)
